@@ -252,6 +252,7 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
             break;
         }
         if ((r = fl_kernels_init(s)) != FL_OK) break;
+        if ((r = fl_density_init()) != FL_OK) break;
         if ((r = fl_cells_init(s)) != FL_OK) break;
         if ((r = fl_pairs_init()) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->dev_err, 256)) != FL_OK) break;
@@ -1393,7 +1394,7 @@ extern "C" int fl_neighbour_passes_in_use(fl_system *s) {
 
 extern "C" int fl_launch_shapes(fl_system *s, int *shapes) {
     if (!s || !shapes) return fl_fail(FL_ERR_ARG, "fl_launch_shapes: null argument");
-    shapes[0] = s->blk_density ? s->blk_density : 256;
+    shapes[0] = fl_density_block(s);
     shapes[1] = s->blk_force ? s->blk_force : 128;
     shapes[2] = s->blk_sort ? s->blk_sort : 256;
     shapes[3] = s->sort_cells ? s->sort_cells : 4;

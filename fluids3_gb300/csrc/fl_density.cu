@@ -1,0 +1,426 @@
+// The density pass (computePressure, fluids4.0/fluid_kernels.cu:112-149).
+//
+// The search block of a cell is gridSrch^2 rows of cells; a row's cells are
+// consecutive in x, so their points are one run of slots, and the reference
+// loop (cells in y, z, x order, members in slot order) visits the rows in
+// order and each row in ascending slots.
+//
+// k_density_rows: a thread per point walks its rows. For gridSrch > 2, whose
+// small cells leave few candidates that are not pairs.
+//
+// k_density: a warp per 32 consecutive slots, for gridSrch 2, whose block
+// holds about twenty candidates per pair. It walks the union of its points'
+// rows once:
+//   1. Staging. 32 slots a time, coalesced; a candidate outside the box of
+//      the warp's points widened by the support radius is dropped, the others
+//      are appended to a buffer in shared memory, in visiting order.
+//   2. Filter, on the tensor cores. With coordinates rounded to whole
+//      thousandths of the box, d^2 - r^2 of 16 points against 8 candidates is
+//      one m16n8k16 product of half-precision integers, exact in FP32; r is h
+//      widened by the most that rounding can move a distance. Its sign bits
+//      become one bit per (point, candidate).
+//   3. Sum. Each lane visits the set bits of its own point in order and
+//      evaluates the pair exactly as the reference does (same test, same
+//      rounding, same order), so neither the filter nor the candidates that
+//      another point of the warp brought in change a bit of the result.
+//
+// What bounds it: instruction issue (88 warp instructions a point, half of them
+// the sum's: about 24 visits a warp, the lanes' mean being 16). A thread per
+// point over flag-pruned candidates took 157, and its chain of dependent loads
+// left small scenes waiting: 2,048 points 35.0 us then, 18.4 now; 65,536:
+// 46.1, 24.7; 1,000,000 (wave tank): 164, 110. With gridSrch 3 (250,000
+// points, 165 candidates and 70 pairs a point) the rows take 95 us, the old
+// loop took 118 and the filter 140: there every third candidate is a pair, and
+// a warp's points come from more runs than one.
+//
+// The tensor instruction is mma.sync: a tile of 16 x 8 with a depth of 16 has
+// too little work for tcgen05's descriptors, and the accumulator's signs
+// are wanted in registers at once.
+#include <algorithm>
+
+#include <cuda_fp16.h>
+
+#include "fl_internal.h"
+
+namespace {
+
+#include "fl_device.cuh"
+#include "fl_step.cuh"
+
+constexpr int kCap = 192;                       // candidates staged per round
+constexpr int kFill = kCap - 32;                // a round stops staging past this
+constexpr int kWords = kCap / 32;               // mask words per point
+constexpr int kMaskRow = kWords + 1;            // (odd: the rows of a tile fall on distinct banks)
+// per warp, in words: candidates (position, slot), the product columns of 32
+// of them, and the points' product rows, whose place the masks then take
+constexpr int kWarpWords = kCap * 4 + 32 * 8 + 32 * 8;
+static_assert(32 * kMaskRow <= 32 * 8, "the masks fit where the product rows were");
+constexpr int kMaxSegments = 8;                 // runs of points a warp takes one by one; beyond, lanes walk alone
+constexpr float kUnits = 1000.0f;               // half the widest side of the box, in units (2 x stays exact in half)
+constexpr float kBase = 2048.0f;                // squares are split into kBase * high + low, both exact in half
+constexpr float kFar = 6.0e4f;                  // times kBase: beyond any square
+constexpr int kDensityThreads = 128;
+constexpr int kRowsMaxThreads = 256;
+
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// v / scale rounded to a whole number, for |v / scale + offset| < 2^22.
+__device__ __forceinline__ float whole(float v, float scale, float offset) {
+    constexpr float kRound = 12582912.0f;   // 1.5 * 2^23: adding it leaves no fraction bits
+    return __fmaf_rn(v, scale, kRound + offset) - kRound;
+}
+
+// d = A (16 points x 16) . B (16 x 8 candidates): lane (g, t) holds rows g and
+// g + 8, columns 2t, 2t + 1, 2t + 8, 2t + 9 of A and the same rows of column
+// g of B, and gets columns 2t, 2t + 1 of rows g (d0, d1) and g + 8 (d2, d3).
+// a row's words: its lanes' (2t, 2t + 1), (2t + 8, 2t + 9) for t = 0..3.
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint2 r0, uint2 r1, uint2 b) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(r0.x), "r"(r1.x), "r"(r0.y), "r"(r1.y), "r"(b.x), "r"(b.y), "f"(0.0f));
+}
+
+// One point's running sum and pair list.
+struct Sum {
+    float4 p;
+    float sum;
+    uint32_t nh;
+    uint32_t *next;      // where its next pair goes (entries 32 words apart)
+};
+
+// Adds the pair with the candidate at q (slot j) if it passes the
+// reference's test. Branch-free: a miss adds +0.0, which leaves the sum's
+// bits unchanged (it starts at +0.0 and its terms are positive). The list
+// store is predicated by hand: compiled as a branch it cost 25 instructions
+// per candidate, a quarter of the pass.
+__device__ __forceinline__ void visit(Sum &s, const DevParams &P, float4 q, uint32_t j, bool on) {
+    float dx2, dy2;
+    const uint64_t dxy = sub2(pk2(s.p.x, s.p.y), pk2(q.x, q.y));
+    const float dz = s.p.z - q.z;
+    up2(mul2(dxy, dxy), dx2, dy2);
+    const float dsq = dx2 + dy2 + dz * dz;
+    const bool hit = on && dsq < P.rd2 && dsq > 0.0f;
+    float t = (P.rd2 - dsq) * P.d2;
+    t = t * t * t;
+    s.sum += hit ? t : 0.0f;
+    const uint32_t cap = hit ? (uint32_t)P.hcap : 0u;
+    asm volatile("{\n.reg .pred p;\nsetp.lt.u32 p, %2, %3;\n@p st.global.u32 [%0], %1;\n}" ::"l"(s.next), "r"(j),
+                 "r"(s.nh), "r"(cap));
+    s.next += hit ? 32 : 0;
+    s.nh += hit ? 1u : 0u;
+}
+
+// One point by itself: every slot of its search block, kAhead positions
+// requested before the first of them is used.
+constexpr uint32_t kAhead = 4;
+__device__ __forceinline__ void walk(const DevParams &P, Sum &s, uint32_t gc, const float4 *__restrict__ pos,
+                                     const uint32_t *__restrict__ off) {
+    const int srch = P.gridSrch, rows = srch * srch;
+    const uint32_t *at = off + ((int)gc - P.nadj);
+    uint32_t j = at[0], j1 = at[srch];
+    for (int r = 1;; r++) {
+        uint32_t nj = 0, nj1 = 0;
+        if (r < rows) {   // the next row's bounds while this one is walked
+            const int a = P.adj[r * srch];
+            nj = at[a];
+            nj1 = at[a + srch];
+        }
+        for (; j < j1; j += kAhead) {
+            float4 q[kAhead];
+#pragma unroll
+            for (uint32_t k = 0; k < kAhead; k++) q[k] = pos[min(j + k, j1 - 1u)];
+#pragma unroll
+            for (uint32_t k = 0; k < kAhead; k++) visit(s, P, q[k], j + k, j + k < j1);
+        }
+        if (r >= rows) break;
+        j = nj;
+        j1 = nj1;
+    }
+}
+
+// The sums of the warp's points in `seg` (consecutive points of one row of
+// cells, a few cells apart at most). All lanes call it.
+__device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg, uint32_t gc, int cx,
+                                        const float4 *__restrict__ pos, const uint32_t *__restrict__ off,
+                                        uint32_t *s_warp) {
+    float4 *const s_cand = reinterpret_cast<float4 *>(s_warp);
+    uint32_t *const s_col = s_warp + kCap * 4, *const s_mask = s_col + 32 * 8;
+    const unsigned lane = lane_id();
+    const int g = (int)(lane >> 2), t = (int)(lane & 3u);
+    const bool mine = (seg >> lane) & 1u;
+    const int first = __ffs(seg) - 1, last = 31 - __clz(seg);
+    const uint32_t ca = __shfl_sync(0xffffffffu, gc, first), cb = __shfl_sync(0xffffffffu, gc, last);
+    const int cxa = __shfl_sync(0xffffffffu, cx, first);
+    constexpr int srch = 2, rows = 4;
+    // the rows of the search block: lane r holds row r's slots [lo, hi)
+    uint32_t lo = 0, hi = 0;
+    if ((int)lane < rows) {
+        const int at = ((int)(lane >> 1) * P.gridRes.z + (int)(lane & 1u)) * P.gridRes.x - P.nadj;
+        lo = off[(int)ca + at];
+        hi = off[(int)cb + at + srch];
+    }
+    const float px = __shfl_sync(0xffffffffu, s.p.x, first), py = __shfl_sync(0xffffffffu, s.p.y, first),
+                pz = __shfl_sync(0xffffffffu, s.p.z, first);
+    const float vx = mine ? s.p.x : px, vy = mine ? s.p.y : py, vz = mine ? s.p.z : pz;
+    const float lx = warp_min(vx), ux = warp_max(vx), ly = warp_min(vy), uy = warp_max(vy), lz = warp_min(vz),
+                uz = warp_max(vz);
+    const float ox = 0.5f * (lx + ux), oy = 0.5f * (ly + uy), oz = 0.5f * (lz + uz);
+    const float ex = fmaxf(ux - ox, ox - lx), ey = fmaxf(uy - oy, oy - ly), ez = fmaxf(uz - oz, oz - lz);
+    const float bx = ex + P.band, by = ey + P.band, bz = ez + P.band;   // a candidate's largest offset
+    // units: a distance between rounded points is off by at most sqrt(3) < 1.8
+    const float k = kUnits / fmaxf(fmaxf(bx, by), bz);
+    const float qx = -ox * k, qy = -oy * k, qz = -oz * k;
+    const float reach = sqrtf(P.rd2) * k + 1.8f, reach2 = ceilf(reach * reach) + 4.0f;
+    const int rel = cx - cxa;   // the point's block starts this many cells into the rows
+    const int span = __shfl_sync(0xffffffffu, rel, last);
+    // With points of at most three cells the product also leaves each point
+    // the candidates of its own block: it holds which cell the point is in,
+    // and per cell whether the candidate lies past its block (those before it
+    // are more than a cell, and so more than h, away). Else the masks are cut
+    // below.
+    const bool cut = !(span <= 2 && P.cellw.x > P.band);
+    __syncwarp();
+    {   // row: -2 (x, y, z), kBase, 1, |x|^2 as (high, low), the cell
+        float x = 0.0f, y = 0.0f, z = 0.0f, high = kFar, low = 0.0f;
+        if (mine) {
+            x = whole(vx, k, qx), y = whole(vy, k, qy), z = whole(vz, k, qz);
+            const float n2 = x * x + y * y + z * z;
+            high = whole(n2, 1.0f / kBase, 0.0f), low = n2 - high * kBase;
+        }
+        uint4 *row = reinterpret_cast<uint4 *>(s_mask + lane * 8);
+        row[0] = make_uint4(half2_bits(-2.0f * x, -2.0f * y), half2_bits(-2.0f * z, kBase), half2_bits(1.0f, high),
+                            half2_bits(low, !cut && rel == 0 ? kBase : 0.0f));
+        row[1] = make_uint4(half2_bits(!cut && rel == 1 ? kBase : 0.0f, !cut && rel == 2 ? kBase : 0.0f), 0u, 0u, 0u);
+    }
+    __syncwarp();
+    uint2 a[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) a[q] = *reinterpret_cast<const uint2 *>(s_mask + (g + 8 * q) * 8 + 2 * t);
+    const bool half0 = (seg & 0xffffu) != 0, half1 = (seg >> 16) != 0;
+
+    int r = -1;
+    uint32_t jb = 0, j1 = 0;
+    bool have = true;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto next = [&]() {   // the next 32 slots: jb (the current row to j1), their positions in q
+        jb += 32;
+        while (jb >= j1) {
+            if (++r >= rows) { have = false; return; }
+            jb = __shfl_sync(0xffffffffu, lo, r);
+            j1 = __shfl_sync(0xffffffffu, hi, r);
+        }
+        q = pos[min(jb + lane, j1 - 1u)];
+    };
+    next();
+    while (have) {
+        int cnt = 0;
+        while (have && cnt <= kFill) {
+            const uint32_t j = jb + lane;
+            const float4 p = q;
+            const bool keep = j < j1 && fabsf(p.x - ox) <= bx && fabsf(p.y - oy) <= by && fabsf(p.z - oz) <= bz;
+            next();
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (keep) s_cand[cnt + __popc(kept & ((1u << lane) - 1u))] = make_float4(p.x, p.y, p.z, __uint_as_float(j));
+            cnt += __popc(kept);
+        }
+        if (cnt == 0) break;
+        const int words = (cnt + 31) >> 5;
+        uint32_t *const row = s_mask + lane * kMaskRow;
+        uint8_t *mb = reinterpret_cast<uint8_t *>(s_mask + g * kMaskRow) + t;
+        __syncwarp();
+        for (int w = 0; w < words; w++, mb += 4) {
+            // this word's columns, a lane each: (x, y, z), |y|^2 - r^2 as
+            // (high, low), kBase, 1, and per cell whether the candidate is
+            // past its block; past the last candidate, near no point
+            const int e = w * 32 + (int)lane;
+            float x = 0.0f, y = 0.0f, z = 0.0f, high = kFar, low = 0.0f;
+            int past = 0;
+            if (e < cnt) {
+                const float4 p = s_cand[e];
+                x = whole(p.x, k, qx), y = whole(p.y, k, qy), z = whole(p.z, k, qz);
+                const float n2 = x * x + y * y + z * z - reach2;
+                high = whole(n2, 1.0f / kBase, 0.0f), low = n2 - high * kBase;
+                past = __float2int_rz((p.x - P.gridMin.x) * P.gridDelta.x) - (cxa - 1) - srch;
+            }
+            constexpr uint32_t kOneHalf = 0x3c00u, kFarHalf = 0x7b53u;
+            uint4 *const col = reinterpret_cast<uint4 *>(s_col + lane * 8);
+            col[0] = make_uint4(half2_bits(x, y), half2_bits(z, high), half2_bits(low, kBase),
+                                past >= 0 ? kOneHalf | kFarHalf << 16 : kOneHalf);
+            col[1] = make_uint4(past >= 2 ? kFarHalf | kFarHalf << 16 : past >= 1 ? kFarHalf : 0u, 0u, 0u, 0u);
+            __syncwarp();
+            // column 2t + b of tile k is candidate 8t + 2k + b, so a lane's
+            // eight signs of a row are byte t of the row's mask word
+            uint2 b[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                b[k] = *reinterpret_cast<const uint2 *>(s_col + ((g >> 1) * 8 + 2 * k + (g & 1)) * 8 + 2 * t);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (!(h ? half1 : half0)) continue;
+                uint32_t m0 = 0, m1 = 0;
+#pragma unroll
+                for (int k = 3; k >= 0; k--) {
+                    float d[4];
+                    mma_16x8x16(d, a[2 * h], a[2 * h + 1], b[k]);
+                    m0 = __funnelshift_l(__float_as_uint(d[1]), m0, 1);
+                    m0 = __funnelshift_l(__float_as_uint(d[0]), m0, 1);
+                    m1 = __funnelshift_l(__float_as_uint(d[3]), m1, 1);
+                    m1 = __funnelshift_l(__float_as_uint(d[2]), m1, 1);
+                }
+                mb[(16 * h) * kMaskRow * 4] = (uint8_t)m0;
+                mb[(16 * h + 8) * kMaskRow * 4] = (uint8_t)m1;
+            }
+            __syncwarp();
+            if (cut) {   // leave each point the candidates of its own search block
+                uint32_t v = 0;
+                for (int k = 0; k <= span; k++) {
+                    const unsigned in = __ballot_sync(0xffffffffu, (uint32_t)(past + srch - k) < (uint32_t)srch);
+                    if (rel == k) v = in;
+                }
+                row[w] &= v;
+            }
+        }
+        __syncwarp();
+        if (mine) {
+            // the set bits in order, the lanes in step; a word without one is
+            // idled through (its record, one past the word, is in the buffer)
+            const int end = words - 1;
+            const float4 *from = s_cand;
+            uint32_t m = row[0];
+            int w = 0;
+            do {
+                const float4 p = from[__clz(__brev(m))];
+                visit(s, P, p, __float_as_uint(p.w), m != 0u);
+                m &= m - 1u;
+                if (m == 0u && w < end) {
+                    from += 32;
+                    m = row[++w];
+                }
+            } while (m != 0u || w < end);
+        }
+        __syncwarp();
+    }
+}
+
+// A point's results: its density, pair count and pair record.
+__device__ __forceinline__ void finish(const DevParams &P, const Sum &s, int i, bool active,
+                                       const float4 *__restrict__ veval, float *__restrict__ press,
+                                       uint32_t *__restrict__ hitcnt, float4 *__restrict__ pairdata) {
+    if (!active) {
+        press[i] = 0.0f;
+        hitcnt[i] = 0;
+        return;
+    }
+    float d = s.sum * P.pmass * P.poly6kern;
+    if (d == 0.0f) d = 1.0f;
+    press[i] = d;
+    hitcnt[i] = s.nh;
+    const float4 e = veval[i];
+    pairdata[2 * (size_t)i] = make_float4(s.p.x, s.p.y, s.p.z, d);
+    pairdata[2 * (size_t)i + 1] = make_float4(e.x, e.y, e.z, 0.0f);
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(kRowsMaxThreads, 1536 / kRowsMaxThreads)
+k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
+               const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
+               float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
+               float4 *__restrict__ pairdata) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const DevParams &P = BATCH ? T.params[T.point_scene[i]] : P0;
+    const uint32_t gc = gcell[i];
+    const bool active = gc != kUndef;
+    Sum s;
+    s.p = pos[i];
+    s.sum = 0.0f;
+    s.nh = 0;
+    s.next = hitlist + list_at(P, i, 0);
+    if (active) walk(P, s, gc, pos, off);
+    finish(P, s, i, active, veval, press, hitcnt, pairdata);
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(1024)
+k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
+          const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
+          float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
+          float4 *__restrict__ pairdata) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lane = lane_id();
+    if (i - (int)lane >= n) return;   // whole warp past n
+    uint32_t *s_warp = s_dyn + (threadIdx.x >> 5) * kWarpWords;
+    const uint32_t gc = (i < n) ? gcell[i] : kUndef;
+    const bool active = gc != kUndef;
+    const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
+    Sum s;
+    s.p = active ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    s.sum = 0.0f;
+    s.nh = 0;
+    s.next = hitlist + list_at(P, i, 0);
+    // consecutive points of one row of cells, at most two cells between
+    // neighbours and 16 cells in all, share a walk
+    const int cx = __float2int_rz((s.p.x - P.gridMin.x) * P.gridDelta.x);
+    const uint32_t row = active ? gc - (uint32_t)cx : kUndef;
+    const uint32_t prow = __shfl_up_sync(0xffffffffu, row, 1);
+    const int pcx = __shfl_up_sync(0xffffffffu, cx, 1);
+    const bool head = active && (lane == 0 || row != prow || cx - pcx > 2 || (cx >> 4) != (pcx >> 4));
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    unsigned heads = __ballot_sync(0xffffffffu, head);
+    if (__popc(heads) <= kMaxSegments) {
+        while (heads) {
+            const int h0 = __ffs(heads) - 1;
+            heads &= heads - 1u;
+            const unsigned upto = heads ? (1u << (__ffs(heads) - 1)) - 1u : 0xffffffffu;
+            const unsigned seg = act & upto & (0xffffffffu << h0);
+            const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + h0]] : P0;
+            segment(PS, s, seg, gc, cx, pos, off, s_warp);
+        }
+    } else if (active) {
+        walk(P, s, gc, pos, off);
+    }
+    if (i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
+}
+
+}  // namespace
+
+int fl_density_init() {
+    const int most = 32 * kWarpWords * (int)sizeof(uint32_t);
+    FL_CUDA_TRY(cudaFuncSetAttribute(k_density<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    FL_CUDA_TRY(cudaFuncSetAttribute(k_density<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return FL_OK;
+}
+
+int fl_density_block(const fl_system *s) { return s->blk_density ? s->blk_density : kDensityThreads; }
+
+int fl_launch_density(fl_system *s) {
+    if (s->n == 0) return FL_OK;
+    if (s->passes == FL_PASSES_POINT_PAIRS && s->D.prune && s->codes_valid) return fl_launch_density_pairs(s);
+    // Positions that have moved since the sort (phases called after an advance
+    // without a new one read them through the old grid) may be anywhere, or
+    // NaN: each point walks alone, as with gridSrch > 2 (in any scene).
+    const bool rows = !s->D.prune || !s->codes_valid;
+    const int bs = rows ? std::min(fl_density_block(s), kRowsMaxThreads) : fl_density_block(s);
+    const size_t smem = rows ? 0 : (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
+    auto kern = rows ? (s->batched ? k_density_rows<true> : k_density_rows<false>)
+                     : (s->batched ? k_density<true> : k_density<false>);
+    kern<<<blocks_for(s->n, bs), bs, smem, s->stream>>>(
+        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
+        s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
+    FL_LAUNCH_CHECK("density");
+    s->lists_valid = 1;
+    return FL_OK;
+}

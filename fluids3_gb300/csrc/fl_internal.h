@@ -119,7 +119,7 @@ struct fl_system {
     // band codes in pos.w while codes_valid is set. Rows 3-5: the same for
     // the lower face, filled only by the adjoint's rebuilt steps (sort mode 2)
     uint32_t *upbits;
-    int codes_valid;
+    int codes_valid;       // the positions are those of the last sort (with gridSrch 2, flags and codes too)
 
     // pairs found by the density pass, reused by the force pass while the
     // positions and grid are unchanged (lists_valid)
@@ -285,6 +285,9 @@ size_t fl_big_cells_cap(int max_points);
 // gather every field cur -> nxt through src (phase-API counting sort)
 int fl_launch_gather_all(fl_system *s);
 int fl_launch_band_codes(fl_system *s);
+// the density pass with pair lists and pair records (fl_density.cu)
+int fl_density_init();   // once per process is enough; outside any stream capture
+int fl_density_block(const fl_system *s);
 int fl_launch_density(fl_system *s);
 int fl_launch_force(fl_system *s);
 // slots [begin, end) (end < 0: n); both whole blocks of fl_force_block(s)

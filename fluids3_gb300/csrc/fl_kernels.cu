@@ -462,79 +462,6 @@ k_gather_all(int n, const uint32_t *__restrict__ src,
     gndx_o[s] = gndx[i];
 }
 
-constexpr int kDensityMaxThreads = 1024;
-
-// computePressure (fluids4.0/fluid_kernels.cu:112-149). FGRID is the
-// identity after a full sort (cu:83), so neighbour slots are read directly.
-// With LIST the slots of the pairs that pass 0 < d^2 < rd2 are recorded, in
-// visiting order, for the force pass (same positions, same test), together
-// with each point's pair record (position and density, evaluated velocity).
-template <bool PRUNE, bool LIST, bool BATCH>
-__global__ void __launch_bounds__(kDensityMaxThreads, 2)
-k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-          const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-          const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-          const float4 *__restrict__ veval, float *__restrict__ press, uint32_t *__restrict__ hitlist,
-          uint32_t *__restrict__ hitcnt, float4 *__restrict__ pairdata) {
-    // pruned: the lanes of a warp take points with the same lower-band bits,
-    // which decide the entries of the search block a point visits
-    extern __shared__ uint32_t s_dyn[];
-    const int i = PRUNE ? band_grouped_slot(n, pos, gcell, 3, s_dyn) : (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= n) return;
-    const DevParams &P = BATCH ? T.params[T.point_scene[i]] : P0;
-    const uint32_t gc = gcell[i];
-    if (gc == kUndef) {
-        press[i] = 0.0f;
-        if (LIST) hitcnt[i] = 0;
-        return;
-    }
-    const int base = (int)gc - P.nadj;
-    const float4 p = pos[i];
-    const uint32_t my_code = __float_as_uint(p.w);
-    float sum = 0.0f;
-    uint32_t nh = 0;
-    // Branch-free: every candidate's term is formed and a miss adds +0.0,
-    // which leaves the sum's bits unchanged (the sum starts at +0.0 and its
-    // terms are positive), so the sum is the reference's; the list store
-    // is predicated. Without the divergent branch the warp skips the
-    // convergence bookkeeping around it (6% faster than branching at 4M).
-    uint32_t *const lrow = hitlist + list_at(P, i, 0);
-    const uint32_t cap = (uint32_t)P.hcap;
-    const float rd2 = P.rd2, d2 = P.d2;
-    auto visit = [&](uint32_t j) {
-        const float4 q = pos[j];
-        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        const float dsq = dx * dx + dy * dy + dz * dz;
-        const bool hit = dsq < rd2 && dsq > 0.0f;
-        float t = (rd2 - dsq) * d2;
-        t = t * t * t;
-        sum += hit ? t : 0.0f;
-        if (LIST) {
-            if (hit && nh < cap) lrow[(size_t)nh * 32u] = j;
-            nh += hit ? 1u : 0u;
-        }
-    };
-    for (int c = 0; c < P.gridAdjCnt; c++) {
-        CandIter it;
-        cand_begin<PRUNE>(it, P, c, base + P.adj[c], my_code, true, off, cnt, upbits);
-        if (PRUNE && it.U == 0u) {   // the own cell: no flags to consult, every slot in order
-            for (uint32_t j = it.lo; j < it.hi; j++) visit(j);
-            continue;
-        }
-        uint32_t j;
-        while (cand_next<PRUNE>(it, P, upbits, j)) visit(j);
-    }
-    sum = sum * P.pmass * P.poly6kern;
-    if (sum == 0.0f) sum = 1.0f;
-    press[i] = sum;
-    if (LIST) {
-        hitcnt[i] = nh;
-        const float4 e = veval[i];
-        pairdata[2 * (size_t)i] = make_float4(p.x, p.y, p.z, sum);
-        pairdata[2 * (size_t)i + 1] = make_float4(e.x, e.y, e.z, 0.0f);
-    }
-}
-
 // computeForce (fluids4.0/fluid_kernels.cu:180-217) in two stages per warp:
 // lanes first walk their candidates with the cheap distance test and push
 // each hit's slot onto a per-thread list in shared memory; whenever some
@@ -1037,7 +964,7 @@ int fl_launch_sort_cells(fl_system *s, int mode, bool late) {
             s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits);
         FL_LAUNCH_CHECK("gather_sorted");
     }
-    s->codes_valid = s->D.prune;
+    s->codes_valid = 1;
     return FL_OK;
 }
 
@@ -1072,7 +999,7 @@ size_t fl_upbits_bytes(const fl_system *s) { return 3 * sizeof(uint32_t) * (size
 static bool use_prune(const fl_system *s) { return s->D.prune && s->codes_valid; }
 
 int fl_launch_band_codes(fl_system *s) {
-    if (!s->D.prune) { s->codes_valid = 0; return FL_OK; }
+    if (!s->D.prune) { s->codes_valid = 1; return FL_OK; }
     const int grid = blocks_for((long long)s->gcells, kThreads / 32);
     FL_CUDA_TRY(cudaMemsetAsync(s->upbits, 0, fl_upbits_bytes(s), s->stream));
     auto kern = s->batched ? k_band_codes<true> : k_band_codes<false>;
@@ -1080,24 +1007,6 @@ int fl_launch_band_codes(fl_system *s) {
                                           s->f[F_POS].cur<float4>(), s->upbits);
     FL_LAUNCH_CHECK("band_codes");
     s->codes_valid = 1;
-    return FL_OK;
-}
-
-template <bool BATCH>
-static auto density_kernel(bool prune) {
-    return prune ? k_density<true, true, BATCH> : k_density<false, true, BATCH>;
-}
-
-int fl_launch_density(fl_system *s) {
-    if (s->n == 0) return FL_OK;
-    if (s->passes == FL_PASSES_POINT_PAIRS && use_prune(s)) return fl_launch_density_pairs(s);
-    auto kern = s->batched ? density_kernel<true>(use_prune(s)) : density_kernel<false>(use_prune(s));
-    const int bs = s->blk_density ? s->blk_density : kThreads;
-    kern<<<blocks_for(s->n, bs), bs, grouping_smem(bs, kBandKeys), s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
-        s->upbits, s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
-    FL_LAUNCH_CHECK("density");
-    s->lists_valid = 1;
     return FL_OK;
 }
 
