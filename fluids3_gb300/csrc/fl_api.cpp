@@ -107,6 +107,8 @@ static void free_grid(fl_system *s) {
     s->tasks = nullptr;
     s->task_cap = 0;
     s->scan_ticket = nullptr;
+    s->tiles.counters = nullptr;
+    s->tiles_listed = 0;
     s->task_counters = nullptr;
     s->scan_status = nullptr;
 }
@@ -134,6 +136,7 @@ static int alloc_grid(fl_system *s) {
     s->scan_ticket = (uint32_t *)((char *)blk + s->grid_pad * sizeof(uint32_t));
     s->task_counters = s->scan_ticket + 1;   // same 256-byte slot as the ticket
     s->crowd_dev = s->scan_ticket + 4;       // cleared with it every step
+    s->tiles.counters = s->scan_ticket + 8;  // also
     s->scan_status = (uint64_t *)((char *)s->scan_ticket + 256);
     s->off = (uint32_t *)off;
     s->scan_epoch = 1;
@@ -161,6 +164,7 @@ static void free_all(fl_system *s) {
     cudaFree(s->cell_pre); cudaFree(s->rank_tmp); cudaFree(s->src); cudaFree(s->upbits);
     cudaFree(s->hitlist); cudaFree(s->hitcnt); cudaFree(s->pairdata);
     cudaFree(s->big_cells); cudaFree(s->big_count);
+    cudaFree(s->tiles.flag); cudaFree(s->tiles.list); cudaFree(s->over_tiles.list); cudaFree(s->over_tiles.counters);
     cudaFree(s->d_scenes); cudaFree(s->point_scene); cudaFree(s->cell_scene);
     free(s->scene_point_base); free(s->scene_n); free(s->scene_cell_base); free(s->scene_ncells);
     free(s->scene_params);
@@ -240,6 +244,11 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         s->D.upwords = (int)((np + 31) / 32 + 1);
         // rows 0-2: upper-band flags; rows 3-5: lower-band flags (adjoint only)
         if ((r = fl_dalloc((void **)&s->upbits, 2 * fl_upbits_bytes(s))) != FL_OK) break;
+        const size_t ntiles = (np + 31) / 32;
+        if ((r = fl_dalloc((void **)&s->tiles.flag, ntiles)) != FL_OK) break;
+        if ((r = fl_dalloc((void **)&s->tiles.list, 4 * ntiles)) != FL_OK) break;
+        if ((r = fl_dalloc((void **)&s->over_tiles.list, 4 * ntiles)) != FL_OK) break;
+        if ((r = fl_dalloc((void **)&s->over_tiles.counters, 256)) != FL_OK) break;
         s->D.hcap = kPairListCap;
         if ((r = fl_dalloc((void **)&s->hitlist, 4 * ((np + 31) / 32) * 32 * (size_t)kPairListCap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->hitcnt, 4 * np)) != FL_OK) break;
@@ -253,6 +262,7 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         }
         if ((r = fl_kernels_init(s)) != FL_OK) break;
         if ((r = fl_density_init()) != FL_OK) break;
+        if ((r = fl_crowd_init()) != FL_OK) break;
         if ((r = fl_cells_init(s)) != FL_OK) break;
         if ((r = fl_pairs_init()) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->dev_err, 256)) != FL_OK) break;
@@ -260,7 +270,8 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         if ((r = alloc_grid(s)) != FL_OK) break;
         if (cudaMemsetAsync(s->dev_err, 0, 256, s->stream) != cudaSuccess ||
             cudaMemsetAsync(s->time_dev, 0, 256, s->stream) != cudaSuccess ||
-            cudaMemsetAsync(s->big_count, 0, 256, s->stream) != cudaSuccess) {
+            cudaMemsetAsync(s->big_count, 0, 256, s->stream) != cudaSuccess ||
+            cudaMemsetAsync(s->over_tiles.counters, 0, 256, s->stream) != cudaSuccess) {
             r = fl_fail(FL_ERR_CUDA, "fl_create: memset failed");
             break;
         }
@@ -785,6 +796,7 @@ static int clear_grid(fl_system *s) {
     // InsertParticlesCUDA clears FGRIDCNT/FGRIDOFF (cpp:2336-2337); here one
     // memset clears the counts, the scan ticket and the scan descriptors.
     FL_CUDA_TRY(cudaMemsetAsync(s->cnt, 0, grid_block_bytes(s), s->stream));
+    s->tiles_listed = 0;
     return FL_OK;
 }
 

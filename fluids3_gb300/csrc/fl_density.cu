@@ -46,6 +46,7 @@ namespace {
 
 #include "fl_device.cuh"
 #include "fl_step.cuh"
+#include "fl_crowd.cuh"
 
 constexpr int kCap = 192;                       // candidates staged per round
 constexpr int kFill = kCap - 32;                // a round stops staging past this
@@ -62,16 +63,6 @@ constexpr float kFar = 6.0e4f;                  // times kBase: beyond any squar
 constexpr int kDensityThreads = 128;
 constexpr int kRowsMaxThreads = 256;
 
-__device__ __forceinline__ float warp_min(float v) {
-    float r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-__device__ __forceinline__ float warp_max(float v) {
-    float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
 __device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&h);
@@ -152,7 +143,7 @@ __device__ __forceinline__ void walk(const DevParams &P, Sum &s, uint32_t gc, co
 
 // The sums of the warp's points in `seg` (consecutive points of one row of
 // cells, a few cells apart at most). All lanes call it.
-__device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg, uint32_t gc, int cx,
+__device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg, uint32_t gc,
                                         const float4 *__restrict__ pos, const uint32_t *__restrict__ off,
                                         uint32_t *s_warp) {
     float4 *const s_cand = reinterpret_cast<float4 *>(s_warp);
@@ -162,7 +153,6 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
     const bool mine = (seg >> lane) & 1u;
     const int first = __ffs(seg) - 1, last = 31 - __clz(seg);
     const uint32_t ca = __shfl_sync(0xffffffffu, gc, first), cb = __shfl_sync(0xffffffffu, gc, last);
-    const int cxa = __shfl_sync(0xffffffffu, cx, first);
     constexpr int srch = 2, rows = 4;
     // the rows of the search block: lane r holds row r's slots [lo, hi)
     uint32_t lo = 0, hi = 0;
@@ -171,18 +161,14 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
         lo = off[(int)ca + at];
         hi = off[(int)cb + at + srch];
     }
-    const float px = __shfl_sync(0xffffffffu, s.p.x, first), py = __shfl_sync(0xffffffffu, s.p.y, first),
-                pz = __shfl_sync(0xffffffffu, s.p.z, first);
-    const float vx = mine ? s.p.x : px, vy = mine ? s.p.y : py, vz = mine ? s.p.z : pz;
-    const float lx = warp_min(vx), ux = warp_max(vx), ly = warp_min(vy), uy = warp_max(vy), lz = warp_min(vz),
-                uz = warp_max(vz);
-    const float ox = 0.5f * (lx + ux), oy = 0.5f * (ly + uy), oz = 0.5f * (lz + uz);
-    const float ex = fmaxf(ux - ox, ox - lx), ey = fmaxf(uy - oy, oy - ly), ez = fmaxf(uz - oz, oz - lz);
-    const float bx = ex + P.band, by = ey + P.band, bz = ez + P.band;   // a candidate's largest offset
+    const Box box = box_of(s.p, seg);
+    const float ox = box.ox, oy = box.oy, oz = box.oz;
+    const float bx = box.ex + P.band, by = box.ey + P.band, bz = box.ez + P.band;   // a candidate's largest offset
     // units: a distance between rounded points is off by at most sqrt(3) < 1.8
     const float k = kUnits / fmaxf(fmaxf(bx, by), bz);
     const float qx = -ox * k, qy = -oy * k, qz = -oz * k;
     const float reach = sqrtf(P.rd2) * k + 1.8f, reach2 = ceilf(reach * reach) + 4.0f;
+    const int cx = __float2int_rz((s.p.x - P.gridMin.x) * P.gridDelta.x), cxa = __shfl_sync(0xffffffffu, cx, first);
     const int rel = cx - cxa;   // the point's block starts this many cells into the rows
     const int span = __shfl_sync(0xffffffffu, rel, last);
     // With points of at most three cells the product also leaves each point
@@ -195,7 +181,7 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
     {   // row: -2 (x, y, z), kBase, 1, |x|^2 as (high, low), the cell
         float x = 0.0f, y = 0.0f, z = 0.0f, high = kFar, low = 0.0f;
         if (mine) {
-            x = whole(vx, k, qx), y = whole(vy, k, qy), z = whole(vz, k, qz);
+            x = whole(s.p.x, k, qx), y = whole(s.p.y, k, qy), z = whole(s.p.z, k, qz);
             const float n2 = x * x + y * y + z * z;
             high = whole(n2, 1.0f / kBase, 0.0f), low = n2 - high * kBase;
         }
@@ -208,6 +194,8 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
     uint2 a[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) a[q] = *reinterpret_cast<const uint2 *>(s_mask + (g + 8 * q) * 8 + 2 * t);
+    // cells along the row from the end of cell ca's block
+    const int past0 = cxa + 1;
     const bool half0 = (seg & 0xffffu) != 0, half1 = (seg >> 16) != 0;
 
     int r = -1;
@@ -252,7 +240,7 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
                 x = whole(p.x, k, qx), y = whole(p.y, k, qy), z = whole(p.z, k, qz);
                 const float n2 = x * x + y * y + z * z - reach2;
                 high = whole(n2, 1.0f / kBase, 0.0f), low = n2 - high * kBase;
-                past = __float2int_rz((p.x - P.gridMin.x) * P.gridDelta.x) - (cxa - 1) - srch;
+                past = __float2int_rz((p.x - P.gridMin.x) * P.gridDelta.x) - past0;
             }
             constexpr uint32_t kOneHalf = 0x3c00u, kFarHalf = 0x7b53u;
             uint4 *const col = reinterpret_cast<uint4 *>(s_col + lane * 8);
@@ -352,16 +340,117 @@ k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, co
     finish(P, s, i, active, veval, press, hitcnt, pairdata);
 }
 
+// A crowded tile, by a whole block (fl_crowd.cuh). Alone, its warp would walk
+// thousands of candidates in one chain: the density launch of 65,536 points
+// after 160 steps of a collapse (up to 4,967 pairs a point) took 1,063 us, now
+// 385; of 32,768 after 100 steps 174, now 119. Six blocks a multiprocessor
+// hide one another's waits (two: 580 us).
+constexpr int kCrowdSlots = 16;       // candidates a warp and round
+constexpr int kCrowdBlocksPerSm = 6;
+struct CrowdShared {              // per warp
+    float4 cand[2][kCrowdSlots];            // position, slot
+    float term[2][kCrowdSlots][32];         // per candidate and point
+    uint32_t hits[2][32];                   // per point: its pairs among the candidates
+    int kept[2];
+};
+static_assert(sizeof(CrowdShared) <= kWarpWords * sizeof(uint32_t), "a warp's shared memory holds its share");
+
+// A call, not inlined: the other tiles' code keeps its registers.
+template <bool BATCH>
+__device__ __noinline__ void crowded_tile(const DevParams &P0, const SceneTab &T, uint32_t tile, int n,
+                                             const float4 *__restrict__ pos, const uint32_t *__restrict__ gcell,
+                                             const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
+                                             float *__restrict__ press, uint32_t *__restrict__ hitlist,
+                                             uint32_t *__restrict__ hitcnt, float4 *__restrict__ pairdata,
+                                             uint32_t *s_dyn) {
+    const unsigned lane = lane_id();
+    const int warp = (int)(threadIdx.x >> 5), from = blockDim.x > 32 ? 1 : 0;   // the first evaluating warp
+    auto shared_of = [&](int w) -> CrowdShared & { return *reinterpret_cast<CrowdShared *>(s_dyn + w * kWarpWords); };
+    CrowdShared &own_sh = shared_of(warp);
+    const int i = (int)(tile * 32u + lane);
+    const uint32_t gc = (i < n) ? gcell[i] : kUndef;
+    const bool active = gc != kUndef;
+    const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
+    Sum s;
+    s.p = active ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    s.sum = 0.0f;
+    s.nh = 0;
+    s.next = hitlist + list_at(P, i, 0);
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    unsigned heads = segment_heads(gc, active);
+    while (heads) {
+        const unsigned seg = next_segment(heads, act);
+        const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + __ffs(seg) - 1]] : P0;
+        const Box box = box_of(s.p, seg);
+        const float bx = box.ex + PS.band, by = box.ey + PS.band, bz = box.ez + PS.band;
+        const float rd2 = PS.rd2, d2 = PS.d2;
+        crowd_segment<kCrowdSlots>(
+            PS, seg, gc, off, [&](bool ok, uint32_t j) { return ok ? pos[j] : make_float4(0.f, 0.f, 0.f, 0.f); },
+            [&](float4 q) { return fabsf(q.x - box.ox) <= bx && fabsf(q.y - box.oy) <= by && fabsf(q.z - box.oz) <= bz; },
+            [&](int buf, int e, uint32_t j, float4 q) { own_sh.cand[buf][e] = make_float4(q.x, q.y, q.z, __uint_as_float(j)); },
+            [&](int buf, int kept, RowRange own) {
+                uint32_t hits = 0;
+#pragma unroll 4
+                for (int e = 0; e < kept; e++) {
+                    const float4 q = own_sh.cand[buf][e];
+                    const float dx = s.p.x - q.x, dy = s.p.y - q.y, dz = s.p.z - q.z;
+                    const float dsq = dx * dx + dy * dy + dz * dz;
+                    const bool hit = dsq < rd2 && dsq > 0.0f && __float_as_uint(q.w) - own.lo < own.len;
+                    float t = (rd2 - dsq) * d2;
+                    t = t * t * t;
+                    own_sh.term[buf][e][lane] = hit ? t : 0.0f;
+                    hits |= (hit ? 1u : 0u) << e;
+                }
+                for (int e = kept; e & 3; e++) own_sh.term[buf][e][lane] = 0.0f;   // whole groups of four
+                own_sh.hits[buf][lane] = hits;
+                if (lane == 0) own_sh.kept[buf] = kept;
+            },
+            [&](int buf, int w) {
+                const CrowdShared &sh = shared_of(w + from);
+                const int kept = sh.kept[buf];
+                for (int e = 0; e < kept; e += 4) {   // a miss adds +0.0; four loads a round trip
+                    float t[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) t[u] = sh.term[buf][e + u][lane];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) s.sum += t[u];
+                }
+                uint32_t hits = sh.hits[buf][lane], k = s.nh;
+                s.nh += __popc(hits);
+                for (; hits && k < (uint32_t)PS.hcap; k++, s.next += 32, hits &= hits - 1u)
+                    *s.next = __float_as_uint(sh.cand[buf][__ffs(hits) - 1].w);
+            });
+    }
+    if (warp == 0 && i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
+}
+
+// The first `workers` blocks take the crowded tiles that the sort's gather
+// listed (tiles.flag, tiles.list; workers 0: none are set apart), the others
+// 32 slots a warp.
 template <bool BATCH>
 __global__ void __launch_bounds__(1024)
 k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
           const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
           float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
-          float4 *__restrict__ pairdata) {
+          float4 *__restrict__ pairdata, const CrowdTiles tiles, int workers) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((int)blockIdx.x < workers) {
+        __shared__ uint32_t s_next;
+        const uint32_t count = tiles.counters[0];
+        if (count == 0) return;
+        for (;;) {
+            if (threadIdx.x == 0) s_next = atomicAdd(&tiles.counters[1], 1u);
+            __syncthreads();
+            const uint32_t k = s_next;
+            __syncthreads();
+            if (k >= count) return;
+            crowded_tile<BATCH>(P0, T, tiles.list[k], n, pos, gcell, off, veval, press, hitlist, hitcnt, pairdata, s_dyn);
+        }
+    }
+    const int i = ((int)blockIdx.x - workers) * (int)blockDim.x + (int)threadIdx.x;
     const unsigned lane = lane_id();
     if (i - (int)lane >= n) return;   // whole warp past n
+    if (workers && tiles.flag[i >> 5]) return;
     uint32_t *s_warp = s_dyn + (threadIdx.x >> 5) * kWarpWords;
     const uint32_t gc = (i < n) ? gcell[i] : kUndef;
     const bool active = gc != kUndef;
@@ -371,23 +460,13 @@ k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const f
     s.sum = 0.0f;
     s.nh = 0;
     s.next = hitlist + list_at(P, i, 0);
-    // consecutive points of one row of cells, at most two cells between
-    // neighbours and 16 cells in all, share a walk
-    const int cx = __float2int_rz((s.p.x - P.gridMin.x) * P.gridDelta.x);
-    const uint32_t row = active ? gc - (uint32_t)cx : kUndef;
-    const uint32_t prow = __shfl_up_sync(0xffffffffu, row, 1);
-    const int pcx = __shfl_up_sync(0xffffffffu, cx, 1);
-    const bool head = active && (lane == 0 || row != prow || cx - pcx > 2 || (cx >> 4) != (pcx >> 4));
     const unsigned act = __ballot_sync(0xffffffffu, active);
-    unsigned heads = __ballot_sync(0xffffffffu, head);
+    unsigned heads = segment_heads(gc, active);
     if (__popc(heads) <= kMaxSegments) {
         while (heads) {
-            const int h0 = __ffs(heads) - 1;
-            heads &= heads - 1u;
-            const unsigned upto = heads ? (1u << (__ffs(heads) - 1)) - 1u : 0xffffffffu;
-            const unsigned seg = act & upto & (0xffffffffu << h0);
-            const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + h0]] : P0;
-            segment(PS, s, seg, gc, cx, pos, off, s_warp);
+            const unsigned seg = next_segment(heads, act);
+            const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + __ffs(seg) - 1]] : P0;
+            segment(PS, s, seg, gc, pos, off, s_warp);
         }
     } else if (active) {
         walk(P, s, gc, pos, off);
@@ -414,12 +493,21 @@ int fl_launch_density(fl_system *s) {
     // NaN: each point walks alone, as with gridSrch > 2 (in any scene).
     const bool rows = !s->D.prune || !s->codes_valid;
     const int bs = rows ? std::min(fl_density_block(s), kRowsMaxThreads) : fl_density_block(s);
-    const size_t smem = rows ? 0 : (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
-    auto kern = rows ? (s->batched ? k_density_rows<true> : k_density_rows<false>)
-                     : (s->batched ? k_density<true> : k_density<false>);
-    kern<<<blocks_for(s->n, bs), bs, smem, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-        s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
+    const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
+    if (rows) {
+        auto kern = s->batched ? k_density_rows<true> : k_density_rows<false>;
+        kern<<<blocks_for(s->n, bs), bs, 0, s->stream>>>(
+            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
+            s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
+    } else {
+        const int workers = s->tiles_listed ? std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32) : 0;
+        auto kern = s->batched ? k_density<true> : k_density<false>;
+        kern<<<workers + blocks_for(s->n, bs), bs, smem, s->stream>>>(
+            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
+            s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata,
+            s->tiles, workers);
+        s->tiles_listed = 0;   // the list is used up
+    }
     FL_LAUNCH_CHECK("density");
     s->lists_valid = 1;
     return FL_OK;

@@ -62,6 +62,14 @@ struct SceneTab {
     const uint16_t *cell_scene;
 };
 
+// Tiles (32 consecutive sorted slots) set apart for whole blocks because
+// their search blocks hold many points: a flag per tile, the list of those
+// set, and [count, ticket].
+struct CrowdTiles {
+    uint8_t *flag;
+    uint32_t *list, *counters;
+};
+
 // One particle field held twice in HBM. Gathers (the counting sort) and the
 // fused force+advance pass write the copy that is not live and then flip,
 // so no kernel overwrites a value that another thread may still read.
@@ -126,6 +134,12 @@ struct fl_system {
     uint32_t *big_cells;   // cell entries above 128 points, listed by the cell sort (fl_big_cells_cap)
     uint32_t *big_count;   // [0] their number, [1] k_sort_big's sign-off count (256 B slot, zeroed at creation)
     int num_sms;
+
+    // tiles whose search blocks are crowded: listed by the sort's gather for
+    // the density pass (counters in the scan ticket's slot, cleared with the
+    // counts), and by the force pass for its crowd kernel (which clears its own)
+    CrowdTiles tiles, over_tiles;
+    int tiles_listed;      // the gather's list is that of the current sort
 
     // cell tasks of the fused step's neighbour passes (fl_cells.cu): (first slot, cell entry)
     // per 64 slots of a cell, listed every step; counters in the scan
@@ -294,6 +308,9 @@ int fl_launch_force(fl_system *s);
 // threads, except end == n
 int fl_launch_force_advance(fl_system *s, float dt, int begin = 0, int end = -1, float *host_pos = nullptr);
 int fl_force_block(const fl_system *s);
+// force (and advance) of the tiles the force pass listed (fl_crowd.cu)
+int fl_crowd_init();   // as fl_density_init
+int fl_launch_force_crowd(fl_system *s, bool advance, float dt, float *host_pos);
 int fl_launch_advance(fl_system *s, float time, float dt, float ss);
 int fl_launch_pack3(fl_system *s, const float4 *src, float *dst, int n, cudaStream_t stream = nullptr);
 int fl_launch_set_time(fl_system *s, int slot, float value);

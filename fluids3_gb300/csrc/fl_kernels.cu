@@ -340,6 +340,13 @@ __device__ __forceinline__ CellCtx cell_ctx(const DevParams &P0, const SceneTab 
 // the canonical within-cell order). The 32 slots of a warp are one word of
 // each slot-flag row, so the warp stores the words whole: rows 0-2 the
 // upper-band flags (ROWS >= 1), rows 3-5 the lower-band flags (ROWS == 2).
+// A tile (warp) of gridSrch 2 whose points' search blocks hold kCrowdedBlock
+// points or more goes to the list the density pass's blocks share. At 1,024 a
+// warp alone takes about 50 us; a lower line (512, 768) sends tiles of a
+// merely dense fluid to the blocks, which test every candidate against every
+// point: 65,536 points after 64 steps 159 and 134 us against 87.
+constexpr uint32_t kCrowdedBlock = 1024;
+
 template <bool BATCH, int ROWS, bool LATE = false>
 __global__ void __launch_bounds__(kThreads)
 k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *__restrict__ src,
@@ -348,11 +355,11 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
                 const float4 *__restrict__ veval_in, const uint32_t *__restrict__ clr_in,
                 float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, float4 *__restrict__ veval_out,
                 uint32_t *__restrict__ clr_out, uint32_t *__restrict__ gcell_out,
-                uint32_t *__restrict__ gndx_out, uint32_t *__restrict__ upbits) {
+                uint32_t *__restrict__ gndx_out, uint32_t *__restrict__ upbits, const CrowdTiles tiles) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= (unsigned)n) return;   // whole warp past n
     const bool valid = s < n;
-    uint32_t code = 0, upwords = 0;
+    uint32_t code = 0, upwords = 0, cell = kUndef;
     if (valid) {
         const uint32_t i = src[s];
         const uint32_t c = cell_pre[i];
@@ -367,7 +374,8 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
             veval_out[s] = veval_in[i];
             clr_out[s] = clr_in[i];
         }
-        gcell_out[s] = (local == P.ncells) ? kUndef : c;
+        cell = (local == P.ncells) ? kUndef : c;
+        gcell_out[s] = cell;
         gndx_out[s] = (uint32_t)s - off[c];
         upwords = (uint32_t)P.upwords;
     }
@@ -379,6 +387,24 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
         for (int row = 0; row < 3 * ROWS; row++) {
             const unsigned b = __ballot_sync(0xffffffffu, valid && ((code >> row) & 1u));
             if (lane == 0) upbits[(size_t)row * upwords + word] = b;
+        }
+        // the tile's candidates: the larger search block of its first and last
+        // points' cells (lanes 0-3 the four rows of one, 4-7 of the other)
+        const unsigned act = __ballot_sync(0xffffffffu, cell != kUndef);
+        const int from = act ? (lane < 4 ? __ffs(act) - 1 : 31 - __clz(act)) : 0;
+        const uint32_t c = __shfl_sync(0xffffffffu, cell, from);
+        uint32_t m = 0;
+        if (act && lane < 8) {
+            const DevParams &P = BATCH ? T.params[T.cell_scene[c]] : P0;
+            const int at = (int)c - P.nadj + ((int)(lane >> 1 & 1u) * P.gridRes.z + (int)(lane & 1u)) * P.gridRes.x;
+            m = off[at + 2] - off[at];
+        }
+        m += __shfl_xor_sync(0xffffffffu, m, 1);
+        m += __shfl_xor_sync(0xffffffffu, m, 2);
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
+        if (lane == 0) {
+            tiles.flag[word] = m >= kCrowdedBlock;
+            if (m >= kCrowdedBlock) tiles.list[atomicAdd(&tiles.counters[0], 1u)] = (uint32_t)word;
         }
     }
 }
@@ -499,101 +525,69 @@ __device__ __forceinline__ void drain_hits(const DevParams &P, ForcePoint &fp, u
     nhits = 0;
 }
 
-// The force on point i (all 32 lanes of the warp must call this). With
-// LIST the pairs come from the density pass's list (every lane draining its
-// own list in step); a point whose pairs overflowed the list walks its
-// candidates again. Without LIST (no density pass since the last sort) the
-// warp walks and drains per-lane hit lists in shared memory.
-template <bool PRUNE, bool LIST>
-__device__ __forceinline__ float3 force_of(const DevParams &P, int i, bool active, uint32_t gc,
-                                           const float4 *__restrict__ pos,
-                                           const float4 *__restrict__ veval,
-                                           const float *__restrict__ press,
-                                           const uint32_t *__restrict__ off,
-                                           const uint32_t *__restrict__ cnt,
-                                           const uint32_t *__restrict__ upbits,
-                                           const uint32_t *__restrict__ hitlist,
-                                           const uint32_t *__restrict__ hitcnt,
-                                           const float4 *__restrict__ pairdata) {
-    ForcePoint fp;
-    fp.f = make_float3(0.0f, 0.0f, 0.0f);
-    uint32_t my_code = 0;
-    int base = 0;
-    if (active) {
-        fp.p = pos[i];
-        fp.vi = veval[i];
-        fp.di = press[i];
-        fp.pi = (fp.di - P.prest_dens) * P.pintstiff;
-        my_code = __float_as_uint(fp.p.w);
-        base = (int)gc - P.nadj;
+// The force on point i, whose data fp holds (all 32 lanes of the warp must
+// call this), from the density pass's pair lists. False: a point's pairs
+// overflowed its list, and the warp's slots are on the crowd kernel's list.
+__device__ __forceinline__ bool force_from_list(const DevParams &P, int i, uint32_t nh, ForcePoint &fp,
+                                                const uint32_t *__restrict__ hitlist,
+                                                const float4 *__restrict__ pairdata, const CrowdTiles &over) {
+    if (__any_sync(0xffffffffu, nh > (uint32_t)P.hcap)) {
+        if (lane_id() == 0) over.list[atomicAdd(&over.counters[0], 1u)] = (uint32_t)(i >> 5);
+        return false;
     }
-    if constexpr (LIST) {
-        // No shared memory here, so the whole unified L1 caches the
-        // neighbour reads. A lane whose list overflowed (rare with 128
-        // entries) walks its candidates and adds each pair as found, in the
-        // same order.
-        const uint32_t nh = active ? hitcnt[i] : 0u;
-        const bool over = nh > (uint32_t)P.hcap;
-        if (!__any_sync(0xffffffffu, over)) {
-            // Four pairs in flight: their records are all requested before
-            // the first of them is evaluated, and the next four list entries
-            // while they are, so the drain (bound by these dependent loads,
-            // not by arithmetic) waits one round trip per four pairs. Each
-            // point still adds its pairs in list order; a lane past its
-            // list's end adds +0.0, which leaves a force sum's bits unchanged
-            // (a sum that starts at +0.0 never becomes -0.0), so the adds
-            // need no branch.
-            const uint32_t most = __reduce_max_sync(0xffffffffu, nh);
-            uint32_t t = 0;
-            uint32_t jn[kPairsInFlight];
+    // Four pairs in flight: their records are all requested before the first
+    // of them is evaluated, and the next four list entries while they are, so
+    // the drain (bound by these dependent loads, not by arithmetic) waits one
+    // round trip per four pairs. Each point still adds its pairs in list
+    // order; a lane past its list's end adds +0.0, which leaves a force sum's
+    // bits unchanged (a sum that starts at +0.0 never becomes -0.0), so the
+    // adds need no branch. No shared memory here, so the whole unified L1
+    // caches the neighbour reads.
+    const uint32_t most = __reduce_max_sync(0xffffffffu, nh);
+    uint32_t t = 0;
+    uint32_t jn[kPairsInFlight];
 #pragma unroll
-            for (uint32_t k = 0; k < kPairsInFlight; k++) jn[k] = (k < nh) ? hitlist[list_at(P, i, k)] : 0u;
-            for (; t + kPairsInFlight <= most; t += kPairsInFlight) {
-                float4 q[kPairsInFlight], v[kPairsInFlight];
+    for (uint32_t k = 0; k < kPairsInFlight; k++) jn[k] = (k < nh) ? hitlist[list_at(P, i, k)] : 0u;
+    for (; t + kPairsInFlight <= most; t += kPairsInFlight) {
+        float4 q[kPairsInFlight], v[kPairsInFlight];
 #pragma unroll
-                for (uint32_t k = 0; k < kPairsInFlight; k++) {
-                    q[k] = make_float4(0.f, 0.f, 0.f, 1.f);
-                    v[k] = q[k];
-                    if (t + k < nh) {
-                        q[k] = pairdata[2 * (size_t)jn[k]];
-                        v[k] = pairdata[2 * (size_t)jn[k] + 1];
-                    }
-                }
-#pragma unroll
-                for (uint32_t k = 0; k < kPairsInFlight; k++) {
-                    const uint32_t tn = t + kPairsInFlight + k;
-                    jn[k] = (tn < nh) ? hitlist[list_at(P, i, tn)] : 0u;
-                }
-#pragma unroll
-                for (uint32_t k = 0; k < kPairsInFlight; k++) {
-                    const float3 tk = pair_term(P, fp.p, fp.pi, fp.vi, fp.di, q[k], v[k], q[k].w);
-                    const bool ok = t + k < nh;
-                    fp.f.x += ok ? tk.x : 0.0f;
-                    fp.f.y += ok ? tk.y : 0.0f;
-                    fp.f.z += ok ? tk.z : 0.0f;
-                }
-            }
-            for (; t < most; t++)
-                if (t < nh) add_pair_force_rec(P, fp, hitlist[list_at(P, i, t)], pairdata);
-            return fp.f;
-        }
-        if (!over) {
-            for (uint32_t t = 0; t < nh; t++) add_pair_force_rec(P, fp, hitlist[list_at(P, i, t)], pairdata);
-            return fp.f;
-        }
-        for (int c = 0; c < P.gridAdjCnt; c++) {
-            CandIter it;
-            cand_begin<PRUNE>(it, P, c, base + P.adj[c], my_code, true, off, cnt, upbits);
-            uint32_t j;
-            while (cand_next<PRUNE>(it, P, upbits, j)) {
-                const float4 q = pos[j];
-                const float dx = fp.p.x - q.x, dy = fp.p.y - q.y, dz = fp.p.z - q.z;
-                const float dsq = dx * dx + dy * dy + dz * dz;
-                if (dsq < P.rd2 && dsq > 0.0f) add_pair_force(P, fp, j, pos, veval, press);
+        for (uint32_t k = 0; k < kPairsInFlight; k++) {
+            q[k] = make_float4(0.f, 0.f, 0.f, 1.f);
+            v[k] = q[k];
+            if (t + k < nh) {
+                q[k] = pairdata[2 * (size_t)jn[k]];
+                v[k] = pairdata[2 * (size_t)jn[k] + 1];
             }
         }
-        return fp.f;
+#pragma unroll
+        for (uint32_t k = 0; k < kPairsInFlight; k++) {
+            const uint32_t tn = t + kPairsInFlight + k;
+            jn[k] = (tn < nh) ? hitlist[list_at(P, i, tn)] : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kPairsInFlight; k++) {
+            const float3 tk = pair_term(P, fp.p, fp.pi, fp.vi, fp.di, q[k], v[k], q[k].w);
+            const bool ok = t + k < nh;
+            fp.f.x += ok ? tk.x : 0.0f;
+            fp.f.y += ok ? tk.y : 0.0f;
+            fp.f.z += ok ? tk.z : 0.0f;
+        }
     }
+    for (; t < most; t++)
+        if (t < nh) add_pair_force_rec(P, fp, hitlist[list_at(P, i, t)], pairdata);
+    return true;
+}
+
+// Without pair lists (no density pass since the last sort) the warp walks
+// and drains per-lane hit lists in shared memory.
+template <bool PRUNE>
+__device__ __forceinline__ void force_by_walk(const DevParams &P, bool active, uint32_t gc, ForcePoint &fp,
+                                              const float4 *__restrict__ pos, const float4 *__restrict__ veval,
+                                              const float *__restrict__ press, const uint32_t *__restrict__ off,
+                                              const uint32_t *__restrict__ cnt,
+                                              const uint32_t *__restrict__ upbits) {
+    const uint32_t my_code = __float_as_uint(fp.p.w);
+    const int base = (int)gc - P.nadj;
     __shared__ uint32_t s_hits[kHitCap * kForceThreads];
     uint32_t *hits = s_hits + threadIdx.x;
     uint32_t nhits = 0;
@@ -615,7 +609,23 @@ __device__ __forceinline__ float3 force_of(const DevParams &P, int i, bool activ
         }
     }
     drain_hits(P, fp, nhits, hits, pos, veval, press);
-    return fp.f;
+}
+
+// Point i's data for its force.
+__device__ __forceinline__ ForcePoint force_point(const DevParams &P, int i, bool active,
+                                                  const float4 *__restrict__ pos, const float4 *__restrict__ veval,
+                                                  const float *__restrict__ press) {
+    ForcePoint fp;
+    fp.p = fp.vi = make_float4(0.f, 0.f, 0.f, 0.f);
+    fp.di = fp.pi = 0.0f;
+    fp.f = make_float3(0.0f, 0.0f, 0.0f);
+    if (active) {
+        fp.p = pos[i];
+        fp.vi = veval[i];
+        fp.di = press[i];
+        fp.pi = (fp.di - P.prest_dens) * P.pintstiff;
+    }
+    return fp;
 }
 
 template <bool PRUNE, bool LIST, bool BATCH>
@@ -625,14 +635,18 @@ k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const flo
         const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
         const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
         const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
-        const float4 *__restrict__ pairdata, float4 *__restrict__ force) {
+        const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ force) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
     const uint32_t gc = (i < n) ? gcell[i] : kUndef;
     const bool active = gc != kUndef;
-    const float3 f = force_of<PRUNE, LIST>(P, i, active, gc, pos, veval, press, off, cnt, upbits,
-                                           hitlist, hitcnt, pairdata);
-    if (i < n) force[i] = active ? make_float4(f.x, f.y, f.z, 0.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    ForcePoint fp = force_point(P, i, active, pos, veval, press);
+    if constexpr (LIST) {
+        if (!force_from_list(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+    } else {
+        force_by_walk<PRUNE>(P, active, gc, fp, pos, veval, press, off, cnt, upbits);
+    }
+    if (i < n) force[i] = f4(fp.f);
 }
 
 // advanceParticles (fluids4.0/fluid_kernels.cu:332-420), in place.
@@ -673,8 +687,8 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
                 const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
                 const uint32_t *__restrict__ upbits,
                 const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
-                const float4 *__restrict__ pairdata, float4 *__restrict__ vel, float4 *__restrict__ force,
-                float4 *__restrict__ pos_out, float4 *__restrict__ veval_out,
+                const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ vel,
+                float4 *__restrict__ force, float4 *__restrict__ pos_out, float4 *__restrict__ veval_out,
                 uint32_t *__restrict__ err, int base, float *__restrict__ host_pos) {
     // host_pos (fl_run_from_host): the new positions also go straight into
     // the caller's page-locked float3 array, in slot order, while the pass
@@ -685,33 +699,13 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
     const uint32_t gc = (i < n) ? gcell[i] : kUndef;
     const bool active = gc != kUndef;
-    const float3 f = force_of<PRUNE, LIST>(P, i, active, gc, pos_in, veval_in, press, off, cnt, upbits,
-                                           hitlist, hitcnt, pairdata);
-    if (i >= n) return;
-    if (!active) {
-        force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        pos_out[i] = make_float4(-1000.f, -1000.f, -1000.f, 0.f);
-        vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        veval_out[i] = veval_in[i];
-        if (host_pos) {
-            host_pos[3 * (size_t)i] = -1000.f;
-            host_pos[3 * (size_t)i + 1] = -1000.f;
-            host_pos[3 * (size_t)i + 2] = -1000.f;
-        }
-        return;
+    ForcePoint fp = force_point(P, i, active, pos_in, veval_in, press);
+    if constexpr (LIST) {
+        if (!force_from_list(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+    } else {
+        force_by_walk<PRUNE>(P, active, gc, fp, pos_in, veval_in, press, off, cnt, upbits);
     }
-    force[i] = f4(f);
-    float3 po, vo, eo;
-    advance_point(P, time, dt, P.sim_scale, f, xyz(pos_in[i]), xyz(vel[i]), xyz(veval_in[i]), po, vo, eo);
-    if (!(isfinite(po.x) && isfinite(po.y) && isfinite(po.z))) atomicOr(err, FL_DEV_NONFINITE);
-    pos_out[i] = f4(po);
-    vel[i] = f4(vo);
-    veval_out[i] = f4(eo);
-    if (host_pos) {
-        host_pos[3 * (size_t)i] = po.x;
-        host_pos[3 * (size_t)i + 1] = po.y;
-        host_pos[3 * (size_t)i + 2] = po.z;
-    }
+    if (i < n) store_step(P, time, dt, i, active, fp, vel, force, pos_out, veval_out, err, host_pos, veval_in);
 }
 
 // ---------------------------------------------------------------------------
@@ -961,8 +955,10 @@ int fl_launch_sort_cells(fl_system *s, int mode, bool late) {
             s->D, fl_scene_tab(s), s->n, s->src, s->cell_pre, s->off, s->f[F_POS].cur<float4>(),
             s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(), s->f[F_CLR].cur<uint32_t>(),
             s->f[F_POS].nxt<float4>(), s->f[F_VEL].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(),
-            s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits);
+            s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits,
+            s->tiles);
         FL_LAUNCH_CHECK("gather_sorted");
+        s->tiles_listed = rows > 0;
     }
     s->codes_valid = 1;
     return FL_OK;
@@ -1028,9 +1024,9 @@ int fl_launch_force(fl_system *s) {
     kern<<<blocks_for(s->n, bs), bs, 0, s->stream>>>(
         s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
         s->f[F_PRESS].cur<float>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits,
-        s->hitlist, s->hitcnt, s->pairdata, s->f[F_FORCE].cur<float4>());
+        s->hitlist, s->hitcnt, s->pairdata, s->over_tiles, s->f[F_FORCE].cur<float4>());
     FL_LAUNCH_CHECK("force");
-    return FL_OK;
+    return s->lists_valid ? fl_launch_force_crowd(s, false, 0.0f, nullptr) : FL_OK;
 }
 
 int fl_force_block(const fl_system *s) { return s->blk_force ? s->blk_force : kForceThreads; }
@@ -1048,11 +1044,11 @@ int fl_launch_force_advance(fl_system *s, float dt, int begin, int end, float *h
     kern<<<blocks_for(count > 0 ? count : 1, bs), bs, 0, s->stream>>>(
         s->D, fl_scene_tab(s), s->n, s->time_dev, s->time_slot, dt, s->f[F_POS].cur<float4>(),
         s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-        s->cnt, s->upbits, s->hitlist, s->hitcnt, s->pairdata,
+        s->cnt, s->upbits, s->hitlist, s->hitcnt, s->pairdata, s->over_tiles,
         s->f[F_VEL].cur<float4>(), s->f[F_FORCE].cur<float4>(),
         s->f[F_POS].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(), s->dev_err, begin, host_pos);
     FL_LAUNCH_CHECK("force_advance");
-    return FL_OK;
+    return s->lists_valid && s->n > 0 ? fl_launch_force_crowd(s, true, dt, host_pos) : FL_OK;
 }
 
 int fl_launch_advance(fl_system *s, float time, float dt, float ss) {

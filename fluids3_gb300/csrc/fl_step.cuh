@@ -152,3 +152,32 @@ __device__ __forceinline__ void advance_point(const DevParams &P, float time, fl
     const float dts = dt / ss;
     pos_o = make_float3(pos.x + vnext.x * dts, pos.y + vnext.y * dts, pos.z + vnext.z * dts);
 }
+
+// The end of the fused step for point i from its force: the force, then walls,
+// limits and leapfrog (or, out of range, parked at (-1000, -1000, -1000) with
+// zero velocity, cu:339-342). host_pos (fl_run_from_host) also gets the new
+// position, packed float x3.
+__device__ __forceinline__ void store_step(const DevParams &P, float time, float dt, int i, bool active,
+                                           const ForcePoint &fp, float4 *__restrict__ vel, float4 *__restrict__ force,
+                                           float4 *__restrict__ pos_out, float4 *__restrict__ veval_out,
+                                           uint32_t *__restrict__ err, float *__restrict__ host_pos,
+                                           const float4 *__restrict__ veval_in) {
+    float3 po = make_float3(-1000.f, -1000.f, -1000.f), vo = make_float3(0.f, 0.f, 0.f);
+    if (active) {
+        force[i] = f4(fp.f);
+        float3 eo;
+        advance_point(P, time, dt, P.sim_scale, fp.f, xyz(fp.p), xyz(vel[i]), xyz(fp.vi), po, vo, eo);
+        if (!(isfinite(po.x) && isfinite(po.y) && isfinite(po.z))) atomicOr(err, FL_DEV_NONFINITE);
+        veval_out[i] = f4(eo);
+    } else {
+        force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        veval_out[i] = veval_in[i];
+    }
+    pos_out[i] = f4(po);
+    vel[i] = f4(vo);
+    if (host_pos) {
+        host_pos[3 * (size_t)i] = po.x;
+        host_pos[3 * (size_t)i + 1] = po.y;
+        host_pos[3 * (size_t)i + 2] = po.z;
+    }
+}
