@@ -83,6 +83,26 @@ __device__ __forceinline__ void mma_16x8x16(float (&d)[4], uint2 r0, uint2 r1, u
         : "r"(r0.x), "r"(r1.x), "r"(r0.y), "r"(r1.y), "r"(b.x), "r"(b.y), "f"(0.0f));
 }
 
+// What a pair needs of the parameters: from the launch's constants, or (BATCH)
+// held here, not read through the scene table for every pair.
+template <bool BATCH>
+struct PairParams {
+    const DevParams &P;
+    __device__ explicit PairParams(const DevParams &p) : P(p) {}
+    __device__ float rd2() const { return P.rd2; }
+    __device__ float d2() const { return P.d2; }
+    __device__ uint32_t cap() const { return (uint32_t)P.hcap; }
+};
+template <>
+struct PairParams<true> {
+    float r, d;
+    uint32_t c;
+    __device__ explicit PairParams(const DevParams &p) : r(p.rd2), d(p.d2), c((uint32_t)p.hcap) {}
+    __device__ float rd2() const { return r; }
+    __device__ float d2() const { return d; }
+    __device__ uint32_t cap() const { return c; }
+};
+
 // One point's running sum and pair list.
 struct Sum {
     float4 p;
@@ -96,17 +116,18 @@ struct Sum {
 // bits unchanged (it starts at +0.0 and its terms are positive). The list
 // store is predicated by hand: compiled as a branch it cost 25 instructions
 // per candidate, a quarter of the pass.
-__device__ __forceinline__ void visit(Sum &s, const DevParams &P, float4 q, uint32_t j, bool on) {
+template <bool BATCH>
+__device__ __forceinline__ void visit(Sum &s, const PairParams<BATCH> &c, float4 q, uint32_t j, bool on) {
     float dx2, dy2;
     const uint64_t dxy = sub2(pk2(s.p.x, s.p.y), pk2(q.x, q.y));
     const float dz = s.p.z - q.z;
     up2(mul2(dxy, dxy), dx2, dy2);
     const float dsq = dx2 + dy2 + dz * dz;
-    const bool hit = on && dsq < P.rd2 && dsq > 0.0f;
-    float t = (P.rd2 - dsq) * P.d2;
+    const bool hit = on && dsq < c.rd2() && dsq > 0.0f;
+    float t = (c.rd2() - dsq) * c.d2();
     t = t * t * t;
     s.sum += hit ? t : 0.0f;
-    const uint32_t cap = hit ? (uint32_t)P.hcap : 0u;
+    const uint32_t cap = hit ? c.cap() : 0u;
     asm volatile("{\n.reg .pred p;\nsetp.lt.u32 p, %2, %3;\n@p st.global.u32 [%0], %1;\n}" ::"l"(s.next), "r"(j),
                  "r"(s.nh), "r"(cap));
     s.next += hit ? 32 : 0;
@@ -116,8 +137,10 @@ __device__ __forceinline__ void visit(Sum &s, const DevParams &P, float4 q, uint
 // One point by itself: every slot of its search block, kAhead positions
 // requested before the first of them is used.
 constexpr uint32_t kAhead = 4;
+template <bool BATCH>
 __device__ __forceinline__ void walk(const DevParams &P, Sum &s, uint32_t gc, const float4 *__restrict__ pos,
                                      const uint32_t *__restrict__ off) {
+    const PairParams<BATCH> pp(P);
     const int srch = P.gridSrch, rows = srch * srch;
     const uint32_t *at = off + ((int)gc - P.nadj);
     uint32_t j = at[0], j1 = at[srch];
@@ -133,7 +156,7 @@ __device__ __forceinline__ void walk(const DevParams &P, Sum &s, uint32_t gc, co
 #pragma unroll
             for (uint32_t k = 0; k < kAhead; k++) q[k] = pos[min(j + k, j1 - 1u)];
 #pragma unroll
-            for (uint32_t k = 0; k < kAhead; k++) visit(s, P, q[k], j + k, j + k < j1);
+            for (uint32_t k = 0; k < kAhead; k++) visit(s, pp, q[k], j + k, j + k < j1);
         }
         if (r >= rows) break;
         j = nj;
@@ -143,6 +166,7 @@ __device__ __forceinline__ void walk(const DevParams &P, Sum &s, uint32_t gc, co
 
 // The sums of the warp's points in `seg` (consecutive points of one row of
 // cells, a few cells apart at most). All lanes call it.
+template <bool BATCH>
 __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg, uint32_t gc,
                                         const float4 *__restrict__ pos, const uint32_t *__restrict__ off,
                                         uint32_t *s_warp) {
@@ -169,6 +193,7 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
     const float qx = -ox * k, qy = -oy * k, qz = -oz * k;
     const float reach = sqrtf(P.rd2) * k + 1.8f, reach2 = ceilf(reach * reach) + 4.0f;
     const int cx = __float2int_rz((s.p.x - P.gridMin.x) * P.gridDelta.x), cxa = __shfl_sync(0xffffffffu, cx, first);
+    const PairParams<BATCH> pp(P);
     const int rel = cx - cxa;   // the point's block starts this many cells into the rows
     const int span = __shfl_sync(0xffffffffu, rel, last);
     // With points of at most three cells the product also leaves each point
@@ -290,7 +315,7 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
             int w = 0;
             do {
                 const float4 p = from[__clz(__brev(m))];
-                visit(s, P, p, __float_as_uint(p.w), m != 0u);
+                visit(s, pp, p, __float_as_uint(p.w), m != 0u);
                 m &= m - 1u;
                 if (m == 0u && w < end) {
                     from += 32;
@@ -336,7 +361,7 @@ k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, co
     s.sum = 0.0f;
     s.nh = 0;
     s.next = hitlist + list_at(P, i, 0);
-    if (active) walk(P, s, gc, pos, off);
+    if (active) walk<BATCH>(P, s, gc, pos, off);
     finish(P, s, i, active, veval, press, hitcnt, pairdata);
 }
 
@@ -466,10 +491,10 @@ k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const f
         while (heads) {
             const unsigned seg = next_segment(heads, act);
             const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + __ffs(seg) - 1]] : P0;
-            segment(PS, s, seg, gc, pos, off, s_warp);
+            segment<BATCH>(PS, s, seg, gc, pos, off, s_warp);
         }
     } else if (active) {
-        walk(P, s, gc, pos, off);
+        walk<BATCH>(P, s, gc, pos, off);
     }
     if (i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
 }
