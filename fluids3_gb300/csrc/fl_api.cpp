@@ -887,23 +887,43 @@ static int record(fl_system *s, TimingState *t, int k) {
     return FL_OK;
 }
 
-// The cell-task passes (fl_cells.cu) need the pruned search (gridSrch 2 in
-// every scene) with band codes from this step's sort. A recording tape keeps
-// the per-point passes (its hooks keep each step's pair lists).
+// Whether steps count as cell-task steps (fl_passes_steps,
+// fl_neighbour_passes_in_use): by mode, or with FL_PASSES_AUTO while a cell is
+// crowded.
 static bool cells_selected(const fl_system *s) {
     return s->passes == FL_PASSES_CELL_TASKS || (s->passes == FL_PASSES_AUTO && s->auto_cells);
 }
 
+static int passes_of_step(const fl_system *s, bool taped) {
+    return cells_selected(s) && s->D.prune && !taped && s->n > 0 ? 1 : 0;
+}
+
+// With FL_PASSES_AUTO the cell-task kernels (fl_cells.cu) run from
+// kCellTasksMin points; below, the per-point kernels, whose crowded tiles are
+// shared by whole blocks (fl_crowd.cuh): there are too few crowded cells to
+// fill the chip with a warp each. Density + force, collapsing dam break, us
+// (crowded tiles shared | cell tasks), after 90, 110 and 140 steps:
+// 65,536 points 375 | 725, 490 | 1,096, 601 | 2,105; 262,144: 695 | 609,
+// 1,299 | 1,928, 3,109 | 4,197; 524,288: 1,169 | 881, 1,631 | 1,635,
+// 4,911 | 5,179; 1,048,576: 1,848 | 1,354, 2,691 | 1,754, 5,704 | 4,434.
+constexpr int kCellTasksMin = 1 << 19;
+
+static bool cell_kernels(const fl_system *s) {
+    return s->passes == FL_PASSES_CELL_TASKS || (cells_selected(s) && s->n >= kCellTasksMin);
+}
+
+// They need the pruned search (gridSrch 2 in every scene) with band codes from
+// this step's sort. A recording tape keeps the per-point passes (its hooks
+// keep each step's pair lists).
 static bool use_cell_passes(const fl_system *s, bool taped) {
-    return cells_selected(s) && s->D.prune && s->codes_valid && !taped && s->n > 0;
+    return cell_kernels(s) && s->D.prune && s->codes_valid && !taped && s->n > 0;
 }
 
 // FL_PASSES_AUTO: measured on GB300 (4M-point wave tank, 10-step runs as it
-// clumps, the largest cell read after each run), the cell tasks take 1.19x
+// clumps, the largest cell read after each run), the cell tasks took 1.19x
 // the per-point step time by a largest cell of 489, 1.04x at 581, 0.91x at
 // 691 and 0.75-0.86x from 789 to 14,935 points (1.69x at the start, 61).
-// The cells grow during a run, so the switch sits a little below where the
-// run-end figures cross. Every step's sort records the
+// Every step's sort records the
 // largest in-range cell above 128 points and sends it to page-locked host
 // memory; the next call reads whatever copy has arrived (a step or two
 // old, no wait) and switches with hysteresis. The passes give identical
@@ -966,8 +986,7 @@ static int run_step(fl_system *s, TimingState *t) {
     FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
     const bool cells = use_cell_passes(s, taped);
-    s->last_step_cells = cells;
-    if (!s->capturing) s->passes_steps[cells ? 1 : 0]++;
+    if (!s->capturing) s->passes_steps[passes_of_step(s, taped)]++;
     if (cells) FL_TRY(fl_launch_make_tasks(s));
     FL_TRY(record(s, t, 4));
     FL_TRY(cells ? fl_launch_density_cells(s) : fl_launch_density(s));
@@ -1058,8 +1077,7 @@ static int run_step_late(fl_system *s, const float *vel3, const float *veval3, c
     FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
     const bool cells = use_cell_passes(s, false);
-    s->last_step_cells = cells;
-    s->passes_steps[cells ? 1 : 0]++;
+    s->passes_steps[passes_of_step(s, false)]++;
     if (cells) FL_TRY(fl_launch_make_tasks(s));
     FL_TRY(cells ? fl_launch_density_cells(s) : fl_launch_density(s));
     FL_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_late, 0));
@@ -1183,8 +1201,7 @@ static int capture_pair(fl_system *s) {
         return fl_fail(FL_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
     s->graph_steps = 2;
-    s->graph_cells = (int)cells_selected(s);
-    s->graph_ran_cells = s->last_step_cells;
+    s->graph_cells = (int)cell_kernels(s);
     for (int k = 0; k < F_COUNT; k++) s->graph_live[k] = live[k];
     return FL_OK;
 }
@@ -1219,12 +1236,12 @@ static int run_steps_graph(fl_system *s, int nsteps) {
     update_auto(s);
     const int pairs = nsteps / 2;
     if (pairs > 0) {
-        bool match = s->graph_exec != nullptr && s->graph_cells == (int)cells_selected(s);
+        bool match = s->graph_exec != nullptr && s->graph_cells == (int)cell_kernels(s);
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
         FL_TRY(begin_run(s));
         for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));
-        s->passes_steps[s->graph_ran_cells ? 1 : 0] += 2 * (int64_t)pairs;
+        s->passes_steps[passes_of_step(s, false)] += 2 * (int64_t)pairs;
         s->time_host_valid = 0;   // the device slot now holds the time
         s->have_insert = 0;
         s->have_offsets = 1;
