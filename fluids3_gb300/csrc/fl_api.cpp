@@ -164,7 +164,7 @@ static void free_all(fl_system *s) {
     cudaFree(s->cell_pre); cudaFree(s->rank_tmp); cudaFree(s->src); cudaFree(s->upbits);
     cudaFree(s->hitlist); cudaFree(s->hitcnt); cudaFree(s->pairdata);
     cudaFree(s->big_cells); cudaFree(s->big_count);
-    cudaFree(s->tiles.flag); cudaFree(s->tiles.list); cudaFree(s->over_tiles.list); cudaFree(s->over_tiles.counters);
+    cudaFree(s->tiles.kind); cudaFree(s->tiles.list); cudaFree(s->over_tiles.list); cudaFree(s->over_tiles.counters);
     cudaFree(s->d_scenes); cudaFree(s->point_scene); cudaFree(s->cell_scene);
     free(s->scene_point_base); free(s->scene_n); free(s->scene_cell_base); free(s->scene_ncells);
     free(s->scene_params);
@@ -245,7 +245,8 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         // rows 0-2: upper-band flags; rows 3-5: lower-band flags (adjoint only)
         if ((r = fl_dalloc((void **)&s->upbits, 2 * fl_upbits_bytes(s))) != FL_OK) break;
         const size_t ntiles = (np + 31) / 32;
-        if ((r = fl_dalloc((void **)&s->tiles.flag, ntiles)) != FL_OK) break;
+        s->tiles.room = s->over_tiles.room = (uint32_t)ntiles;
+        if ((r = fl_dalloc((void **)&s->tiles.kind, ntiles)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->tiles.list, 4 * ntiles)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->over_tiles.list, 4 * ntiles)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->over_tiles.counters, 256)) != FL_OK) break;

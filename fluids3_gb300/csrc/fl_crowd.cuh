@@ -11,6 +11,17 @@
 // tiles go to whichever block is free.
 #pragma once
 
+// Puts a tile on its class's list (one lane calls it).
+__device__ __forceinline__ void list_tile(const CrowdTiles &t, uint32_t tile, bool packed) {
+    const uint32_t k = atomicAdd(&t.counters[packed ? 1 : 0], 1u);
+    t.list[packed ? t.room - 1u - k : k] = tile;
+}
+
+// The k-th of `packed` packed tiles followed by the crowded ones.
+__device__ __forceinline__ uint32_t tile_at(const CrowdTiles &t, uint32_t k, uint32_t packed) {
+    return t.list[k < packed ? t.room - 1u - k : k - packed];
+}
+
 // The lane's search-block row: slots [lo, lo + len).
 struct RowRange {
     uint32_t lo, len;

@@ -62,12 +62,13 @@ struct SceneTab {
     const uint16_t *cell_scene;
 };
 
-// Tiles (32 consecutive sorted slots) set apart for whole blocks because
-// their search blocks hold many points: a flag per tile, the list of those
-// set, and [count, ticket].
+// Tiles (32 consecutive sorted slots) whose search blocks are crowded (1) or
+// packed (2): a class per tile, and a list of each class in one array of
+// `room` entries, the crowded from its front, the packed from its back.
 struct CrowdTiles {
-    uint8_t *flag;
-    uint32_t *list, *counters;
+    uint8_t *kind;
+    uint32_t *list, *counters;   // counters: crowded tiles, packed ones, two tickets, blocks done
+    uint32_t room;
 };
 
 // One particle field held twice in HBM. Gathers (the counting sort) and the

@@ -19,6 +19,7 @@ namespace {
 
 #include "fl_device.cuh"
 #include "fl_step.cuh"
+#include "fl_crowd.cuh"
 
 // insertParticles (fluids4.0/fluid_kernels.cu:22-53) with warp-aggregated
 // counting: a run of consecutive lanes that land in the same cell elects its
@@ -345,7 +346,9 @@ __device__ __forceinline__ CellCtx cell_ctx(const DevParams &P0, const SceneTab 
 // warp alone takes about 50 us; a lower line (512, 768) sends tiles of a
 // merely dense fluid to the blocks, which test every candidate against every
 // point: 65,536 points after 64 steps 159 and 134 us against 87.
-constexpr uint32_t kCrowdedBlock = 1024;
+// Packed tiles (kPackedBlock) are listed apart: where crowded tiles are many
+// and left to a warp each, one of 16,000 candidates would outlast the rest.
+constexpr uint32_t kCrowdedBlock = 1024, kPackedBlock = 4096;
 
 template <bool BATCH, int ROWS, bool LATE = false>
 __global__ void __launch_bounds__(kThreads)
@@ -403,8 +406,8 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
         m += __shfl_xor_sync(0xffffffffu, m, 2);
         m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
         if (lane == 0) {
-            tiles.flag[word] = m >= kCrowdedBlock;
-            if (m >= kCrowdedBlock) tiles.list[atomicAdd(&tiles.counters[0], 1u)] = (uint32_t)word;
+            tiles.kind[word] = m >= kPackedBlock ? 2 : m >= kCrowdedBlock ? 1 : 0;
+            if (m >= kCrowdedBlock) list_tile(tiles, (uint32_t)word, m >= kPackedBlock);
         }
     }
 }
@@ -499,6 +502,7 @@ k_gather_all(int n, const uint32_t *__restrict__ src,
 constexpr int kForceThreads = 128;
 constexpr int kHitCap = 32;
 constexpr uint32_t kPairsInFlight = 4;   // pairs of a list drained per round of loads
+constexpr uint32_t kPackedPairs = 1024;  // pairs of a point that put its tile on the crowd kernel's packed list
 
 // Neighbour j's data from the field arrays.
 __device__ __forceinline__ void add_pair_force(const DevParams &P, ForcePoint &fp, uint32_t j,
@@ -532,7 +536,8 @@ __device__ __forceinline__ bool force_from_list(const DevParams &P, int i, uint3
                                                 const uint32_t *__restrict__ hitlist,
                                                 const float4 *__restrict__ pairdata, const CrowdTiles &over) {
     if (__any_sync(0xffffffffu, nh > (uint32_t)P.hcap)) {
-        if (lane_id() == 0) over.list[atomicAdd(&over.counters[0], 1u)] = (uint32_t)(i >> 5);
+        const bool packed = __any_sync(0xffffffffu, nh >= kPackedPairs);
+        if (lane_id() == 0) list_tile(over, (uint32_t)(i >> 5), packed);
         return false;
     }
     // Four pairs in flight: their records are all requested before the first
