@@ -101,15 +101,11 @@ int fl_dalloc(void **p, size_t bytes) {
 static void free_grid(fl_system *s) {
     cudaFree(s->cnt);
     cudaFree(s->off);
-    cudaFree(s->tasks);
     s->codes_valid = 0;
     s->cnt = s->off = nullptr;
-    s->tasks = nullptr;
-    s->task_cap = 0;
     s->scan_ticket = nullptr;
     s->tiles.counters = nullptr;
     s->tiles_listed = 0;
-    s->task_counters = nullptr;
     s->scan_status = nullptr;
 }
 
@@ -124,18 +120,13 @@ static int alloc_grid(fl_system *s) {
     const size_t entries = (size_t)s->gcells;
     s->scan_tiles = (int)((entries + tile - 1) / tile);
     s->grid_pad = (size_t)s->scan_tiles * tile;
-    void *blk = nullptr, *off = nullptr, *tasks = nullptr;
+    void *blk = nullptr, *off = nullptr;
     FL_TRY(fl_dalloc(&blk, grid_block_bytes(s)));
     int r = fl_dalloc(&off, s->grid_pad * sizeof(uint32_t));
     if (r != FL_OK) { cudaFree(blk); return r; }
-    s->task_cap = fl_task_cap(s->max_points, s->gcells);
-    r = fl_dalloc(&tasks, s->task_cap * sizeof(uint2));
-    if (r != FL_OK) { cudaFree(blk); cudaFree(off); return r; }
-    s->tasks = (uint2 *)tasks;
     s->cnt = (uint32_t *)blk;
     s->scan_ticket = (uint32_t *)((char *)blk + s->grid_pad * sizeof(uint32_t));
-    s->task_counters = s->scan_ticket + 1;   // same 256-byte slot as the ticket
-    s->crowd_dev = s->scan_ticket + 4;       // cleared with it every step
+    s->crowd_dev = s->scan_ticket + 4;       // same 256-byte slot as the ticket: cleared with it every step
     s->tiles.counters = s->scan_ticket + 8;  // also
     s->scan_status = (uint64_t *)((char *)s->scan_ticket + 256);
     s->off = (uint32_t *)off;
@@ -202,7 +193,7 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
     FL_TRY(check_derived(p));
     fl_system *s = (fl_system *)calloc(1, sizeof(fl_system));
     if (!s) return fl_fail(FL_ERR_NOMEM, "fl_create: host allocation failed");
-    s->passes = FL_PASSES_AUTO;   // per-point passes, cell tasks once cells crowd (fl_set_neighbour_passes)
+    s->passes = FL_PASSES_AUTO;
     int r = FL_OK;
     do {
         if (cudaGetDevice(&s->device) != cudaSuccess) {
@@ -264,7 +255,6 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         if ((r = fl_kernels_init(s)) != FL_OK) break;
         if ((r = fl_density_init()) != FL_OK) break;
         if ((r = fl_crowd_init()) != FL_OK) break;
-        if ((r = fl_cells_init(s)) != FL_OK) break;
         if ((r = fl_pairs_init()) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->dev_err, 256)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->time_dev, 256)) != FL_OK) break;
@@ -335,7 +325,6 @@ extern "C" int fl_batch_create(const fl_params *params, const int *counts, int n
         s->P = params[0];
         s->batched = 1;
         s->nscenes = nscenes;
-        if ((r = fl_cells_init(s)) != FL_OK) break;
         if ((r = fl_pairs_init()) != FL_OK) break;
         free_grid(s);
         s->ncells = (int)ncell;
@@ -899,36 +888,11 @@ static int passes_of_step(const fl_system *s, bool taped) {
     return cells_selected(s) && s->D.prune && !taped && s->n > 0 ? 1 : 0;
 }
 
-// With FL_PASSES_AUTO the cell-task kernels (fl_cells.cu) run from
-// kCellTasksMin points; below, the per-point kernels, whose crowded tiles are
-// shared by whole blocks (fl_crowd.cuh): there are too few crowded cells to
-// fill the chip with a warp each. Density + force, collapsing dam break, us
-// (crowded tiles shared | cell tasks), after 90, 110 and 140 steps:
-// 65,536 points 375 | 725, 490 | 1,096, 601 | 2,105; 262,144: 695 | 609,
-// 1,299 | 1,928, 3,109 | 4,197; 524,288: 1,169 | 881, 1,631 | 1,635,
-// 4,911 | 5,179; 1,048,576: 1,848 | 1,354, 2,691 | 1,754, 5,704 | 4,434.
-constexpr int kCellTasksMin = 1 << 19;
-
-static bool cell_kernels(const fl_system *s) {
-    return s->passes == FL_PASSES_CELL_TASKS || (cells_selected(s) && s->n >= kCellTasksMin);
-}
-
-// They need the pruned search (gridSrch 2 in every scene) with band codes from
-// this step's sort. A recording tape keeps the per-point passes (its hooks
-// keep each step's pair lists).
-static bool use_cell_passes(const fl_system *s, bool taped) {
-    return cell_kernels(s) && s->D.prune && s->codes_valid && !taped && s->n > 0;
-}
-
-// FL_PASSES_AUTO: measured on GB300 (4M-point wave tank, 10-step runs as it
-// clumps, the largest cell read after each run), the cell tasks took 1.19x
-// the per-point step time by a largest cell of 489, 1.04x at 581, 0.91x at
-// 691 and 0.75-0.86x from 789 to 14,935 points (1.69x at the start, 61).
-// Every step's sort records the
-// largest in-range cell above 128 points and sends it to page-locked host
-// memory; the next call reads whatever copy has arrived (a step or two
-// old, no wait) and switches with hysteresis. The passes give identical
-// results, so when the switch happens changes no result.
+// FL_PASSES_AUTO: every step's sort records the largest in-range cell above
+// 128 points and sends it to page-locked host memory; the next call reads
+// whatever copy has arrived (a step or two old, no wait) and switches what
+// the steps count as, with hysteresis. The kernels are the same either way:
+// crowded tiles are found, and shared between warps, in every step.
 constexpr uint32_t kAutoCellsOn = 512, kAutoCellsOff = 384;
 
 static void update_auto(fl_system *s) {
@@ -986,13 +950,11 @@ static int run_step(fl_system *s, TimingState *t) {
     FL_TRY(fl_launch_sort_cells(s, 1));
     FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
-    const bool cells = use_cell_passes(s, taped);
     if (!s->capturing) s->passes_steps[passes_of_step(s, taped)]++;
-    if (cells) FL_TRY(fl_launch_make_tasks(s));
     FL_TRY(record(s, t, 4));
-    FL_TRY(cells ? fl_launch_density_cells(s) : fl_launch_density(s));
+    FL_TRY(fl_launch_density(s));
     FL_TRY(record(s, t, 5));
-    FL_TRY(cells ? fl_launch_force_cells(s, s->P.dt, nullptr) : fl_launch_force_advance(s, s->P.dt));
+    FL_TRY(fl_launch_force_advance(s, s->P.dt));
     FL_TRY(join_crowd(s));
     flip(s, F_POS); flip(s, F_VEVAL);
     s->codes_valid = 0;
@@ -1019,11 +981,6 @@ int fl_rebuild_grid(fl_system *s) {
 
 int fl_recompute_step(fl_system *s) {
     FL_TRY(fl_rebuild_grid(s));
-    if (use_cell_passes(s, false)) {   // the cell-task density, writing the same pair lists
-        FL_TRY(fl_launch_make_tasks(s));
-        FL_TRY(fl_launch_density_cells(s, true));
-        return FL_OK;
-    }
     FL_TRY(fl_launch_density(s));
     return FL_OK;
 }
@@ -1077,21 +1034,13 @@ static int run_step_late(fl_system *s, const float *vel3, const float *veval3, c
     FL_TRY(fl_launch_sort_cells(s, 1, true));
     FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
-    const bool cells = use_cell_passes(s, false);
     s->passes_steps[passes_of_step(s, false)]++;
-    if (cells) FL_TRY(fl_launch_make_tasks(s));
-    FL_TRY(cells ? fl_launch_density_cells(s) : fl_launch_density(s));
+    FL_TRY(fl_launch_density(s));
     FL_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_late, 0));
     FL_TRY(fl_launch_gather_late(s, vel3, veval3, clr));
-    if (cells) {
-        // the force pass also writes the new positions into the caller's
-        // page-locked array as it goes (no separate readback)
-        FL_TRY(fl_launch_force_cells(s, s->P.dt, pos_out ? (float *)mapped_device_ptr(pos_out) : nullptr));
-    } else {
-        // the force pass writes the new positions into the caller's
-        // page-locked array as it goes (no separate readback)
-        FL_TRY(fl_launch_force_advance(s, s->P.dt, 0, -1, pos_out ? (float *)mapped_device_ptr(pos_out) : nullptr));
-    }
+    // the force pass writes the new positions into the caller's page-locked
+    // array as it goes (no separate readback)
+    FL_TRY(fl_launch_force_advance(s, s->P.dt, 0, -1, pos_out ? (float *)mapped_device_ptr(pos_out) : nullptr));
     FL_TRY(join_crowd(s));
     flip(s, F_POS); flip(s, F_VEVAL);
     s->codes_valid = 0;
@@ -1202,7 +1151,6 @@ static int capture_pair(fl_system *s) {
         return fl_fail(FL_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
     s->graph_steps = 2;
-    s->graph_cells = (int)cell_kernels(s);
     for (int k = 0; k < F_COUNT; k++) s->graph_live[k] = live[k];
     return FL_OK;
 }
@@ -1237,7 +1185,7 @@ static int run_steps_graph(fl_system *s, int nsteps) {
     update_auto(s);
     const int pairs = nsteps / 2;
     if (pairs > 0) {
-        bool match = s->graph_exec != nullptr && s->graph_cells == (int)cell_kernels(s);
+        bool match = s->graph_exec != nullptr;
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
         FL_TRY(begin_run(s));

@@ -249,7 +249,7 @@ __device__ __forceinline__ void sign_off(const CrowdTiles &t) {
 // The tiles of the classes with few (below), a block per tile. `ends`: no
 // k_force_alone follows.
 template <bool BATCH, bool ADVANCE>
-__global__ void __launch_bounds__(kCrowdThreads, BATCH ? 2 : 1)
+__global__ void __launch_bounds__(kCrowdThreads, BATCH ? 2 : 0)
 k_force_crowd(const __grid_constant__ DevParams P0, const SceneTab T, int n, const __grid_constant__ ForceArgs a,
               uint32_t line, bool ends) {
     extern __shared__ __align__(16) uint8_t s_dyn[];

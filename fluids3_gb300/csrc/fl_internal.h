@@ -142,15 +142,8 @@ struct fl_system {
     CrowdTiles tiles, over_tiles;
     int tiles_listed;      // the gather's list is that of the current sort
 
-    // cell tasks of the fused step's neighbour passes (fl_cells.cu): (first slot, cell entry)
-    // per 64 slots of a cell, listed every step; counters in the scan
-    // ticket's slot (cleared with the counts)
-    uint2 *tasks;
-    size_t task_cap;
-    uint32_t *task_counters;
     int passes;            // FL_PASSES_*: the neighbour passes of the fused step
     int auto_cells;        // FL_PASSES_AUTO: a cell is crowded (hysteresis state)
-    int graph_cells;       // the captured step pair runs the cell tasks
     int capturing;         // run_step is being captured into the step-pair graph
     int64_t passes_steps[2]; // fused steps issued with the per-point passes / the cell tasks
     uint32_t *crowd_dev;   // largest in-range cell above 128 points, this step (0: none)
@@ -158,7 +151,6 @@ struct fl_system {
     uint32_t *crowd_host;  // page-locked [count, epoch], sent after each step's sort
     uint32_t auto_epoch;   // host: the current state's epoch
     int adj_revmode;       // FL_REVERSE_*: how the adjoint finds its reverse pair lists
-    int cells_grid[2];     // blocks of the cell-task density and force passes (all resident)
 
     uint32_t *hitlist;     // ceil(N/32) * hcap * 32 entries
     uint32_t *hitcnt;      // per point
@@ -324,19 +316,8 @@ int fl_conservation_chunks(int max_scene_points);
 int fl_launch_conservation(fl_system *s, const int *sbase, const int *sn, int nchunks, double *partial);
 int fl_launch_sample_volume(fl_system *s, const int res[3], const float bmin[3], const float bmax[3],
                             float scalar, float gausskern, float h2, float *out);
-// cell-task passes of the fused step (fl_cells.cu)
-size_t fl_task_cap(int max_points, int gcells);
-int fl_cells_init(fl_system *s);   // after num_sms and batched are set
-int fl_launch_make_tasks(fl_system *s);
-// densities and pair records, plus the force pass's hit masks or (lists) the
-// per-point pair lists and counts in the per-point pass's layout
-int fl_launch_density_cells(fl_system *s, bool lists = false);
 int fl_launch_density_pairs(fl_system *s);
 int fl_pairs_init();   // once per process is enough; outside any stream capture
-// force + advance over the tasks from the hit masks; host_pos (a
-// device-usable pointer to page-locked host memory, or null) also receives
-// the new positions as float x3
-int fl_launch_force_cells(fl_system *s, float dt, float *host_pos);
 size_t fl_scan_tile();
 size_t fl_upbits_bytes(const fl_system *s);
 size_t fl_scan_scratch_bytes(int ntiles);

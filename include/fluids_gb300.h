@@ -335,26 +335,22 @@ int fl_set_launch_shapes(fl_system *s, const int *shapes);
 
 /* Which neighbour passes the fused step (fl_run, fl_run_steps,
  * fl_run_from_host) uses; all give bit-identical densities, forces and
- * states. FL_PASSES_PER_POINT (the faster step while cells are small): one thread
- * per point walks its own search block (fluids4.0/fluid_kernels.cu:112-149
- * as written) and records its pair list, which the force pass drains.
- * FL_PASSES_CELL_TASKS: one warp per 64 points of a cell walks their shared
- * search block once, in lockstep, staged in shared memory, recording hit
- * masks; the force pass walks the block again and evaluates the hits
- * pair-parallel. Used where the pruned search applies (gridSrch 2 in every
- * scene) and no tape is recording; the phase entry points and recording
- * tapes always use the per-point passes. FL_PASSES_POINT_PAIRS: the
- * per-point passes, except that where the pruned search applies one thread
- * walks the search block once for two points of a cell with the same
- * lower-band bits (which visit the same candidates in the same order); this
- * one holds for every density pass of the system (fused step, phase entry
- * points, tapes). FL_PASSES_AUTO (the default): the per-point passes until
- * the largest in-range cell reaches 512 points, the cell tasks from then
- * until it falls below 384 (each step's sort records the largest cell; a
- * fused-step call acts on the last value that has reached the host, a
- * step or two old). No counterpart in the reference (which has only the
- * per-point walk). fl_neighbour_passes returns the mode set;
- * fl_neighbour_passes_in_use the passes the next fused step takes
+ * states. FL_PASSES_PER_POINT, FL_PASSES_CELL_TASKS and FL_PASSES_AUTO (the
+ * default) run the same kernels: each point's density and pair list from a
+ * walk that 32 consecutive slots share, its force from the list, and crowded
+ * tiles of slots shared between warps wherever a step has them. The three
+ * differ in what their steps count as (fl_passes_steps): with FL_PASSES_AUTO
+ * as per-point steps until the largest in-range cell reaches 512 points, as
+ * cell-task steps from then until it falls below 384 (each step's sort records
+ * the largest cell; a fused-step call acts on the last value that has reached
+ * the host, a step or two old); steps of a search with gridSrch other than 2
+ * and taped steps always count as per-point steps. FL_PASSES_POINT_PAIRS:
+ * where gridSrch is 2, one thread walks the search block once for two points
+ * of a cell with the same lower-band bits (which visit the same candidates in
+ * the same order); this one holds for every density pass of the system (fused
+ * step, phase entry points, tapes). No counterpart in the reference (which has
+ * only the per-point walk). fl_neighbour_passes returns the mode set;
+ * fl_neighbour_passes_in_use what the next fused step counts as
  * (FL_PASSES_AUTO resolved with the latest count on the host: after
  * fl_sync, the last step's). */
 #define FL_PASSES_PER_POINT   0
@@ -364,8 +360,8 @@ int fl_set_launch_shapes(fl_system *s, const int *shapes);
 int fl_set_neighbour_passes(fl_system *s, int mode);
 int fl_neighbour_passes(const fl_system *s);
 int fl_neighbour_passes_in_use(fl_system *s);
-/* Fused steps issued since creation with the per-point passes (counts[0])
- * and with the cell tasks (counts[1]) -- what FL_PASSES_AUTO chose. */
+/* Fused steps issued since creation that counted as per-point steps
+ * (counts[0]) and as cell-task steps (counts[1]). */
 int fl_passes_steps(const fl_system *s, int64_t *counts);
 
 /* Wait for the system stream; returns FL_ERR_DEVICE if a kernel raised the
