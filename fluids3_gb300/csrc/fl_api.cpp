@@ -171,8 +171,6 @@ static void free_all(fl_system *s) {
         if (s->ev[k]) cudaEventDestroy(s->ev[k]);
     if (s->ev_early) cudaEventDestroy(s->ev_early);
     if (s->ev_late) cudaEventDestroy(s->ev_late);
-    if (s->ev_crowd) cudaEventDestroy(s->ev_crowd);
-    if (s->ev_crowd_done) cudaEventDestroy(s->ev_crowd_done);
     for (int k = 0; k < 2; k++)
         if (s->ev_auto[k]) cudaEventDestroy(s->ev_auto[k]);
     cudaFree(s->crowd_epoch);
@@ -210,6 +208,10 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
             break;
         }
         s->crowd_host[0] = s->crowd_host[1] = 0;
+        if (cudaHostGetDevicePointer(&s->crowd_report, s->crowd_host, 0) != cudaSuccess) {
+            r = fl_fail(FL_ERR_CUDA, "fl_create: page-locked memory is not mapped");
+            break;
+        }
         if ((r = fl_dalloc((void **)&s->crowd_epoch, 256)) != FL_OK) break;
         if (cudaMemset(s->crowd_epoch, 0, 256) != cudaSuccess) {
             r = fl_fail(FL_ERR_CUDA, "fl_create: memset failed");
@@ -803,7 +805,7 @@ extern "C" int fl_insert_particles(fl_system *s, uint32_t *gcell, uint32_t *gndx
     FL_TRY(clear_grid(s));
     FL_TRY(fl_launch_insert(s, s->f[F_GCELL].cur<uint32_t>()));
     // canonical gndx: offsets, arrival-order index scatter, per-cell sort
-    FL_TRY(fl_launch_scan(s, s->gcells, 0));
+    FL_TRY(fl_launch_scan(s, s->gcells));
     FL_TRY(fl_launch_scatter_index(s));
     FL_TRY(fl_launch_sort_cells(s, 0));
     s->codes_valid = 0;
@@ -821,7 +823,7 @@ extern "C" int fl_prefix_sum_cells(fl_system *s, uint32_t *goff, int zero_offset
     if (!s) return fl_fail(FL_ERR_ARG, "fl_prefix_sum_cells: null system");
     fl_tape_touch(s);
     if (!s->have_insert) return fl_fail(FL_ERR_STATE, "fl_prefix_sum_cells before fl_insert_particles");
-    FL_TRY(fl_launch_scan(s, s->gcells, 1));
+    // (the insert has scanned the counts already, for the within-cell ranks)
     s->have_offsets = 1;
     s->offsets_inclusive = zero_offsets ? 0 : 1;
     if (goff) FL_TRY(fl_get_buffer(s, FL_FGRIDOFF, goff, 4 * (size_t)s->ncells));
@@ -838,7 +840,6 @@ extern "C" int fl_counting_sort_full(fl_system *s, float *ppos) {
     FL_TRY(fl_launch_gather_all(s));
     for (int k = 0; k < F_COUNT; k++) flip(s, k);
     s->lists_valid = 0;
-    FL_TRY(fl_launch_band_codes(s));
     s->have_grid = 1;
     s->have_insert = 0;   // the pre-sort cell list no longer matches the order
     if (ppos) FL_TRY(fl_get_buffer(s, FL_FPOS, ppos, 12 * (size_t)s->n));
@@ -913,26 +914,6 @@ static int reset_auto(fl_system *s) {
     return fl_launch_set_word(s, s->crowd_epoch, s->auto_epoch);
 }
 
-// After the sort: the count and the epoch go to the host on the side stream,
-// off the step's critical path; join_crowd makes the step's end wait for
-// them (the next step's memset clears the count).
-static int send_crowd(fl_system *s) {
-    if (s->passes != FL_PASSES_AUTO || !s->crowd_host) return FL_OK;
-    FL_CUDA_TRY(cudaEventRecord(s->ev_crowd, s->stream));
-    FL_CUDA_TRY(cudaStreamWaitEvent(s->side, s->ev_crowd, 0));
-    FL_CUDA_TRY(cudaMemcpyAsync(s->crowd_host, s->crowd_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->side));
-    FL_CUDA_TRY(cudaMemcpyAsync(s->crowd_host + 1, s->crowd_epoch, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                s->side));
-    FL_CUDA_TRY(cudaEventRecord(s->ev_crowd_done, s->side));
-    return FL_OK;
-}
-
-static int join_crowd(fl_system *s) {
-    if (s->passes != FL_PASSES_AUTO || !s->crowd_host) return FL_OK;
-    FL_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_crowd_done, 0));
-    return FL_OK;
-}
-
 static int run_step(fl_system *s, TimingState *t) {
     // InsertParticles, PrefixSumCells, CountingSortFull, ComputePressure,
     // ComputeForce + Advance (cpp:507-515) as eight launches (the sort is a
@@ -943,19 +924,17 @@ static int run_step(fl_system *s, TimingState *t) {
     FL_TRY(clear_grid(s));
     FL_TRY(fl_launch_insert(s, nullptr));
     FL_TRY(record(s, t, 1));
-    FL_TRY(fl_launch_scan(s, s->gcells, 0));
+    FL_TRY(fl_launch_scan(s, s->gcells));
     FL_TRY(record(s, t, 2));
     FL_TRY(fl_launch_scatter_index(s));
     FL_TRY(record(s, t, 3));
     FL_TRY(fl_launch_sort_cells(s, 1));
-    FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
     if (!s->capturing) s->passes_steps[passes_of_step(s, taped)]++;
     FL_TRY(record(s, t, 4));
     FL_TRY(fl_launch_density(s));
     FL_TRY(record(s, t, 5));
     FL_TRY(fl_launch_force_advance(s, s->P.dt));
-    FL_TRY(join_crowd(s));
     flip(s, F_POS); flip(s, F_VEVAL);
     s->codes_valid = 0;
     s->lists_valid = 0;
@@ -971,7 +950,7 @@ int fl_step_fused(fl_system *s) { return run_step(s, nullptr); }
 int fl_rebuild_grid(fl_system *s) {
     FL_TRY(clear_grid(s));
     FL_TRY(fl_launch_insert(s, nullptr));
-    FL_TRY(fl_launch_scan(s, s->gcells, 0));
+    FL_TRY(fl_launch_scan(s, s->gcells));
     FL_TRY(fl_launch_scatter_index(s));
     FL_TRY(fl_launch_sort_cells(s, 2));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
@@ -1000,18 +979,9 @@ static TimingState *active_timing(fl_system *s) {
     return t;
 }
 
-static int begin_run(fl_system *s) {
-    if (!s->time_host_valid) return FL_OK;
-    // host time is authoritative: publish it to the slot the next step reads
-    // (as a kernel argument: a copy from pageable host memory could make the
-    // host wait for the stream)
-    return fl_launch_set_time(s, s->time_slot, s->time);
-}
-
 extern "C" int fl_run(fl_system *s) {
     if (!s) return fl_fail(FL_ERR_ARG, "fl_run: null system");
     update_auto(s);
-    FL_TRY(begin_run(s));
     FL_TRY(run_step(s, active_timing(s)));
     if (s->time_host_valid) s->time += s->P.dt;   // AdvanceTime (cpp:529), same float add
     s->have_insert = 0;
@@ -1029,10 +999,9 @@ static int run_step_late(fl_system *s, const float *vel3, const float *veval3, c
                          float *pos_out) {
     FL_TRY(clear_grid(s));
     FL_TRY(fl_launch_insert(s, nullptr));
-    FL_TRY(fl_launch_scan(s, s->gcells, 0));
+    FL_TRY(fl_launch_scan(s, s->gcells));
     FL_TRY(fl_launch_scatter_index(s));
     FL_TRY(fl_launch_sort_cells(s, 1, true));
-    FL_TRY(send_crowd(s));
     flip(s, F_POS); flip(s, F_VEL); flip(s, F_VEVAL); flip(s, F_CLR); flip(s, F_GCELL); flip(s, F_GNDX);
     s->passes_steps[passes_of_step(s, false)]++;
     FL_TRY(fl_launch_density(s));
@@ -1041,7 +1010,6 @@ static int run_step_late(fl_system *s, const float *vel3, const float *veval3, c
     // the force pass writes the new positions into the caller's page-locked
     // array as it goes (no separate readback)
     FL_TRY(fl_launch_force_advance(s, s->P.dt, 0, -1, pos_out ? (float *)mapped_device_ptr(pos_out) : nullptr));
-    FL_TRY(join_crowd(s));
     flip(s, F_POS); flip(s, F_VEVAL);
     s->codes_valid = 0;
     s->lists_valid = 0;
@@ -1053,8 +1021,6 @@ static int ensure_side(fl_system *s) {
     if (!s->side) FL_CUDA_TRY(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));   // the input copies
     if (!s->ev_early) FL_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_early, cudaEventDisableTiming));
     if (!s->ev_late) FL_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_late, cudaEventDisableTiming));
-    if (!s->ev_crowd) FL_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_crowd, cudaEventDisableTiming));
-    if (!s->ev_crowd_done) FL_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_crowd_done, cudaEventDisableTiming));
     for (int k = 0; k < 2; k++)
         if (!s->ev_auto[k]) FL_CUDA_TRY(cudaEventCreateWithFlags(&s->ev_auto[k], cudaEventDisableTiming));
     return FL_OK;
@@ -1110,7 +1076,6 @@ extern "C" int fl_run_from_host(fl_system *s, int n, const float *pos, const flo
     if (clr) FL_CUDA_TRY(cudaMemcpyAsync(stage_clr, clr, 4 * (size_t)n, cudaMemcpyHostToDevice, s->side));
     FL_CUDA_TRY(cudaEventRecord(s->ev_late, s->side));
     fl_reset_progress(s);
-    FL_TRY(begin_run(s));
     const int r = run_step_late(s, stage_vel, stage_vev, stage_clr, pos_out);
     // the host arrays are the caller's again once the step (and the
     // input copies on the side stream) are done
@@ -1157,9 +1122,10 @@ static int capture_pair(fl_system *s) {
 
 static int run_steps_graph(fl_system *s, int nsteps);
 
-// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps, each
-// chunk's passes chosen from the counts of the chunk two before it (waited
-// for, so one chunk stays queued and the GPU never idles).
+// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps. What a
+// chunk's steps count as comes from the counts of the chunk two before it, the
+// second chunk's from the first two steps (waited for, while the steps queued
+// after them keep the GPU busy).
 constexpr int kAutoChunk = 32;
 
 extern "C" int fl_run_steps(fl_system *s, int nsteps) {
@@ -1173,8 +1139,13 @@ extern "C" int fl_run_steps(fl_system *s, int nsteps) {
     int left = nsteps;
     for (int k = 0; left > 0; k++) {
         const int c = left < kAutoChunk ? left : kAutoChunk;
-        if (k >= 2) FL_CUDA_TRY(cudaEventSynchronize(s->ev_auto[k & 1]));
-        FL_TRY(run_steps_graph(s, c));
+        if (k == 0) {
+            FL_TRY(run_steps_graph(s, 2));
+            FL_CUDA_TRY(cudaEventRecord(s->ev_auto[1], s->stream));
+        } else {
+            FL_CUDA_TRY(cudaEventSynchronize(s->ev_auto[k & 1]));
+        }
+        FL_TRY(run_steps_graph(s, k == 0 ? c - 2 : c));
         FL_CUDA_TRY(cudaEventRecord(s->ev_auto[k & 1], s->stream));
         left -= c;
     }
@@ -1188,8 +1159,7 @@ static int run_steps_graph(fl_system *s, int nsteps) {
         bool match = s->graph_exec != nullptr;
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
-        FL_TRY(begin_run(s));
-        for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));
+            for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));
         s->passes_steps[passes_of_step(s, false)] += 2 * (int64_t)pairs;
         s->time_host_valid = 0;   // the device slot now holds the time
         s->have_insert = 0;
@@ -1224,12 +1194,9 @@ static int save_slot(fl_system *s, int slot) {
         for (int k = 0; k < F_COUNT; k++) FL_TRY(fl_dalloc(&s->ckpt[slot][k], s->f[k].esz * np));
         FL_TRY(fl_dalloc((void **)&s->ckpt_time[slot], 256));
     }
-    for (int k = 0; k < F_COUNT; k++)
-        if (s->n > 0)
-            FL_CUDA_TRY(cudaMemcpyAsync(s->ckpt[slot][k], s->f[k].cur<void>(), s->f[k].esz * (size_t)s->n,
-                                        cudaMemcpyDeviceToDevice, s->stream));
-    FL_CUDA_TRY(cudaMemcpyAsync(s->ckpt_time[slot], s->time_dev + s->time_slot, sizeof(float),
-                                cudaMemcpyDeviceToDevice, s->stream));
+    void *live[F_COUNT];
+    for (int k = 0; k < F_COUNT; k++) live[k] = s->f[k].cur<void>();
+    FL_TRY(fl_launch_copy_state(s, s->n, live, s->ckpt[slot], s->time_dev + s->time_slot, s->ckpt_time[slot], false));
     s->ckpt_n[slot] = s->n;
     s->ckpt_host_time[slot] = s->time;
     s->ckpt_host_valid[slot] = s->time_host_valid;
@@ -1245,13 +1212,11 @@ extern "C" int fl_checkpoint_restore(fl_system *s, int slot) {
 
 static int restore_slot(fl_system *s, int slot) {
     s->n = s->ckpt_n[slot];
-    FL_TRY(reset_auto(s));
-    for (int k = 0; k < F_COUNT; k++)
-        if (s->n > 0)
-            FL_CUDA_TRY(cudaMemcpyAsync(s->f[k].cur<void>(), s->ckpt[slot][k], s->f[k].esz * (size_t)s->n,
-                                        cudaMemcpyDeviceToDevice, s->stream));
-    FL_CUDA_TRY(cudaMemcpyAsync(s->time_dev + s->time_slot, s->ckpt_time[slot], sizeof(float),
-                                cudaMemcpyDeviceToDevice, s->stream));
+    s->auto_cells = 0;   // as reset_auto, its word in the same launch
+    s->auto_epoch++;
+    void *live[F_COUNT];
+    for (int k = 0; k < F_COUNT; k++) live[k] = s->f[k].cur<void>();
+    FL_TRY(fl_launch_copy_state(s, s->n, s->ckpt[slot], live, s->ckpt_time[slot], s->time_dev + s->time_slot, true));
     s->time = s->ckpt_host_time[slot];
     s->time_host_valid = s->ckpt_host_valid[slot];
     fl_reset_progress(s);

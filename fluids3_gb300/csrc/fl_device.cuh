@@ -57,24 +57,9 @@ __device__ __forceinline__ uint32_t band_code(const DevParams &P, int c, float4 
 }
 
 // Upper-band flags of the sorted slots, one bit per slot and axis:
-// upbits[axis * upwords + (slot >> 5)] bit (slot & 31). Published by the
-// 32 lanes of a warp for 32 consecutive slots base + lane (all lanes call).
-// The adjoint's rebuilt steps also publish the lower-band flags (code bits
-// 3-5) into rows 3-5 the same way (upbits + 3 * upwords, `code >> 3`).
-__device__ __forceinline__ void publish_upbits(const DevParams &P, uint32_t *upbits, uint32_t base,
-                                               uint32_t code, bool valid) {
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t w0 = base >> 5, sh = base & 31u;
-#pragma unroll
-    for (int ax = 0; ax < 3; ax++) {
-        const unsigned b = __ballot_sync(0xffffffffu, valid && ((code >> ax) & 1u));
-        if (b) {
-            uint32_t *row = upbits + (size_t)ax * P.upwords;
-            if (lane == 0) atomicOr(&row[w0], b << sh);
-            if (lane == 1 && sh) atomicOr(&row[w0 + 1], b >> (32u - sh));
-        }
-    }
-}
+// upbits[axis * upwords + (slot >> 5)] bit (slot & 31), written by the sort's
+// gather (publish_tile). The adjoint's rebuilt steps also publish the
+// lower-band flags (code bits 3-5), in rows 3-5 the same way.
 
 // Axes (bit 0 x, 1 y, 2 z) along which adjacency entry k (y,z,x order,
 // fluid_system.cpp:2266-2270) reaches into the lower neighbour cell.

@@ -148,7 +148,8 @@ struct fl_system {
     int64_t passes_steps[2]; // fused steps issued with the per-point passes / the cell tasks
     uint32_t *crowd_dev;   // largest in-range cell above 128 points, this step (0: none)
     uint32_t *crowd_epoch; // device: the state's epoch (bumped when the state is replaced)
-    uint32_t *crowd_host;  // page-locked [count, epoch], sent after each step's sort
+    uint32_t *crowd_host;  // page-locked [count, epoch], written by each step's sort
+    void *crowd_report;    // its device-side address
     uint32_t auto_epoch;   // host: the current state's epoch
     int adj_revmode;       // FL_REVERSE_*: how the adjoint finds its reverse pair lists
 
@@ -199,7 +200,7 @@ struct fl_system {
     // colours in while the step's first kernels run, and its two events
     // (created on first use)
     cudaStream_t side;
-    cudaEvent_t ev_early, ev_late, ev_crowd, ev_crowd_done, ev_auto[2];
+    cudaEvent_t ev_early, ev_late, ev_auto[2];
 
     // per-phase event timing (PERF_PUSH/PERF_POP of Run, cpp:507-515)
     int timing;
@@ -270,7 +271,7 @@ int fl_launch_compose(fl_system *s, int n, const uint32_t *src, const uint32_t *
 // dst[k][0..n) = src[k][0..n) for k < count (<= 3), one kernel pass
 int fl_launch_copy3(fl_system *s, int n, int count, const float4 *const *src, float4 *const *dst);
 int fl_launch_insert(fl_system *s, uint32_t *gcell_pre_or_null);
-int fl_launch_scan(fl_system *s, int count, int clear_status);
+int fl_launch_scan(fl_system *s, int count);
 int fl_launch_scatter_index(fl_system *s);
 // mode 0: rank only (sorted src + canonical gndx into f[F_GNDX].cur, pre-sort order)
 // mode 1: sorted src, then a gather of pos/vel/veval/clr/gcell/gndx into the
@@ -289,7 +290,6 @@ int fl_kernels_init(fl_system *s);
 size_t fl_big_cells_cap(int max_points);
 // gather every field cur -> nxt through src (phase-API counting sort)
 int fl_launch_gather_all(fl_system *s);
-int fl_launch_band_codes(fl_system *s);
 // the density pass with pair lists and pair records (fl_density.cu)
 int fl_density_init();   // once per process is enough; outside any stream capture
 int fl_density_block(const fl_system *s);
@@ -304,7 +304,10 @@ int fl_crowd_init();   // as fl_density_init
 int fl_launch_force_crowd(fl_system *s, bool advance, float dt, float *host_pos);
 int fl_launch_advance(fl_system *s, float time, float dt, float ss);
 int fl_launch_pack3(fl_system *s, const float4 *src, float *dst, int n, cudaStream_t stream = nullptr);
-int fl_launch_set_time(fl_system *s, int slot, float value);
+// every per-point field of a state of n points (src, dst by F_* field) and its
+// time; new_epoch: s->auto_epoch becomes the device's epoch too
+int fl_launch_copy_state(fl_system *s, int n, void *const *src, void *const *dst, const float *time_src,
+                         float *time_dst, bool new_epoch);
 int fl_launch_set_word(fl_system *s, uint32_t *word, uint32_t value);
 int fl_launch_unpack3(fl_system *s, const float *src, float4 *dst, int n);
 // up to 4 float3 -> float4 fields in one pass (src[k] may be host-mapped)

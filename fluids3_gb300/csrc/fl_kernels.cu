@@ -124,6 +124,8 @@ struct SortArgs {
     uint32_t big_cap;
     int gcells;                        // internal cell entries (all scenes, bins included)
     uint32_t *crowd_max;               // largest in-range cell above 128 points (atomic max)
+    const uint32_t *epoch;             // the state's epoch, and where it goes with the count: page-locked
+    volatile unsigned long long *report;   // host memory, or null
     const DevParams *scenes;           // batched: the scene table (bins at cell_base + ncells)
     const uint16_t *cell_scene;
     int ncells0;                       // single scene: its bin's entry
@@ -304,6 +306,8 @@ k_sort_big(const __grid_constant__ SortArgs a) {
             for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) a.gndx_pre[a.src[o + k]] = k;
         __syncthreads();
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.report)
+        *a.report = (unsigned long long)*a.epoch << 32 | *a.crowd_max;
     // the last block to finish clears the list for the next sort (every
     // block has read the count before it signs off)
     if (threadIdx.x == 0) {
@@ -350,6 +354,39 @@ __device__ __forceinline__ CellCtx cell_ctx(const DevParams &P0, const SceneTab 
 // and left to a warp each, one of 16,000 candidates would outlast the rest.
 constexpr uint32_t kCrowdedBlock = 1024, kPackedBlock = 4096;
 
+// What a warp of sorted slots publishes about them: the slot flags (code: each
+// lane's band code), and the tile's class. cell: each lane's cell entry, kUndef
+// past n and out of range. All lanes call it.
+template <bool BATCH, int ROWS>
+__device__ __forceinline__ void publish_tile(const DevParams &P0, const SceneTab &T, size_t word, uint32_t code,
+                                             uint32_t cell, const uint32_t *__restrict__ off,
+                                             uint32_t *__restrict__ upbits, uint32_t upwords, const CrowdTiles &tiles) {
+    const unsigned lane = lane_id();
+#pragma unroll
+    for (int row = 0; row < 3 * ROWS; row++) {
+        const unsigned b = __ballot_sync(0xffffffffu, (code >> row) & 1u);
+        if (lane == 0) upbits[(size_t)row * upwords + word] = b;
+    }
+    // the tile's candidates: the larger search block of its first and last
+    // points' cells (lanes 0-3 the four rows of one, 4-7 of the other)
+    const unsigned act = __ballot_sync(0xffffffffu, cell != kUndef);
+    const int from = act ? (lane < 4 ? __ffs(act) - 1 : 31 - __clz(act)) : 0;
+    const uint32_t c = __shfl_sync(0xffffffffu, cell, from);
+    uint32_t m = 0;
+    if (act && lane < 8) {
+        const DevParams &P = BATCH ? T.params[T.cell_scene[c]] : P0;
+        const int at = (int)c - P.nadj + ((int)(lane >> 1 & 1u) * P.gridRes.z + (int)(lane & 1u)) * P.gridRes.x;
+        m = off[at + 2] - off[at];
+    }
+    m += __shfl_xor_sync(0xffffffffu, m, 1);
+    m += __shfl_xor_sync(0xffffffffu, m, 2);
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
+    if (lane == 0) {
+        tiles.kind[word] = m >= kPackedBlock ? 2 : m >= kCrowdedBlock ? 1 : 0;
+        if (m >= kCrowdedBlock) list_tile(tiles, (uint32_t)word, m >= kPackedBlock);
+    }
+}
+
 template <bool BATCH, int ROWS, bool LATE = false>
 __global__ void __launch_bounds__(kThreads)
 k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *__restrict__ src,
@@ -382,34 +419,9 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
         gndx_out[s] = (uint32_t)s - off[c];
         upwords = (uint32_t)P.upwords;
     }
-    if constexpr (ROWS >= 1) {
-        const size_t word = (size_t)(s >> 5);
-        const unsigned lane = lane_id();
-        upwords = __shfl_sync(0xffffffffu, upwords, 0);   // lane 0 holds a point (s0 < n)
-#pragma unroll
-        for (int row = 0; row < 3 * ROWS; row++) {
-            const unsigned b = __ballot_sync(0xffffffffu, valid && ((code >> row) & 1u));
-            if (lane == 0) upbits[(size_t)row * upwords + word] = b;
-        }
-        // the tile's candidates: the larger search block of its first and last
-        // points' cells (lanes 0-3 the four rows of one, 4-7 of the other)
-        const unsigned act = __ballot_sync(0xffffffffu, cell != kUndef);
-        const int from = act ? (lane < 4 ? __ffs(act) - 1 : 31 - __clz(act)) : 0;
-        const uint32_t c = __shfl_sync(0xffffffffu, cell, from);
-        uint32_t m = 0;
-        if (act && lane < 8) {
-            const DevParams &P = BATCH ? T.params[T.cell_scene[c]] : P0;
-            const int at = (int)c - P.nadj + ((int)(lane >> 1 & 1u) * P.gridRes.z + (int)(lane & 1u)) * P.gridRes.x;
-            m = off[at + 2] - off[at];
-        }
-        m += __shfl_xor_sync(0xffffffffu, m, 1);
-        m += __shfl_xor_sync(0xffffffffu, m, 2);
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
-        if (lane == 0) {
-            tiles.kind[word] = m >= kPackedBlock ? 2 : m >= kCrowdedBlock ? 1 : 0;
-            if (m >= kCrowdedBlock) list_tile(tiles, (uint32_t)word, m >= kPackedBlock);
-        }
-    }
+    if constexpr (ROWS >= 1)   // (lane 0 holds a point: s0 < n)
+        publish_tile<BATCH, ROWS>(P0, T, (size_t)(s >> 5), code, cell, off, upbits,
+                                  __shfl_sync(0xffffffffu, upwords, 0), tiles);
 }
 
 // The velocities, evaluated velocities and colours of a step whose state
@@ -437,58 +449,47 @@ k_gather_late(int n, const uint32_t *__restrict__ src, const float *__restrict__
     clr_out[s] = clr ? clr[i] : 0u;
 }
 
-// Band codes and upper-band slot flags for an already sorted grid
-// (phase-API path, after k_gather_all): warp per cell, codes into pos.w.
-template <bool BATCH>
-__global__ void __launch_bounds__(kThreads)
-k_band_codes(const __grid_constant__ DevParams P0, const SceneTab T, int gcells,
-             const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
-             float4 *__restrict__ pos, uint32_t *__restrict__ upbits) {
-    const int c = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    if (c >= gcells) return;
-    const uint32_t m = cnt[c];
-    if (m == 0) return;
-    const uint32_t o = off[c];
-    const CellCtx cx = cell_ctx<BATCH>(P0, T, c);
-    const DevParams &P = *cx.P;
-    const unsigned lane = lane_id();
-    for (uint32_t kb = 0; kb < m; kb += 32) {
-        const uint32_t k = kb + lane;
-        const bool valid = k < m;
-        uint32_t code = 0;
-        if (valid) {
-            float4 p = pos[o + k];
-            code = band_code(P, cx.local, p);
-            p.w = __uint_as_float(code);
-            pos[o + k] = p;
-        }
-        publish_upbits(P, upbits, o + kb, code, valid);
-    }
-}
-
 // Phase-API counting sort (countingSortFull, fluids4.0/fluid_kernels.cu:56-87)
-// as a gather through the canonical src: every field moves cur -> nxt.
+// as a gather through the canonical src: every field moves cur -> nxt, and
+// with PRUNE the slots' band codes and flags are published as the fused
+// step's gather does.
+template <bool BATCH, bool PRUNE>
 __global__ void __launch_bounds__(kThreads)
-k_gather_all(int n, const uint32_t *__restrict__ src,
-             const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *__restrict__ src,
+             const uint32_t *__restrict__ off, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
              const float4 *__restrict__ veval, const float4 *__restrict__ force,
              const float *__restrict__ press, const uint32_t *__restrict__ clr,
              const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ gndx,
              float4 *__restrict__ pos_o, float4 *__restrict__ vel_o,
              float4 *__restrict__ veval_o, float4 *__restrict__ force_o,
              float *__restrict__ press_o, uint32_t *__restrict__ clr_o,
-             uint32_t *__restrict__ gcell_o, uint32_t *__restrict__ gndx_o) {
+             uint32_t *__restrict__ gcell_o, uint32_t *__restrict__ gndx_o, uint32_t *__restrict__ upbits,
+             const CrowdTiles tiles) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const uint32_t i = src[s];
-    pos_o[s] = pos[i];
-    vel_o[s] = vel[i];
-    veval_o[s] = veval[i];
-    force_o[s] = force[i];
-    press_o[s] = press[i];
-    clr_o[s] = clr[i];
-    gcell_o[s] = gcell[i];
-    gndx_o[s] = gndx[i];
+    if (s - (int)lane_id() >= n) return;   // whole warp past n
+    uint32_t code = 0, cell = kUndef;
+    if (s < n) {
+        const uint32_t i = src[s];
+        cell = gcell[i];
+        float4 p = pos[i];
+        if (PRUNE) {
+            if (cell != kUndef) {
+                const DevParams &P = BATCH ? T.params[T.cell_scene[cell]] : P0;
+                code = band_code(P, (int)cell - P.cell_base, p);
+            }
+            p.w = __uint_as_float(code);
+        }
+        pos_o[s] = p;
+        vel_o[s] = vel[i];
+        veval_o[s] = veval[i];
+        force_o[s] = force[i];
+        press_o[s] = press[i];
+        clr_o[s] = clr[i];
+        gcell_o[s] = cell;
+        gndx_o[s] = gndx[i];
+    }
+    if constexpr (PRUNE)
+        publish_tile<BATCH, 1>(P0, T, (size_t)(s >> 5), code, cell, off, upbits, (uint32_t)P0.upwords, tiles);
 }
 
 // computeForce (fluids4.0/fluid_kernels.cu:180-217) in two stages per warp:
@@ -714,7 +715,34 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
 }
 
 // ---------------------------------------------------------------------------
-__global__ void k_set_time(float *time_dev, float value) { *time_dev = value; }
+// A checkpoint's save or restore in one pass: every per-point field, the time
+// and (restore) the state's epoch.
+struct StateCopy {
+    const float4 *src4[4];
+    float4 *dst4[4];
+    const uint32_t *src1[4];
+    uint32_t *dst1[4];
+    const float *time_src;
+    float *time_dst;
+    uint32_t *epoch;      // null: left alone
+    uint32_t epoch_value;
+};
+
+__global__ void __launch_bounds__(kThreads) k_copy_state(int n, const __grid_constant__ StateCopy c) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        *c.time_dst = *c.time_src;
+        if (c.epoch) *c.epoch = c.epoch_value;
+    }
+    if (i >= n) return;
+    float4 v[4];
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) { v[k] = c.src4[k][i]; w[k] = c.src1[k][i]; }
+#pragma unroll
+    for (int k = 0; k < 4; k++) { c.dst4[k][i] = v[k]; c.dst1[k][i] = w[k]; }
+}
+
 __global__ void k_set_word(uint32_t *word, uint32_t value) { *word = value; }
 
 __global__ void k_pack3(int n, const float4 *__restrict__ src, float *__restrict__ dst) {
@@ -877,6 +905,8 @@ int fl_launch_sort_cells(fl_system *s, int mode, bool late) {
     a.big_cap = (uint32_t)fl_big_cells_cap(s->max_points);
     a.gcells = s->gcells;
     a.crowd_max = s->crowd_dev;
+    a.epoch = s->crowd_epoch;
+    a.report = mode == 1 ? (volatile unsigned long long *)s->crowd_report : nullptr;
     a.scenes = s->batched ? s->d_scenes : nullptr;
     a.cell_scene = s->cell_scene;
     a.ncells0 = s->ncells;
@@ -938,36 +968,27 @@ int fl_launch_gather_late(fl_system *s, const float *vel3, const float *veval3, 
 
 int fl_launch_gather_all(fl_system *s) {
     if (s->n == 0) return FL_OK;
-    k_gather_all<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-        s->n, s->src,
+    auto kern = s->batched ? (s->D.prune ? k_gather_all<true, true> : k_gather_all<true, false>)
+                           : (s->D.prune ? k_gather_all<false, true> : k_gather_all<false, false>);
+    kern<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
+        s->D, fl_scene_tab(s), s->n, s->src, s->off,
         s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
         s->f[F_FORCE].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_CLR].cur<uint32_t>(),
         s->f[F_GCELL].cur<uint32_t>(), s->f[F_GNDX].cur<uint32_t>(),
         s->f[F_POS].nxt<float4>(), s->f[F_VEL].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(),
         s->f[F_FORCE].nxt<float4>(), s->f[F_PRESS].nxt<float>(), s->f[F_CLR].nxt<uint32_t>(),
-        s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>());
+        s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits, s->tiles);
     FL_LAUNCH_CHECK("gather_all");
+    s->codes_valid = 1;
+    s->tiles_listed = s->D.prune;
     return FL_OK;
 }
 
 size_t fl_upbits_bytes(const fl_system *s) { return 3 * sizeof(uint32_t) * (size_t)s->D.upwords; }
 
 // Pruned neighbour passes need gridSrch == 2 (every scene of a batch) and
-// band codes that match the live positions (set by the fused sort or
-// fl_launch_band_codes).
+// band codes that match the live positions (set by the sort's gather).
 static bool use_prune(const fl_system *s) { return s->D.prune && s->codes_valid; }
-
-int fl_launch_band_codes(fl_system *s) {
-    if (!s->D.prune) { s->codes_valid = 1; return FL_OK; }
-    const int grid = blocks_for((long long)s->gcells, kThreads / 32);
-    FL_CUDA_TRY(cudaMemsetAsync(s->upbits, 0, fl_upbits_bytes(s), s->stream));
-    auto kern = s->batched ? k_band_codes<true> : k_band_codes<false>;
-    kern<<<grid, kThreads, 0, s->stream>>>(s->D, fl_scene_tab(s), s->gcells, s->off, s->cnt,
-                                          s->f[F_POS].cur<float4>(), s->upbits);
-    FL_LAUNCH_CHECK("band_codes");
-    s->codes_valid = 1;
-    return FL_OK;
-}
 
 template <bool LIST, bool BATCH>
 static auto force_kernel(bool prune) {
@@ -1024,9 +1045,22 @@ int fl_launch_advance(fl_system *s, float time, float dt, float ss) {
     return FL_OK;
 }
 
-int fl_launch_set_time(fl_system *s, int slot, float value) {
-    k_set_time<<<1, 1, 0, s->stream>>>(s->time_dev + slot, value);
-    FL_LAUNCH_CHECK("set_time");
+int fl_launch_copy_state(fl_system *s, int n, void *const *src, void *const *dst, const float *time_src,
+                         float *time_dst, bool new_epoch) {
+    static const int field4[4] = {F_POS, F_VEL, F_VEVAL, F_FORCE}, field1[4] = {F_PRESS, F_CLR, F_GCELL, F_GNDX};
+    StateCopy c;
+    for (int k = 0; k < 4; k++) {
+        c.src4[k] = (const float4 *)src[field4[k]];
+        c.dst4[k] = (float4 *)dst[field4[k]];
+        c.src1[k] = (const uint32_t *)src[field1[k]];
+        c.dst1[k] = (uint32_t *)dst[field1[k]];
+    }
+    c.time_src = time_src;
+    c.time_dst = time_dst;
+    c.epoch = new_epoch ? s->crowd_epoch : nullptr;
+    c.epoch_value = s->auto_epoch;
+    k_copy_state<<<blocks_for(n > 0 ? n : 1, kThreads), kThreads, 0, s->stream>>>(n, c);
+    FL_LAUNCH_CHECK("copy_state");
     return FL_OK;
 }
 

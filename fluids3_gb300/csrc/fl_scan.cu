@@ -139,15 +139,12 @@ size_t fl_scan_tile() { return kTile; }
 // Ticket (padded to 256 B) followed by one descriptor per tile.
 size_t fl_scan_scratch_bytes(int ntiles) { return 256 + sizeof(uint64_t) * (size_t)ntiles; }
 
-// Exclusive scan of s->cnt[0 .. count) into s->off. With clear_status the
-// ticket and descriptors are zeroed first; otherwise the caller has
-// already cleared them (together with the counts).
-int fl_launch_scan(fl_system *s, int count, int clear_status) {
+// Exclusive scan of s->cnt[0 .. count) into s->off. The caller has cleared the
+// ticket and descriptors (together with the counts).
+int fl_launch_scan(fl_system *s, int count) {
     const int ntiles = (int)((count + kTile - 1) / kTile);
     if (ntiles > s->scan_tiles)
         return fl_fail(FL_ERR_ARG, "scan: %d tiles exceed the %d allocated", ntiles, s->scan_tiles);
-    if (clear_status)
-        FL_CUDA_TRY(cudaMemsetAsync(s->scan_ticket, 0, fl_scan_scratch_bytes(s->scan_tiles), s->stream));
     k_scan<<<ntiles, kThreads, 0, s->stream>>>(s->cnt, s->off, s->scan_status, s->scan_ticket,
                                                ntiles, s->scan_epoch, /*inclusive=*/0,
                                                s->dev_err, kSpinLimit, 0u);
