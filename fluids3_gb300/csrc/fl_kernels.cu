@@ -282,6 +282,9 @@ k_sort_big(const __grid_constant__ SortArgs a) {
     if (threadIdx.x == 0) s_nbig = min(*(volatile uint32_t *)a.big_count, a.big_cap);
     __syncthreads();
     const uint32_t nbig = s_nbig;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.report)
+        *a.report = (unsigned long long)*a.epoch << 32 | *a.crowd_max;
+    if (nbig == 0) return;   // nothing to sort, nothing to clear
     for (uint32_t b = blockIdx.x; b < nbig; b += gridDim.x) {
         const uint32_t c = a.big_cells[b];
         const uint32_t m = a.cnt[c], o = a.off[c];
@@ -307,8 +310,6 @@ k_sort_big(const __grid_constant__ SortArgs a) {
             for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) a.gndx_pre[a.src[o + k]] = k;
         __syncthreads();
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.report)
-        *a.report = (unsigned long long)*a.epoch << 32 | *a.crowd_max;
     // the last block to finish clears the list for the next sort (every
     // block has read the count before it signs off)
     if (threadIdx.x == 0) {

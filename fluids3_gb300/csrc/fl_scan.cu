@@ -5,8 +5,8 @@
 //
 // Each CTA takes a tile of kTile counts (dynamic tile id from a ticket, so a
 // tile's predecessors were all scheduled before it), scans it, publishes
-// its aggregate, then walks back over predecessor descriptors until it
-// meets an inclusive prefix. A descriptor is 64 bits:
+// its aggregate, then one warp walks back over predecessor descriptors, 32
+// at a time, until it meets an inclusive prefix. A descriptor is 64 bits:
 //   [63:62] flag (1 = aggregate, 2 = inclusive prefix), [61:32] launch
 //   epoch, [31:0] value.
 // The host zeroes the descriptors and the ticket before every launch (one
@@ -36,6 +36,37 @@ __device__ __forceinline__ void st_release(uint64_t *p, uint64_t v) {
 }
 __device__ __forceinline__ uint64_t pack(uint64_t flag, uint32_t epoch, uint32_t value) {
     return (flag << 62) | ((uint64_t)(epoch & 0x3fffffffu) << 32) | value;
+}
+
+// The sum of all tiles up to `last`, by one warp: 32 descriptors a round, each
+// lane waiting (bounded) for its own, up to the nearest inclusive prefix. One
+// thread walking back a descriptor a time took a round trip to L2 for each:
+// 9.8 us for 25 tiles, 11.4 for 90.
+__device__ __forceinline__ uint32_t look_back(const uint64_t *status, int last, uint32_t epoch, uint32_t *err,
+                                              int spin_limit) {
+    const int lane = (int)(threadIdx.x & 31u);
+    uint32_t prefix = 0;
+    for (int j = last; j >= 0; j -= 32) {
+        uint64_t d = pack(kFlagPrefix, epoch, 0);   // (before the first tile: nothing)
+        if (j - lane >= 0) {
+            for (int spins = 0;;) {
+                d = ld_acquire(&status[j - lane]);
+                if ((d >> 62) != 0 && (uint32_t)((d >> 32) & 0x3fffffffu) == (epoch & 0x3fffffffu)) break;
+                if (++spins > spin_limit) {
+                    atomicOr(err, FL_DEV_SPIN_TIMEOUT);
+                    d = pack(kFlagPrefix, epoch, 0);
+                    break;
+                }
+                __nanosleep(32);
+            }
+        }
+        __syncwarp();
+        const unsigned ends = __ballot_sync(0xffffffffu, (d >> 62) == kFlagPrefix);
+        const int upto = ends ? __ffs(ends) - 1 : 31;
+        prefix += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)d : 0u);
+        if (ends) break;
+    }
+    return prefix;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -88,34 +119,16 @@ k_scan(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, uint64_t *st
     const uint32_t tile_total = s_warp[kThreads / 32 - 1];
     const uint32_t thread_excl = (warp ? s_warp[warp - 1] : 0u) + x - thread_total;
 
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
         uint32_t prefix = 0;
-        if (tile == 0) {
-            st_release(&status[0], pack(kFlagPrefix, epoch, tile_total));
-        } else {
-            st_release(&status[tile], pack(kFlagAgg, epoch, tile_total));
-            int j = (int)tile - 1;
-            while (j >= 0) {
-                uint64_t d;
-                int spins = 0;
-                for (;;) {
-                    d = ld_acquire(&status[j]);
-                    if ((d >> 62) != 0 && (uint32_t)((d >> 32) & 0x3fffffffu) == (epoch & 0x3fffffffu))
-                        break;
-                    if (++spins > spin_limit) {
-                        atomicOr(err, FL_DEV_SPIN_TIMEOUT);
-                        d = pack(kFlagPrefix, epoch, 0);
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-                prefix += (uint32_t)d;
-                if ((d >> 62) == kFlagPrefix) break;
-                j--;
-            }
-            st_release(&status[tile], pack(kFlagPrefix, epoch, prefix + tile_total));
+        if (tile > 0) {
+            if (lane == 0) st_release(&status[tile], pack(kFlagAgg, epoch, tile_total));
+            prefix = look_back(status, (int)tile - 1, epoch, err, spin_limit);
         }
-        s_prefix = prefix;
+        if (lane == 0) {
+            st_release(&status[tile], pack(kFlagPrefix, epoch, prefix + tile_total));
+            s_prefix = prefix;
+        }
     }
     __syncthreads();
     const uint32_t start = s_prefix + thread_excl;
