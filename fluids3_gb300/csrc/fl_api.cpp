@@ -226,9 +226,9 @@ extern "C" int fl_create(const fl_params *p, int max_points, fl_system **out) {
         s->nscenes = 1;
         const size_t np = (size_t)(max_points > 0 ? max_points : 1);
         const size_t esz[F_COUNT] = {16, 16, 16, 16, 4, 4, 4, 4};
-        for (int k = 0; k < F_COUNT && r == FL_OK; k++) {
+        for (int k = 0; k < F_COUNT && r == FL_OK; k++) {   // (walks of a row read a few slots past its end)
             s->f[k].esz = esz[k];
-            for (int c = 0; c < 2 && r == FL_OK; c++) r = fl_dalloc(&s->f[k].p[c], esz[k] * np);
+            for (int c = 0; c < 2 && r == FL_OK; c++) r = fl_dalloc(&s->f[k].p[c], esz[k] * (np + 8));
         }
         if (r != FL_OK) break;
         if ((r = fl_dalloc((void **)&s->cell_pre, 4 * np)) != FL_OK) break;

@@ -5,8 +5,9 @@
 // loop (cells in y, z, x order, members in slot order) visits the rows in
 // order and each row in ascending slots.
 //
-// k_density_rows: a thread per point walks its rows. For gridSrch > 2, whose
-// small cells leave few candidates that are not pairs.
+// k_density_rows: a thread per point walks its rows, the warp's pair lists
+// written through shared memory (ring_walk). For gridSrch > 2, whose small
+// cells leave few candidates that are not pairs.
 //
 // k_density: a warp per 32 consecutive slots, for gridSrch 2, whose block
 // holds about twenty candidates per pair. It walks the union of its points'
@@ -29,9 +30,10 @@
 // point over flag-pruned candidates took 157, and its chain of dependent loads
 // left small scenes waiting: 2,048 points 35.0 us then, 18.4 now; 65,536:
 // 46.1, 24.7; 1,000,000 (wave tank): 164, 110. With gridSrch 3 (250,000
-// points, 165 candidates and 70 pairs a point) the rows take 95 us, the old
+// points, 165 candidates and 70 pairs a point) the rows take 69 us, the old
 // loop took 118 and the filter 140: there every third candidate is a pair, and
-// a warp's points come from more runs than one.
+// a warp's points come from more runs than one. Staging a row's run in shared
+// memory for the warp took 112 (most warps then walk two runs).
 //
 // The tensor instruction is mma.sync: a tile of 16 x 8 with a depth of 16 has
 // too little work for tcgen05's descriptors, and the accumulator's signs
@@ -327,6 +329,97 @@ __device__ __forceinline__ void segment(const DevParams &P, Sum &s, unsigned seg
     }
 }
 
+// The points of a warp, each by itself, for rows that leave few candidates
+// that are not pairs. All lanes call it. The lanes' pair counts drift apart, so
+// a list entry stored when its pair was found went to a line of its own a lane;
+// now entry t waits in `ring` (shared memory: kRing entries a lane) until all
+// lanes have reached it. One at `lim` or past it, ahead of the slowest lane by
+// more than the ring holds, is stored at once. 250,000 points with gridSrch 3:
+// 96 us with every entry stored when found, 81 with 16 entries a lane, 69 with
+// 32; 40 resident warps of 48 registers, 48 of 40 took 81.
+constexpr uint32_t kRing = 32;
+constexpr uint32_t kRingAhead = 4;
+template <bool BATCH>
+__device__ __forceinline__ void ring_visit(Sum &s, const PairParams<BATCH> &c, float4 q, uint32_t j, uint32_t k,
+                                           uint32_t left, uint32_t lim, uint32_t past, uint32_t ring) {
+    float dx2, dy2;
+    const uint64_t dxy = sub2(pk2(s.p.x, s.p.y), pk2(q.x, q.y));
+    const float dz = s.p.z - q.z;
+    up2(mul2(dxy, dxy), dx2, dy2);
+    const float dsq = dx2 + dy2 + dz * dz;
+    float t = (c.rd2() - dsq) * c.d2();
+    t = t * t * t;
+    asm volatile(
+        "{\n"
+        ".reg .pred hit, in, out;\n"
+        ".reg .u32 at, d;\n"
+        ".reg .u64 to;\n"
+        "setp.lt.u32 hit, %2, %3;\n"
+        "setp.lt.and.f32 hit, %4, %5, hit;\n"
+        "setp.gt.and.f32 hit, %4, 0f00000000, hit;\n"
+        "setp.lt.and.u32 in, %1, %10, hit;\n"
+        "sub.u32 d, %1, %10;\n"
+        "setp.lt.and.u32 out, d, %11, hit;\n"
+        "and.b32 at, %1, %9;\n"
+        "mad.lo.u32 at, at, 128, %8;\n"
+        "@in st.shared.u32 [at], %6;\n"
+        "mad.wide.u32 to, %1, 128, %12;\n"
+        "@out st.global.u32 [to], %6;\n"
+        "@hit add.rn.f32 %0, %0, %7;\n"
+        "@hit add.u32 %1, %1, 1;\n"
+        "}"
+        : "+f"(s.sum), "+r"(s.nh)
+        : "r"(k), "r"(left), "f"(dsq), "f"(c.rd2()), "r"(j), "f"(t), "r"(ring), "n"(kRing - 1u), "r"(lim), "r"(past),
+          "l"(s.next)
+        : "memory");
+}
+// (s.next stays at the list's start.)
+template <bool BATCH>
+__device__ __forceinline__ void ring_walk(const DevParams &P, Sum &s, bool active, uint32_t gc,
+                                          const float4 *__restrict__ pos, const uint32_t *__restrict__ off,
+                                          uint32_t *ring) {
+    const PairParams<BATCH> pp(P);
+    const int srch = P.gridSrch, own = srch * srch,
+              rows = BATCH ? (int)__reduce_max_sync(0xffffffffu, (unsigned)own) : own;
+    const uint32_t *at = off + (active ? (int)gc - P.nadj : 0);
+    uint32_t j = 0, j1 = 0;
+    if (active) { j = at[0]; j1 = at[srch]; }
+    const uint32_t cap = pp.cap(), sring = (uint32_t)__cvta_generic_to_shared(ring + lane_id());
+    uint32_t done = 0, lim = min(kRing, cap);   // entries that all lanes have written; the ring's end
+    uint32_t d0 = 0, d1 = 0;                    // entries [d0, d1) were stored at once
+    for (int r = 1;; r++) {
+        uint32_t nj = 0, nj1 = 0;
+        if (r < own && active) {   // the next row's bounds while this one is walked
+            const int a = P.adj[r * srch];
+            nj = at[a];
+            nj1 = at[a + srch];
+        }
+        const uint32_t past = cap - lim;
+        const float4 *from = pos + j;   // (read a few slots past the row's end, and past the last point)
+        for (; j < j1; j += kRingAhead, from += kRingAhead) {
+            float4 q[kRingAhead];
+#pragma unroll
+            for (uint32_t k = 0; k < kRingAhead; k++) q[k] = from[k];
+            const uint32_t left = j1 - j;
+#pragma unroll
+            for (uint32_t k = 0; k < kRingAhead; k++) ring_visit(s, pp, q[k], j + k, k, left, lim, past, sring);
+        }
+        const bool end = r >= rows;
+        uint32_t low = end ? __reduce_max_sync(0xffffffffu, s.nh)
+                           : __reduce_min_sync(0xffffffffu, active ? s.nh : 0xffffffffu);
+        low = low == 0xffffffffu ? 0u : min(low, cap);
+        const uint32_t held = min(lim, s.nh);
+        for (uint32_t t = done; t < low; t++)
+            if (t < held && t - d0 >= d1 - d0) s.next[32u * t] = ring[(t & (kRing - 1u)) * 32u + lane_id()];
+        if (end) break;
+        done = max(done, low);
+        if (s.nh > lim && done >= d1) d0 = lim, d1 = s.nh;
+        if (s.nh <= lim || d1 == s.nh) lim = min(done + kRing, cap);
+        j = nj;
+        j1 = nj1;
+    }
+}
+
 // A point's results: its density, pair count and pair record.
 __device__ __forceinline__ void finish(const DevParams &P, const Sum &s, int i, bool active,
                                        const float4 *__restrict__ veval, float *__restrict__ press,
@@ -346,23 +439,23 @@ __device__ __forceinline__ void finish(const DevParams &P, const Sum &s, int i, 
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(kRowsMaxThreads, 1536 / kRowsMaxThreads)
+__global__ void __launch_bounds__(kRowsMaxThreads, 1280 / kRowsMaxThreads)
 k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
                const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
                float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
                float4 *__restrict__ pairdata) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const DevParams &P = BATCH ? T.params[T.point_scene[i]] : P0;
-    const uint32_t gc = gcell[i];
+    const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
+    const uint32_t gc = (i < n) ? gcell[i] : kUndef;
     const bool active = gc != kUndef;
     Sum s;
-    s.p = pos[i];
+    s.p = active ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     s.sum = 0.0f;
     s.nh = 0;
     s.next = hitlist + list_at(P, i, 0);
-    if (active) walk<BATCH>(P, s, gc, pos, off);
-    finish(P, s, i, active, veval, press, hitcnt, pairdata);
+    extern __shared__ __align__(16) uint32_t s_dyn[];
+    ring_walk<BATCH>(P, s, active, gc, pos, off, s_dyn + (threadIdx.x >> 5) * (32 * kRing));
+    if (i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
 }
 
 // A crowded tile, by a whole block (fl_crowd.cuh). Alone, its warp would walk
@@ -532,7 +625,7 @@ int fl_launch_density(fl_system *s) {
     const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
     if (rows) {
         auto kern = s->batched ? k_density_rows<true> : k_density_rows<false>;
-        kern<<<blocks_for(s->n, bs), bs, 0, s->stream>>>(
+        kern<<<blocks_for(s->n, bs), bs, (size_t)(bs / 32) * 32 * kRing * sizeof(uint32_t), s->stream>>>(
             s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
             s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
     } else {
