@@ -48,7 +48,7 @@ constexpr int kAdjThreads = 128;
 __device__ __forceinline__ const DevParams &scene_params(const DevParams &P0, const SceneTab &T, int s) {
     return T.params ? T.params[T.point_scene[s]] : P0;
 }
-constexpr int kReduceThreads = 256;
+constexpr int kReduceThreads = 512;
 constexpr int kReduceChunk = 4096;   // points per partial-sum block
 
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
@@ -652,9 +652,15 @@ k_adj_revsort(int n, int hcap_in, uint32_t *__restrict__ revlist, uint32_t *__re
 // (k_adj_revwalk's list), so the long pair arithmetic runs with the lanes
 // busy. A point whose own or reverse list overflowed is appended to the
 // crowd list instead, and k_adj_crowd_force adds those pairs. Writes dL/dE
-// through the permutation, accumulates dL/dX into xa, stores dL/drho and
-// the parameter partials (dL/dvisc, dL/drest_density, dL/dIntStiff) of its
-// own pairs.
+// through the permutation, accumulates dL/dX into xa, stores the parameter
+// partials (dL/dvisc, dL/drest_density, dL/dIntStiff) of its own pairs and,
+// over the dL/dE that it has used up in ea, what the density adjoint's pairs
+// read: (position, dL/drho).
+//
+// Bound by instruction issue and the waits on its four loads a pair (1,200,000
+// points: 98 warp instructions a pair, 250 us, 62% of the issue slots). Slower
+// there: position, velocity and density in one record for a 256-bit load 299
+// (two pairs in flight 293); the next list entry fetched ahead by hand 280.
 template <bool PRUNE>
 __global__ void __launch_bounds__(kAdjThreads, 8)
 k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
@@ -662,8 +668,8 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
             const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
             const uint32_t *__restrict__ upbits, const uint32_t *__restrict__ hitlist,
             const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ src,
-            const float4 *__restrict__ fb, float4 *__restrict__ xa, const float4 *__restrict__ ea,
-            float *__restrict__ rb, float4 *__restrict__ pc, float4 *__restrict__ e_out,
+            const float4 *__restrict__ fb, float4 *__restrict__ xa, float4 *ea, float4 *__restrict__ pc,
+            float4 *__restrict__ e_out,
             const uint32_t *__restrict__ revlist, const uint32_t *__restrict__ revcnt, const CrowdList crowd) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = scene_params(P0, T, s < n ? s : 0);
@@ -716,14 +722,14 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
     const uint32_t dst = src[s];
     if (!active) {
         e_out[dst] = ea[s];
-        rb[s] = 0.0f;
+        ea[s] = make_float4(0.f, 0.f, 0.f, 0.f);
         pc[s] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
     const float4 x0 = xa[s], e0 = ea[s];
     xa[s] = make_float4(x0.x + acc.x.x, x0.y + acc.x.y, x0.z + acc.x.z, 0.f);
     e_out[dst] = make_float4(e0.x + acc.e.x, e0.y + acc.e.y, e0.z + acc.e.z, 0.f);
-    rb[s] = acc.r;
+    ea[s] = make_float4(X.x, X.y, X.z, acc.r);
     pc[s] = make_float4(acc.gv, acc.gr, acc.gk, 0.f);
 }
 
@@ -732,7 +738,9 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 // every pair of owner o. Own pairs from the density pass's list (those in
 // the point's own cell are reverse pairs too), reverse pairs in the other
 // cells from the list k_adj_revwalk recorded; the finished dL/dX goes
-// through the permutation. With walk_overflow off (as fl_backward launches
+// through the permutation. A neighbour's position and dL/drho come in one load
+// (xr; two loads took 113 us at 1,200,000 points, one takes 98). With
+// walk_overflow off (as fl_backward launches
 // it) a point whose list overflowed is left to k_adj_crowd_density, which
 // spreads its pairs over a block; on, the point walks them itself. (The
 // per-thread walk is kept compiled in: without it this kernel's list loops
@@ -741,13 +749,12 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 template <bool PRUNE>
 __global__ void __launch_bounds__(kAdjThreads)
 k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
-              const float4 *__restrict__ pos, const uint32_t *__restrict__ gcell,
+              const float4 *__restrict__ pos, const float4 *__restrict__ xr, const uint32_t *__restrict__ gcell,
               const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
               const uint32_t *__restrict__ upbits, const uint32_t *__restrict__ hitlist,
               const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revlist,
               const uint32_t *__restrict__ revcnt, const uint32_t *__restrict__ src,
-              const float *__restrict__ rb, const float4 *__restrict__ xa, float4 *__restrict__ x_out,
-              bool walk_overflow) {
+              const float4 *__restrict__ xa, float4 *__restrict__ x_out, bool walk_overflow) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const DevParams &P = scene_params(P0, T, s);
@@ -762,29 +769,27 @@ k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
     const float3 X = xyz(p4);
     const uint32_t my_code = __float_as_uint(p4.w);
     const float kmp = -6.0f * P.d2 * P.pmass * P.poly6kern;
-    const float gs = kmp * rb[s];
+    const float gs = kmp * xr[s].w;
     float3 xacc = make_float3(0.f, 0.f, 0.f);
     // own pair (owner s): + gs w^2 (X_s - X_j)
-    auto own = [&](uint32_t j) {
-        const float4 q = pos[j];
+    auto own = [&](const float4 &q) {
         const float3 D = make_float3(X.x - q.x, X.y - q.y, X.z - q.z);
         const float w = (P.rd2 - (D.x * D.x + D.y * D.y + D.z * D.z)) * P.d2;
         const float k = gs * w * w;
         xacc.x += k * D.x; xacc.y += k * D.y; xacc.z += k * D.z;
     };
     // reverse pair (owner o): - g_o w^2 (X_o - X_s)
-    auto rev = [&](uint32_t o) {
-        const float4 q = pos[o];
+    auto rev = [&](const float4 &q) {
         const float3 D = make_float3(q.x - X.x, q.y - X.y, q.z - X.z);
         const float w = (P.rd2 - (D.x * D.x + D.y * D.y + D.z * D.z)) * P.d2;
-        const float k = kmp * rb[o] * w * w;
+        const float k = kmp * q.w * w * w;
         xacc.x -= k * D.x; xacc.y -= k * D.y; xacc.z -= k * D.z;
     };
     // own pairs; those in the own cell are reverse pairs as well
     const uint32_t c_lo = off[gc], c_hi = c_lo + cnt[gc];
-    auto both = [&](uint32_t j) {
-        if (gs != 0.0f) own(j);
-        if (j >= c_lo && j < c_hi) rev(j);
+    auto both = [&](uint32_t j, const float4 &q) {
+        if (gs != 0.0f) own(q);
+        if (j >= c_lo && j < c_hi) rev(q);
     };
     const uint32_t nh = hitcnt[s];
     // the lists are read four entries per round, all requested before the
@@ -796,9 +801,12 @@ k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 #pragma unroll
             for (int k = 0; k < 4; k++) j[k] = hitlist[list_at(P, s, t + k)];
 #pragma unroll
-            for (int k = 0; k < 4; k++) both(j[k]);
+            for (int k = 0; k < 4; k++) both(j[k], xr[j[k]]);
         }
-        for (; t < nh; t++) both(hitlist[list_at(P, s, t)]);
+        for (; t < nh; t++) {
+            const uint32_t j = hitlist[list_at(P, s, t)];
+            both(j, xr[j]);
+        }
     } else if (walk_overflow) {
         const int base = (int)gc - P.nadj;
         for (int c = 0; c < P.gridAdjCnt; c++) {
@@ -806,9 +814,9 @@ k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
             cand_begin<PRUNE>(it, P, c, base + P.adj[c], my_code, true, off, cnt, upbits);
             uint32_t j;
             while (cand_next<PRUNE>(it, P, upbits, j)) {
-                const float4 q = pos[j];
+                const float4 q = xr[j];
                 const float dsq = dsq_rn(p4.x - q.x, p4.y - q.y, p4.z - q.z);
-                if (dsq < P.rd2 && dsq > 0.0f) both(j);
+                if (dsq < P.rd2 && dsq > 0.0f) both(j, q);
             }
         }
     }
@@ -821,18 +829,18 @@ k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 #pragma unroll
             for (int k = 0; k < 4; k++) o[k] = revlist[list_at(P, s, t + k)];
 #pragma unroll
-            for (int k = 0; k < 4; k++) rev(o[k]);
+            for (int k = 0; k < 4; k++) rev(xr[o[k]]);
         }
-        for (; t < nr; t++) rev(revlist[list_at(P, s, t)]);
+        for (; t < nr; t++) rev(xr[revlist[list_at(P, s, t)]]);
     } else if (walk_overflow) {
         const uint32_t *lobits = upbits + 3 * (size_t)P.upwords;
         RevIter it;
         rev_begin<PRUNE>(it, P, gc, my_code, true);
         uint32_t o;
         while (rev_next<PRUNE>(it, P, off, cnt, lobits, o)) {
-            const float4 q = pos[o];
+            const float4 q = xr[o];
             const float dsq = dsq_rn(q.x - X.x, q.y - X.y, q.z - X.z);
-            if (dsq < P.rd2 && dsq > 0.0f) rev(o);
+            if (dsq < P.rd2 && dsq > 0.0f) rev(q);
         }
     }
     x_out[dst] = make_float4(x0.x + xacc.x, x0.y + xacc.y, x0.z + xacc.z, 0.f);
@@ -923,7 +931,7 @@ k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const 
                   const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
                   const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
                   const uint32_t *__restrict__ src, const float4 *__restrict__ fb, float4 *__restrict__ xa,
-                  float4 *__restrict__ e_out, float *__restrict__ rb, float4 *__restrict__ pc, const CrowdList L) {
+                  float4 *__restrict__ e_out, float4 *__restrict__ xr, float4 *__restrict__ pc, const CrowdList L) {
     __shared__ float s_red[kCrowdThreads / 32][10];
     __shared__ uint32_t s_nlist;
     if (threadIdx.x == 0) s_nlist = min(*(volatile uint32_t *)L.count, L.cap);
@@ -960,7 +968,7 @@ k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const 
             const float4 x0 = xa[s], e0 = e_out[dst], c0 = pc[s];
             xa[s] = make_float4(x0.x + v[0], x0.y + v[1], x0.z + v[2], 0.f);
             e_out[dst] = make_float4(e0.x + v[3], e0.y + v[4], e0.z + v[5], 0.f);
-            rb[s] += v[6];
+            xr[s].w += v[6];
             pc[s] = make_float4(c0.x + v[7], c0.y + v[8], c0.z + v[9], 0.f);
         }
         __syncthreads();
@@ -976,7 +984,7 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
                     const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
                     const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
                     const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
-                    const uint32_t *__restrict__ src, const float *__restrict__ rb, float4 *__restrict__ x_out,
+                    const uint32_t *__restrict__ src, const float4 *__restrict__ xr, float4 *__restrict__ x_out,
                     const CrowdList L) {
     __shared__ float s_red[kCrowdThreads / 32][3];
     __shared__ uint32_t s_nlist;
@@ -990,13 +998,13 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
         const float4 p4 = pos[s];
         const float3 X = xyz(p4);
         const float kmp = -6.0f * P.d2 * P.pmass * P.poly6kern;
-        const float gs = kmp * rb[s];
+        const float gs = kmp * xr[s].w;
         const uint32_t c_lo = off[gc], c_hi = c_lo + cnt[gc], hcap = (uint32_t)P.hcap;
         float3 part = make_float3(0.f, 0.f, 0.f);
         auto rev = [&](uint32_t o, float4 q) {   // owner o: - g_o w^2 (X_o - X_s)
             const float3 D = make_float3(q.x - X.x, q.y - X.y, q.z - X.z);
             const float w = (P.rd2 - (D.x * D.x + D.y * D.y + D.z * D.z)) * P.d2;
-            const float k = kmp * rb[o] * w * w;
+            const float k = kmp * xr[o].w * w * w;
             part.x -= k * D.x; part.y -= k * D.y; part.z -= k * D.z;
         };
         crowd_chunks<PRUNE>(P, gc, __float_as_uint(p4.w), hitcnt[s] > hcap, revcnt[s] > hcap, off, cnt, upbits,
@@ -1030,8 +1038,9 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
 }
 
 // Parameter partials summed per scene in double, in a fixed order: block
-// (chunk, scene) sums its chunk, then one thread per scene adds the chunk
-// sums in chunk order onto the running totals.
+// (chunk, scene) sums its chunk, then one warp per scene adds the chunk sums
+// onto the running totals. Few blocks run, so a thread's loads wait together
+// (one by one: 12 us at 65,536 points).
 __global__ void __launch_bounds__(kReduceThreads)
 k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, const int *__restrict__ sn,
                 int nchunks, double *__restrict__ partial) {
@@ -1039,9 +1048,15 @@ k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, co
     const int b = sbase[scene], m = sn[scene];
     const int lo = chunk * kReduceChunk;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int k = lo + (int)threadIdx.x; k < lo + kReduceChunk && k < m; k += kReduceThreads) {
-        const float4 v = pc[b + k];
-        a0 += (double)v.x; a1 += (double)v.y; a2 += (double)v.z;
+    float4 v[kReduceChunk / kReduceThreads];   // all requested before the first is used
+#pragma unroll
+    for (int k = 0; k < kReduceChunk / kReduceThreads; k++) {
+        const int at = lo + k * kReduceThreads + (int)threadIdx.x;
+        v[k] = at < m ? pc[b + at] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kReduceChunk / kReduceThreads; k++) {
+        a0 += (double)v[k].x; a1 += (double)v[k].y; a2 += (double)v[k].z;
     }
     for (int d = 16; d > 0; d >>= 1) {
         a0 += __shfl_down_sync(0xffffffffu, a0, d);
@@ -1247,8 +1262,8 @@ int fl_launch_adj_advance(fl_system *s, const float *time_ptr, const float4 *for
 
 static int crowd_grid(const fl_system *s) { return 4 * s->num_sms; }
 
-int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4 *xa, const float4 *ea, float *rb,
-                        float4 *pc, float4 *e_out, uint32_t *revlist, uint32_t *revcnt, uint32_t *crowd,
+int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4 *xa, float4 *ea, float4 *pc,
+                        float4 *e_out, uint32_t *revlist, uint32_t *revcnt, uint32_t *crowd,
                         uint32_t *crowd_count, uint32_t *revlong, uint32_t *revlong_count) {
     if (s->n == 0) return FL_OK;
     if (s->max_points > (int)kSlotMask)
@@ -1284,30 +1299,30 @@ int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4
     kern<<<blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream>>>(
         s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
         rr, s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitlist,
-        s->hitcnt, s->src, fb, xa, ea, rb, pc, e_out, revlist, revcnt, CrowdList{crowd, crowd_count, (uint32_t)s->n});
+        s->hitcnt, s->src, fb, xa, ea, pc, e_out, revlist, revcnt, CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_force");
     auto crowd_kern = pr ? k_adj_crowd_force<true> : k_adj_crowd_force<false>;
     crowd_kern<<<crowd_grid(s), kCrowdThreads, 0, s->stream>>>(
         s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(), rr,
-        s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitcnt, revcnt, s->src, fb, xa, e_out, rb, pc,
+        s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitcnt, revcnt, s->src, fb, xa, e_out, ea, pc,
         CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_crowd_force");
     return FL_OK;
 }
 
-int fl_launch_adj_density(fl_system *s, const uint32_t *revlist, const uint32_t *revcnt, const float *rb,
+int fl_launch_adj_density(fl_system *s, const uint32_t *revlist, const uint32_t *revcnt, const float4 *xr,
                           const float4 *xa, float4 *x_out, uint32_t *crowd, uint32_t *crowd_count) {
     if (s->n == 0) return FL_OK;
     const bool pr = adj_prune(s);
     auto kern = pr ? k_adj_density<true> : k_adj_density<false>;
     kern<<<blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-        s->cnt, s->upbits, s->hitlist, s->hitcnt, revlist, revcnt, s->src, rb, xa, x_out, false);
+        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), xr, s->f[F_GCELL].cur<uint32_t>(), s->off,
+        s->cnt, s->upbits, s->hitlist, s->hitcnt, revlist, revcnt, s->src, xa, x_out, false);
     FL_LAUNCH_CHECK("adj_density");
     auto crowd_kern = pr ? k_adj_crowd_density<true> : k_adj_crowd_density<false>;
     crowd_kern<<<crowd_grid(s), kCrowdThreads, 0, s->stream>>>(
         s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits,
-        s->hitcnt, revcnt, s->src, rb, x_out, CrowdList{crowd, crowd_count, (uint32_t)s->n});
+        s->hitcnt, revcnt, s->src, xr, x_out, CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_crowd_density");
     return FL_OK;
 }

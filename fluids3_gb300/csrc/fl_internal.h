@@ -254,10 +254,11 @@ int fl_launch_adj_advance(fl_system *s, const float *time_ptr, const float4 *for
 // (capacity n; the count starts at zero); revlong / revlong_count: the
 // points whose transposed reverse lists are walked again (capacity n; the
 // count starts at zero)
-int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4 *xa, const float4 *ea, float *rb,
-                        float4 *pc, float4 *e_out, uint32_t *revlist, uint32_t *revcnt, uint32_t *crowd,
+// ea: dL/dE in, (position, dL/drho) out, fl_launch_adj_density's xr.
+int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4 *xa, float4 *ea, float4 *pc,
+                        float4 *e_out, uint32_t *revlist, uint32_t *revcnt, uint32_t *crowd,
                         uint32_t *crowd_count, uint32_t *revlong, uint32_t *revlong_count);
-int fl_launch_adj_density(fl_system *s, const uint32_t *revlist, const uint32_t *revcnt, const float *rb,
+int fl_launch_adj_density(fl_system *s, const uint32_t *revlist, const uint32_t *revcnt, const float4 *xr,
                           const float4 *xa, float4 *x_out, uint32_t *crowd, uint32_t *crowd_count);
 int fl_param_chunks(int max_scene_points);
 // acc += partial sums x 2^gexp (gexp null: x 1)

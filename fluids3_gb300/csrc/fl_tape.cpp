@@ -37,7 +37,6 @@ struct fl_tape {
     float4 *g[2][3];        // adjoint of (pos, vel, veval), ping-pong across steps
     int gcur;
     float4 *xa, *ea, *fb, *pc;
-    float *rb;
     float2 *rr;                   // per slot: density and its reciprocal
     uint32_t *revlist, *revcnt;   // reverse pairs (transposed pair lists), for both pair adjoints
     uint32_t *crowd, *crowd_count; // points whose pair lists overflowed (count cleared per reverse step)
@@ -66,7 +65,7 @@ static void tape_release(fl_tape *t) {
         cudaFree(t->ident[k]);
         for (int j = 0; j < 3; j++) cudaFree(t->g[k][j]);
     }
-    cudaFree(t->xa); cudaFree(t->ea); cudaFree(t->fb); cudaFree(t->pc); cudaFree(t->rb);
+    cudaFree(t->xa); cudaFree(t->ea); cudaFree(t->fb); cudaFree(t->pc);
     cudaFree(t->revlist); cudaFree(t->revcnt); cudaFree(t->rr);
     cudaFree(t->crowd); cudaFree(t->crowd_count); cudaFree(t->revlong);
     cudaFree(t->partial); cudaFree(t->acc); cudaFree(t->sbase); cudaFree(t->sn);
@@ -167,7 +166,6 @@ extern "C" int fl_tape_begin_ex(fl_system *s, int max_steps, int every, int flag
         if ((r = fl_dalloc((void **)&t->ea, 16 * cap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&t->fb, 16 * cap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&t->pc, 16 * cap)) != FL_OK) break;
-        if ((r = fl_dalloc((void **)&t->rb, 4 * cap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&t->revcnt, 4 * cap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&t->crowd, 4 * cap)) != FL_OK) break;
         if ((r = fl_dalloc((void **)&t->revlong, 4 * cap)) != FL_OK) break;
@@ -318,9 +316,9 @@ static int backward_step(fl_system *s, fl_tape *t, const float4 *state, const fl
         FL_CUDA_TRY(cudaMemsetAsync(t->crowd_count, 0, 2 * sizeof(uint32_t), s->stream));
         FL_TRY(fl_launch_adj_advance(s, t->time + k, force, t->g[c][0], t->g[c][1], t->g[c][2], t->xa, t->ea,
                                      t->fb, t->g[x][1], t->rr));
-        FL_TRY(fl_launch_adj_force(s, t->rr, t->fb, t->xa, t->ea, t->rb, t->pc, t->g[x][2], t->revlist,
+        FL_TRY(fl_launch_adj_force(s, t->rr, t->fb, t->xa, t->ea, t->pc, t->g[x][2], t->revlist,
                                    t->revcnt, t->crowd, t->crowd_count, t->revlong, t->crowd_count + 1));
-        FL_TRY(fl_launch_adj_density(s, t->revlist, t->revcnt, t->rb, t->xa, t->g[x][0], t->crowd,
+        FL_TRY(fl_launch_adj_density(s, t->revlist, t->revcnt, t->ea, t->xa, t->g[x][0], t->crowd,
                                      t->crowd_count));
         FL_TRY(fl_launch_param_reduce(s, t->pc, t->sbase, t->sn, t->nchunks, t->partial, t->gexp, t->acc));
         FL_TRY(fl_launch_adj_rescale(s, t->g[x][0], t->g[x][1], t->g[x][2], t->gmax, t->gexp));
