@@ -177,6 +177,7 @@ k_adj_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, con
               const float4 *__restrict__ xo_b, const float4 *__restrict__ vo_b, const float4 *__restrict__ eo_b,
               float4 *__restrict__ xa, float4 *__restrict__ ea, float4 *__restrict__ fb,
               float4 *__restrict__ v_out, float2 *__restrict__ rr) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const DevParams &P = scene_params(P0, T, s);
@@ -506,6 +507,7 @@ k_adj_revwalk(const __grid_constant__ DevParams P0, const SceneTab T, int n, con
               const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
               const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
               uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+    follow_previous();
     extern __shared__ uint32_t s_dyn[];
     const int s = PRUNE ? band_grouped_slot(n, pos, gcell, 0, s_dyn) : (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (s >= n) return;
@@ -521,6 +523,7 @@ k_adj_revwalk_listed(const __grid_constant__ DevParams P0, const SceneTab T, con
                      const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
                      const uint32_t *__restrict__ listed, const uint32_t *__restrict__ listed_count,
                      uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+    follow_previous();
     const uint32_t m = *listed_count;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
         const int s = (int)listed[k];
@@ -547,6 +550,7 @@ k_adj_revscatter(const __grid_constant__ DevParams P0, const SceneTab T, int n, 
                  const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
                  const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
                  uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+    follow_previous();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     const uint32_t gq = gcell[q];
@@ -625,6 +629,7 @@ __device__ __forceinline__ void sort_row(uint32_t *row, uint32_t c) {   // entry
 __global__ void __launch_bounds__(kThreads)
 k_adj_revsort(int n, int hcap_in, uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt,
               uint32_t *__restrict__ listed, uint32_t *__restrict__ listed_count) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= (unsigned)n) return;   // whole warp past n
     const uint32_t hcap = (uint32_t)hcap_in;
@@ -671,6 +676,7 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
             const float4 *__restrict__ fb, float4 *__restrict__ xa, float4 *ea, float4 *__restrict__ pc,
             float4 *__restrict__ e_out,
             const uint32_t *__restrict__ revlist, const uint32_t *__restrict__ revcnt, const CrowdList crowd) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = scene_params(P0, T, s < n ? s : 0);
     const uint32_t gc = (s < n) ? gcell[s] : kUndef;
@@ -755,6 +761,7 @@ k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
               const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revlist,
               const uint32_t *__restrict__ revcnt, const uint32_t *__restrict__ src,
               const float4 *__restrict__ xa, float4 *__restrict__ x_out, bool walk_overflow) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const DevParams &P = scene_params(P0, T, s);
@@ -932,6 +939,7 @@ k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const 
                   const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
                   const uint32_t *__restrict__ src, const float4 *__restrict__ fb, float4 *__restrict__ xa,
                   float4 *__restrict__ e_out, float4 *__restrict__ xr, float4 *__restrict__ pc, const CrowdList L) {
+    follow_previous();
     __shared__ float s_red[kCrowdThreads / 32][10];
     __shared__ uint32_t s_nlist;
     if (threadIdx.x == 0) s_nlist = min(*(volatile uint32_t *)L.count, L.cap);
@@ -986,6 +994,7 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
                     const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
                     const uint32_t *__restrict__ src, const float4 *__restrict__ xr, float4 *__restrict__ x_out,
                     const CrowdList L) {
+    follow_previous();
     __shared__ float s_red[kCrowdThreads / 32][3];
     __shared__ uint32_t s_nlist;
     if (threadIdx.x == 0) s_nlist = min(*(volatile uint32_t *)L.count, L.cap);
@@ -1044,6 +1053,7 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
 __global__ void __launch_bounds__(kReduceThreads)
 k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, const int *__restrict__ sn,
                 int nchunks, double *__restrict__ partial) {
+    follow_previous();
     const int chunk = blockIdx.x, scene = blockIdx.y;
     const int b = sbase[scene], m = sn[scene];
     const int lo = chunk * kReduceChunk;
@@ -1076,6 +1086,7 @@ k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, co
 
 __global__ void k_param_final(int nscenes, int nchunks, const double *__restrict__ partial,
                               const int *__restrict__ gexp, double *__restrict__ acc) {
+    follow_previous();
     // one warp per scene: lane l takes chunks l, l+32, ...; fixed shuffle tree
     const int scene = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (scene >= nscenes) return;
@@ -1123,6 +1134,7 @@ __device__ __forceinline__ uint32_t gmax_bits(const float4 a, const float4 b, co
 __global__ void __launch_bounds__(kGmaxThreads)
 k_adj_gmax(int n, const uint16_t *__restrict__ point_scene, const float4 *__restrict__ gx,
            const float4 *__restrict__ gv, const float4 *__restrict__ ge, uint32_t *__restrict__ gmax) {
+    follow_previous();
     __shared__ uint32_t s_max[kGmaxThreads / 32];
     const int b0 = blockIdx.x * kGmaxPoints;
     const int last = min(b0 + kGmaxPoints, n) - 1;
@@ -1173,6 +1185,7 @@ __device__ __forceinline__ int rescale_exponent(uint32_t bits) {
 __global__ void __launch_bounds__(kThreads)
 k_adj_rescale(int n, const uint16_t *__restrict__ point_scene, float4 *__restrict__ gx, float4 *__restrict__ gv,
               float4 *__restrict__ ge, const uint32_t *__restrict__ gmax) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int k = rescale_exponent(gmax[point_scene ? point_scene[i] : 0u]);
@@ -1190,6 +1203,7 @@ k_adj_rescale(int n, const uint16_t *__restrict__ point_scene, float4 *__restric
 __global__ void __launch_bounds__(kThreads)
 k_adj_apply_exponent(int n, const uint16_t *__restrict__ point_scene, float4 *__restrict__ gx,
                      float4 *__restrict__ gv, float4 *__restrict__ ge, const int *__restrict__ gexp) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int k = gexp[point_scene ? point_scene[i] : 0u];
@@ -1202,6 +1216,7 @@ k_adj_apply_exponent(int n, const uint16_t *__restrict__ point_scene, float4 *__
 }
 
 __global__ void k_adj_bump(int nscenes, uint32_t *__restrict__ gmax, int *__restrict__ gexp) {
+    follow_previous();
     const int sc = blockIdx.x * blockDim.x + threadIdx.x;
     if (sc >= nscenes) return;
     gexp[sc] += rescale_exponent(gmax[sc]);
@@ -1212,6 +1227,7 @@ __global__ void k_adj_bump(int nscenes, uint32_t *__restrict__ gmax, int *__rest
 // out = src; src null: the identity).
 __global__ void k_compose(int n, const uint32_t *__restrict__ src, const uint32_t *__restrict__ in,
                           uint32_t *__restrict__ out) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     out[s] = src ? (in ? in[src[s]] : src[s]) : (uint32_t)s;
@@ -1226,6 +1242,7 @@ struct Copy3 {
 };
 
 __global__ void __launch_bounds__(kThreads) k_copy3(int n, const __grid_constant__ Copy3 c) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     for (int k = 0; k < c.count; k++) c.dst[k][i] = c.src[k][i];
@@ -1241,7 +1258,7 @@ int fl_launch_copy3(fl_system *s, int n, int count, const float4 *const *src, fl
     Copy3 c = {};
     c.count = count;
     for (int k = 0; k < count && k < 3; k++) { c.src[k] = src[k]; c.dst[k] = dst[k]; }
-    k_copy3<<<blocks_for(n, kThreads), kThreads, 0, s->stream>>>(n, c);
+    launch(k_copy3, blocks_for(n, kThreads), kThreads, 0, s->stream, n, c);
     FL_LAUNCH_CHECK("copy3");
     return FL_OK;
 }
@@ -1275,9 +1292,9 @@ int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4
                       (s->adj_revmode == FL_REVERSE_AUTO && s->n < FL_REVERSE_TRANSPOSE_MIN);
     if (walk) {
         auto walk = pr ? k_adj_revwalk<true> : k_adj_revwalk<false>;
-        walk<<<blocks_for(s->n, kThreads), kThreads, grouping_smem(kThreads, kBandKeys), s->stream>>>(
-            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
-            s->upbits, revlist, revcnt);
+        launch(walk, blocks_for(s->n, kThreads), kThreads, grouping_smem(kThreads, kBandKeys), s->stream, s->D,
+               fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
+               s->upbits, revlist, revcnt);
         FL_LAUNCH_CHECK("adj_revwalk");
     } else {
         FL_CUDA_TRY(cudaMemsetAsync(revcnt, 0, 4 * (size_t)s->n, s->stream));
@@ -1286,26 +1303,24 @@ int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4
             s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
             s->upbits, s->hitlist, s->hitcnt, revlist, revcnt);
         FL_LAUNCH_CHECK("adj_revscatter");
-        k_adj_revsort<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(s->n, s->D.hcap, revlist, revcnt,
-                                                                              revlong, revlong_count);
+        launch(k_adj_revsort, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->n, s->D.hcap, revlist, revcnt,
+               revlong, revlong_count);
         FL_LAUNCH_CHECK("adj_revsort");
         auto listed = pr ? k_adj_revwalk_listed<true> : k_adj_revwalk_listed<false>;
-        listed<<<crowd_grid(s), kThreads, 0, s->stream>>>(
-            s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
-            s->upbits, revlong, revlong_count, revlist, revcnt);
+        launch(listed, crowd_grid(s), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(),
+               s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, revlong, revlong_count, revlist, revcnt);
         FL_LAUNCH_CHECK("adj_revwalk_listed");
     }
     auto kern = pr ? k_adj_force<true> : k_adj_force<false>;
-    kern<<<blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
-        rr, s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitlist,
-        s->hitcnt, s->src, fb, xa, ea, pc, e_out, revlist, revcnt, CrowdList{crowd, crowd_count, (uint32_t)s->n});
+    launch(kern, blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+           s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(), rr, s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
+           s->upbits, s->hitlist, s->hitcnt, s->src, fb, xa, ea, pc, e_out, revlist, revcnt,
+           CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_force");
     auto crowd_kern = pr ? k_adj_crowd_force<true> : k_adj_crowd_force<false>;
-    crowd_kern<<<crowd_grid(s), kCrowdThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(), rr,
-        s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitcnt, revcnt, s->src, fb, xa, e_out, ea, pc,
-        CrowdList{crowd, crowd_count, (uint32_t)s->n});
+    launch(crowd_kern, crowd_grid(s), kCrowdThreads, 0, s->stream, s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(),
+           s->f[F_VEVAL].cur<float4>(), rr, s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitcnt,
+           revcnt, s->src, fb, xa, e_out, ea, pc, CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_crowd_force");
     return FL_OK;
 }
@@ -1315,14 +1330,14 @@ int fl_launch_adj_density(fl_system *s, const uint32_t *revlist, const uint32_t 
     if (s->n == 0) return FL_OK;
     const bool pr = adj_prune(s);
     auto kern = pr ? k_adj_density<true> : k_adj_density<false>;
-    kern<<<blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), xr, s->f[F_GCELL].cur<uint32_t>(), s->off,
-        s->cnt, s->upbits, s->hitlist, s->hitcnt, revlist, revcnt, s->src, xa, x_out, false);
+    launch(kern, blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+           s->f[F_POS].cur<float4>(), xr, s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitlist,
+           s->hitcnt, revlist, revcnt, s->src, xa, x_out, false);
     FL_LAUNCH_CHECK("adj_density");
     auto crowd_kern = pr ? k_adj_crowd_density<true> : k_adj_crowd_density<false>;
-    crowd_kern<<<crowd_grid(s), kCrowdThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits,
-        s->hitcnt, revcnt, s->src, xr, x_out, CrowdList{crowd, crowd_count, (uint32_t)s->n});
+    launch(crowd_kern, crowd_grid(s), kCrowdThreads, 0, s->stream, s->D, fl_scene_tab(s), s->f[F_POS].cur<float4>(),
+           s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitcnt, revcnt, s->src, xr, x_out,
+           CrowdList{crowd, crowd_count, (uint32_t)s->n});
     FL_LAUNCH_CHECK("adj_crowd_density");
     return FL_OK;
 }
@@ -1335,9 +1350,9 @@ int fl_launch_param_reduce(fl_system *s, const float4 *pc, const int *sbase, con
                            double *partial, const int *gexp, double *acc) {
     if (s->n == 0) return FL_OK;
     dim3 grid((unsigned)nchunks, (unsigned)s->nscenes);
-    k_param_partial<<<grid, kReduceThreads, 0, s->stream>>>(pc, sbase, sn, nchunks, partial);
+    launch(k_param_partial, grid, kReduceThreads, 0, s->stream, pc, sbase, sn, nchunks, partial);
     FL_LAUNCH_CHECK("param_partial");
-    k_param_final<<<blocks_for(s->nscenes, 4), 128, 0, s->stream>>>(s->nscenes, nchunks, partial, gexp, acc);
+    launch(k_param_final, blocks_for(s->nscenes, 4), 128, 0, s->stream, s->nscenes, nchunks, partial, gexp, acc);
     FL_LAUNCH_CHECK("param_final");
     return FL_OK;
 }
@@ -1353,11 +1368,11 @@ int fl_launch_adj_apply_exponent(fl_system *s, float4 *gx, float4 *gv, float4 *g
 int fl_launch_adj_rescale(fl_system *s, float4 *gx, float4 *gv, float4 *ge, uint32_t *gmax, int *gexp) {
     if (s->n == 0) return FL_OK;
     const uint16_t *ps = s->batched ? s->point_scene : nullptr;
-    k_adj_gmax<<<blocks_for(s->n, kGmaxPoints), kGmaxThreads, 0, s->stream>>>(s->n, ps, gx, gv, ge, gmax);
+    launch(k_adj_gmax, blocks_for(s->n, kGmaxPoints), kGmaxThreads, 0, s->stream, s->n, ps, gx, gv, ge, gmax);
     FL_LAUNCH_CHECK("adj_gmax");
-    k_adj_rescale<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(s->n, ps, gx, gv, ge, gmax);
+    launch(k_adj_rescale, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->n, ps, gx, gv, ge, gmax);
     FL_LAUNCH_CHECK("adj_rescale");
-    k_adj_bump<<<blocks_for(s->nscenes, 128), 128, 0, s->stream>>>(s->nscenes, gmax, gexp);
+    launch(k_adj_bump, blocks_for(s->nscenes, 128), 128, 0, s->stream, s->nscenes, gmax, gexp);
     FL_LAUNCH_CHECK("adj_bump");
     return FL_OK;
 }

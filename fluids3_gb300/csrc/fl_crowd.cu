@@ -249,6 +249,7 @@ template <bool BATCH, bool ADVANCE>
 __global__ void __launch_bounds__(kCrowdThreads, BATCH ? 2 : 0)
 k_force_crowd(const __grid_constant__ DevParams P0, const SceneTab T, int n, const __grid_constant__ ForceArgs a,
               uint32_t line, bool ends) {
+    follow_previous();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     __shared__ uint32_t s_next;
     volatile uint32_t *const counters = a.tiles.counters;
@@ -271,6 +272,7 @@ template <bool BATCH, bool ADVANCE>
 __global__ void __launch_bounds__(kAloneThreads)
 k_force_alone(const __grid_constant__ DevParams P0, const SceneTab T, int n, const __grid_constant__ ForceArgs a,
               uint32_t line) {
+    follow_previous();
     __shared__ AloneShared s_sh[kAloneThreads / 32];
     volatile uint32_t *const counters = a.tiles.counters;
     const uint32_t crowded = counters[0], packed = counters[1];
@@ -323,12 +325,13 @@ int fl_launch_force_crowd(fl_system *s, bool advance, float dt, float *host_pos)
     const bool ends = (uint32_t)tiles < line;   // too few points for a class of that many tiles
     auto kern = advance ? (s->batched ? k_force_crowd<true, true> : k_force_crowd<false, true>)
                         : (s->batched ? k_force_crowd<true, false> : k_force_crowd<false, false>);
-    kern<<<std::min(2 * s->num_sms, tiles), kCrowdThreads, kCrowdSmem, s->stream>>>(s->D, fl_scene_tab(s), s->n, a,
-                                                                                    line, ends);
+    launch(kern, std::min(2 * s->num_sms, tiles), kCrowdThreads, kCrowdSmem, s->stream, s->D, fl_scene_tab(s), s->n,
+           a, line, ends);
     if (!ends) {
         auto alone = advance ? (s->batched ? k_force_alone<true, true> : k_force_alone<false, true>)
                              : (s->batched ? k_force_alone<true, false> : k_force_alone<false, false>);
-        alone<<<kAloneBlocksPerSm * s->num_sms, kAloneThreads, 0, s->stream>>>(s->D, fl_scene_tab(s), s->n, a, line);
+        launch(alone, kAloneBlocksPerSm * s->num_sms, kAloneThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n, a,
+               line);
     }
     FL_LAUNCH_CHECK("force_crowd");
     return FL_OK;

@@ -444,6 +444,7 @@ k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, co
                const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
                float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
                float4 *__restrict__ pairdata) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
     const uint32_t gc = (i < n) ? gcell[i] : kUndef;
@@ -556,6 +557,7 @@ k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const f
           const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
           float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
           float4 *__restrict__ pairdata, const CrowdTiles tiles, int workers) {
+    follow_previous();
     extern __shared__ __align__(16) uint32_t s_dyn[];
     if ((int)blockIdx.x < workers) {
         __shared__ uint32_t s_next;
@@ -625,16 +627,15 @@ int fl_launch_density(fl_system *s) {
     const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
     if (rows) {
         auto kern = s->batched ? k_density_rows<true> : k_density_rows<false>;
-        kern<<<blocks_for(s->n, bs), bs, (size_t)(bs / 32) * 32 * kRing * sizeof(uint32_t), s->stream>>>(
-            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-            s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
+        launch(kern, blocks_for(s->n, bs), bs, (size_t)(bs / 32) * 32 * kRing * sizeof(uint32_t), s->stream, s->D,
+               fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
+               s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
     } else {
         const int workers = s->tiles_listed ? std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32) : 0;
         auto kern = s->batched ? k_density<true> : k_density<false>;
-        kern<<<workers + blocks_for(s->n, bs), bs, smem, s->stream>>>(
-            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-            s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata,
-            s->tiles, workers);
+        launch(kern, workers + blocks_for(s->n, bs), bs, smem, s->stream, s->D, fl_scene_tab(s), s->n,
+               s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),
+               s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata, s->tiles, workers);
         s->tiles_listed = 0;   // the list is used up
     }
     FL_LAUNCH_CHECK("density");

@@ -4,6 +4,8 @@
 // pair-list layout. Included inside each file's anonymous namespace.
 #pragma once
 
+#include "fl_launch.cuh"
+
 constexpr int kThreads = 256;
 constexpr uint32_t kUndef = FL_GRID_UNDEF;
 constexpr float kEpsilon = 0.00001f;   // EPSILON, fluids4.0/fluid_kernels.cuh:17

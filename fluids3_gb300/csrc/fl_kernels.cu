@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kThreads)
 k_insert(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
          uint32_t *__restrict__ cell_out, uint32_t *__restrict__ rank_out,
          uint32_t *__restrict__ gcell_out, uint32_t *__restrict__ cnt) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
     uint32_t cell = 0;
@@ -69,6 +70,7 @@ k_insert(const __grid_constant__ DevParams P0, const SceneTab T, int n, const fl
 __global__ void __launch_bounds__(kThreads)
 k_scatter_index(int n, const uint32_t *__restrict__ cell_pre, const uint32_t *__restrict__ rank,
                 const uint32_t *__restrict__ off, uint32_t *__restrict__ src) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     src[off[cell_pre[i]] + rank[i]] = (uint32_t)i;
@@ -171,6 +173,7 @@ constexpr int kSortCells = 4;
 template <int MODE, int CELLS>
 __global__ void __launch_bounds__(kThreads)
 k_sort_cells(const __grid_constant__ SortArgs a) {
+    follow_previous();
     const int c0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * CELLS;
     if (c0 >= a.gcells) return;
     const unsigned lane = lane_id();
@@ -277,6 +280,7 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t 
 template <int MODE>
 __global__ void __launch_bounds__(kBigThreads)
 k_sort_big(const __grid_constant__ SortArgs a) {
+    follow_previous();
     extern __shared__ uint32_t s_keys[];
     __shared__ uint32_t s_nbig;
     if (threadIdx.x == 0) s_nbig = min(*(volatile uint32_t *)a.big_count, a.big_cap);
@@ -398,6 +402,7 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
                 float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, float4 *__restrict__ veval_out,
                 uint32_t *__restrict__ clr_out, uint32_t *__restrict__ gcell_out,
                 uint32_t *__restrict__ gndx_out, uint32_t *__restrict__ upbits, const CrowdTiles tiles) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= (unsigned)n) return;   // whole warp past n
     const bool valid = s < n;
@@ -441,6 +446,7 @@ __global__ void __launch_bounds__(kThreads)
 k_gather_late(int n, const uint32_t *__restrict__ src, const float *__restrict__ vel3,
               const float *__restrict__ veval3, const uint32_t *__restrict__ clr, float4 *__restrict__ vel_out,
               float4 *__restrict__ veval_out, uint32_t *__restrict__ clr_out, float4 *__restrict__ pairdata) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = src[s];
@@ -467,6 +473,7 @@ k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, cons
              float *__restrict__ press_o, uint32_t *__restrict__ clr_o,
              uint32_t *__restrict__ gcell_o, uint32_t *__restrict__ gndx_o, uint32_t *__restrict__ upbits,
              const CrowdTiles tiles) {
+    follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s - (int)lane_id() >= n) return;   // whole warp past n
     uint32_t code = 0, cell = kUndef;
@@ -630,6 +637,7 @@ k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const flo
         const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
         const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
         const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ force) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
     const uint32_t gc = (i < n) ? gcell[i] : kUndef;
@@ -649,6 +657,7 @@ __global__ void __launch_bounds__(kThreads)
 k_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, float time, float dt, float ss,
           const uint32_t *__restrict__ gcell, const float4 *__restrict__ force,
           float4 *__restrict__ pos, float4 *__restrict__ vel, float4 *__restrict__ veval) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const DevParams &P = BATCH ? T.params[T.point_scene[i]] : P0;
@@ -684,6 +693,7 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
                 const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ vel,
                 float4 *__restrict__ force, float4 *__restrict__ pos_out, float4 *__restrict__ veval_out,
                 uint32_t *__restrict__ err, int base, float *__restrict__ host_pos) {
+    follow_previous();
     // host_pos (fl_run_from_host): the new positions also go straight into
     // the caller's page-locked float3 array, in slot order, while the pass
     // runs (each warp's 384 contiguous bytes over the host link)
@@ -717,6 +727,7 @@ struct StateCopy {
 };
 
 __global__ void __launch_bounds__(kThreads) k_copy_state(int n, const __grid_constant__ StateCopy c) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
         *c.time_dst = *c.time_src;
@@ -734,6 +745,7 @@ __global__ void __launch_bounds__(kThreads) k_copy_state(int n, const __grid_con
 __global__ void k_set_word(uint32_t *word, uint32_t value) { *word = value; }
 
 __global__ void k_pack3(int n, const float4 *__restrict__ src, float *__restrict__ dst) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 v = src[i];
@@ -741,6 +753,7 @@ __global__ void k_pack3(int n, const float4 *__restrict__ src, float *__restrict
 }
 
 __global__ void k_unpack3(int n, const float *__restrict__ src, float4 *__restrict__ dst) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     dst[i] = make_float4(src[3 * i + 0], src[3 * i + 1], src[3 * i + 2], 0.0f);
@@ -755,6 +768,7 @@ struct Unpack3Set {
 };
 
 __global__ void k_unpack3_set(int n, const __grid_constant__ Unpack3Set u) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float3 v[4];
@@ -770,6 +784,7 @@ __global__ void k_unpack3_set(int n, const __grid_constant__ Unpack3Set u) {
 // out-of-range bin per earlier scene; the reference layout does not.
 __global__ void k_gcell_ref(int n, const uint32_t *__restrict__ gcell, const uint16_t *__restrict__ scene,
                             uint32_t *__restrict__ out) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t g = gcell[i];
@@ -777,6 +792,7 @@ __global__ void k_gcell_ref(int n, const uint32_t *__restrict__ gcell, const uin
 }
 
 __global__ void k_grid_identity(int n, const uint32_t *__restrict__ gcell, uint32_t *__restrict__ dst) {
+    follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     dst[i] = gcell ? ((gcell[i] != kUndef) ? (uint32_t)i : kUndef) : kUndef;
@@ -796,6 +812,7 @@ __global__ void __launch_bounds__(kConsThreads)
 k_conservation(const __grid_constant__ DevParams P0, const SceneTab T, const int *__restrict__ sbase,
                const int *__restrict__ sn, int nchunks, const float4 *__restrict__ pos,
                const float4 *__restrict__ vel, double *__restrict__ partial) {
+    follow_previous();
     const int chunk = blockIdx.x, scene = blockIdx.y;
     const DevParams &P = T.params ? T.params[scene] : P0;
     const int b = sbase[scene], m = sn[scene];
@@ -838,6 +855,7 @@ __global__ void k_integrity(const __grid_constant__ DevParams P0, const SceneTab
                             const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
                             const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ gndx,
                             unsigned long long *bad) {
+    follow_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= gcells) return;
     const CellCtx cx = cell_ctx<BATCH>(P0, T, g);
@@ -870,8 +888,8 @@ int fl_launch_insert(fl_system *s, uint32_t *gcell_pre_or_null) {
 
 int fl_launch_scatter_index(fl_system *s) {
     if (s->n == 0) return FL_OK;
-    k_scatter_index<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-        s->n, s->cell_pre, s->rank_tmp, s->off, s->src);
+    launch(k_scatter_index, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->n, s->cell_pre, s->rank_tmp,
+           s->off, s->src);
     FL_LAUNCH_CHECK("scatter_index");
     return FL_OK;
 }
@@ -913,15 +931,15 @@ int fl_launch_sort_cells(fl_system *s, int mode, bool late) {
     const int big_grid = (int)std::min<size_t>((size_t)s->num_sms, fl_big_cells_cap(s->n));
     const size_t big_smem = kBigChunk * sizeof(uint32_t);
     if (mode == 0) {
-        sort_kernel(0)<<<grid, bs, 0, s->stream>>>(a);
+        launch(sort_kernel(0), grid, bs, 0, s->stream, a);
         FL_LAUNCH_CHECK("sort_cells");
-        k_sort_big<0><<<big_grid, kBigThreads, big_smem, s->stream>>>(a);
+        launch(k_sort_big<0>, big_grid, kBigThreads, big_smem, s->stream, a);
         FL_LAUNCH_CHECK("sort_big");
         return FL_OK;
     }
-    sort_kernel(1)<<<grid, bs, 0, s->stream>>>(a);
+    launch(sort_kernel(1), grid, bs, 0, s->stream, a);
     FL_LAUNCH_CHECK("sort_cells");
-    k_sort_big<1><<<big_grid, kBigThreads, big_smem, s->stream>>>(a);
+    launch(k_sort_big<1>, big_grid, kBigThreads, big_smem, s->stream, a);
     FL_LAUNCH_CHECK("sort_big");
     if (s->n > 0) {
         const int rows = s->D.prune ? mode : 0;
@@ -932,12 +950,11 @@ int fl_launch_sort_cells(fl_system *s, int mode, bool late) {
                                                 : rows == 1 ? k_gather_sorted<true, 1> : k_gather_sorted<true, 0>)
                                    : (rows == 2 ? k_gather_sorted<false, 2>
                                                 : rows == 1 ? k_gather_sorted<false, 1> : k_gather_sorted<false, 0>);
-        gather<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-            s->D, fl_scene_tab(s), s->n, s->src, s->cell_pre, s->off, s->f[F_POS].cur<float4>(),
-            s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(), s->f[F_CLR].cur<uint32_t>(),
-            s->f[F_POS].nxt<float4>(), s->f[F_VEL].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(),
-            s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits,
-            s->tiles);
+        launch(gather, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n, s->src,
+               s->cell_pre, s->off, s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
+               s->f[F_CLR].cur<uint32_t>(), s->f[F_POS].nxt<float4>(), s->f[F_VEL].nxt<float4>(),
+               s->f[F_VEVAL].nxt<float4>(), s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(),
+               s->f[F_GNDX].nxt<uint32_t>(), s->upbits, s->tiles);
         FL_LAUNCH_CHECK("gather_sorted");
         s->tiles_listed = rows > 0;
     }
@@ -958,14 +975,13 @@ int fl_launch_gather_all(fl_system *s) {
     if (s->n == 0) return FL_OK;
     auto kern = s->batched ? (s->D.prune ? k_gather_all<true, true> : k_gather_all<true, false>)
                            : (s->D.prune ? k_gather_all<false, true> : k_gather_all<false, false>);
-    kern<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->src, s->off,
-        s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
-        s->f[F_FORCE].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_CLR].cur<uint32_t>(),
-        s->f[F_GCELL].cur<uint32_t>(), s->f[F_GNDX].cur<uint32_t>(),
-        s->f[F_POS].nxt<float4>(), s->f[F_VEL].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(),
-        s->f[F_FORCE].nxt<float4>(), s->f[F_PRESS].nxt<float>(), s->f[F_CLR].nxt<uint32_t>(),
-        s->f[F_GCELL].nxt<uint32_t>(), s->f[F_GNDX].nxt<uint32_t>(), s->upbits, s->tiles);
+    launch(kern, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n, s->src, s->off,
+           s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
+           s->f[F_FORCE].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_CLR].cur<uint32_t>(),
+           s->f[F_GCELL].cur<uint32_t>(), s->f[F_GNDX].cur<uint32_t>(), s->f[F_POS].nxt<float4>(),
+           s->f[F_VEL].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(), s->f[F_FORCE].nxt<float4>(),
+           s->f[F_PRESS].nxt<float>(), s->f[F_CLR].nxt<uint32_t>(), s->f[F_GCELL].nxt<uint32_t>(),
+           s->f[F_GNDX].nxt<uint32_t>(), s->upbits, s->tiles);
     FL_LAUNCH_CHECK("gather_all");
     s->codes_valid = 1;
     s->tiles_listed = s->D.prune;
@@ -993,10 +1009,9 @@ int fl_launch_force(fl_system *s) {
     auto kern = s->lists_valid ? (s->batched ? force_kernel<true, true>(pr) : force_kernel<true, false>(pr))
                                : (s->batched ? force_kernel<false, true>(pr) : force_kernel<false, false>(pr));
     const int bs = s->blk_force ? s->blk_force : kForceThreads;
-    kern<<<blocks_for(s->n, bs), bs, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
-        s->f[F_PRESS].cur<float>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits,
-        s->hitlist, s->hitcnt, s->pairdata, s->over_tiles, s->f[F_FORCE].cur<float4>());
+    launch(kern, blocks_for(s->n, bs), bs, 0, s->stream, s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(),
+           s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
+           s->upbits, s->hitlist, s->hitcnt, s->pairdata, s->over_tiles, s->f[F_FORCE].cur<float4>());
     FL_LAUNCH_CHECK("force");
     return s->lists_valid ? fl_launch_force_crowd(s, false, 0.0f, nullptr) : FL_OK;
 }
@@ -1013,12 +1028,11 @@ int fl_launch_force_advance(fl_system *s, float dt, int begin, int end, float *h
     if (begin % bs != 0 || (end != s->n && end % bs != 0) || begin > end)
         return fl_fail(FL_ERR_ARG, "force_advance: slot range [%d, %d) not in whole blocks of %d", begin, end, bs);
     const int count = end - begin;
-    kern<<<blocks_for(count > 0 ? count : 1, bs), bs, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->time_dev, s->time_slot, dt, s->f[F_POS].cur<float4>(),
-        s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-        s->cnt, s->upbits, s->hitlist, s->hitcnt, s->pairdata, s->over_tiles,
-        s->f[F_VEL].cur<float4>(), s->f[F_FORCE].cur<float4>(),
-        s->f[F_POS].nxt<float4>(), s->f[F_VEVAL].nxt<float4>(), s->dev_err, begin, host_pos);
+    launch(kern, blocks_for(count > 0 ? count : 1, bs), bs, 0, s->stream, s->D, fl_scene_tab(s), s->n, s->time_dev,
+           s->time_slot, dt, s->f[F_POS].cur<float4>(), s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(),
+           s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitlist, s->hitcnt, s->pairdata,
+           s->over_tiles, s->f[F_VEL].cur<float4>(), s->f[F_FORCE].cur<float4>(), s->f[F_POS].nxt<float4>(),
+           s->f[F_VEVAL].nxt<float4>(), s->dev_err, begin, host_pos);
     FL_LAUNCH_CHECK("force_advance");
     return s->lists_valid && s->n > 0 ? fl_launch_force_crowd(s, true, dt, host_pos) : FL_OK;
 }
@@ -1026,9 +1040,9 @@ int fl_launch_force_advance(fl_system *s, float dt, int begin, int end, float *h
 int fl_launch_advance(fl_system *s, float time, float dt, float ss) {
     if (s->n == 0) return FL_OK;
     auto kern = s->batched ? k_advance<true> : k_advance<false>;
-    kern<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, time, dt, ss, s->f[F_GCELL].cur<uint32_t>(), s->f[F_FORCE].cur<float4>(),
-        s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>());
+    launch(kern, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n, time, dt, ss,
+           s->f[F_GCELL].cur<uint32_t>(), s->f[F_FORCE].cur<float4>(), s->f[F_POS].cur<float4>(),
+           s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>());
     FL_LAUNCH_CHECK("advance");
     return FL_OK;
 }
@@ -1047,7 +1061,7 @@ int fl_launch_copy_state(fl_system *s, int n, void *const *src, void *const *dst
     c.time_dst = time_dst;
     c.epoch = new_epoch ? s->crowd_epoch : nullptr;
     c.epoch_value = s->auto_epoch;
-    k_copy_state<<<blocks_for(n > 0 ? n : 1, kThreads), kThreads, 0, s->stream>>>(n, c);
+    launch(k_copy_state, blocks_for(n > 0 ? n : 1, kThreads), kThreads, 0, s->stream, n, c);
     FL_LAUNCH_CHECK("copy_state");
     return FL_OK;
 }

@@ -20,6 +20,8 @@
 
 namespace {
 
+#include "fl_launch.cuh"
+
 constexpr int kThreads = 256;
 constexpr int kItems = 16;
 constexpr int kTile = kThreads * kItems;   // 4096 counts per tile
@@ -73,6 +75,7 @@ __global__ void __launch_bounds__(kThreads)
 k_scan(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, uint64_t *status,
        uint32_t *ticket, int ntiles, uint32_t epoch, int inclusive, uint32_t *err, int spin_limit,
        uint32_t first_tile) {
+    follow_previous();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[kThreads / 32];
     __shared__ uint32_t s_prefix;
@@ -158,9 +161,8 @@ int fl_launch_scan(fl_system *s, int count) {
     const int ntiles = (int)((count + kTile - 1) / kTile);
     if (ntiles > s->scan_tiles)
         return fl_fail(FL_ERR_ARG, "scan: %d tiles exceed the %d allocated", ntiles, s->scan_tiles);
-    k_scan<<<ntiles, kThreads, 0, s->stream>>>(s->cnt, s->off, s->scan_status, s->scan_ticket,
-                                               ntiles, s->scan_epoch, /*inclusive=*/0,
-                                               s->dev_err, kSpinLimit, 0u);
+    launch(k_scan, ntiles, kThreads, 0, s->stream, s->cnt, s->off, s->scan_status, s->scan_ticket, ntiles,
+           s->scan_epoch, /*inclusive=*/0, s->dev_err, kSpinLimit, 0u);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fl_fail(FL_ERR_CUDA, "scan launch: %s", cudaGetErrorString(e));
     return FL_OK;
