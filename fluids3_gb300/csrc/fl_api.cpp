@@ -786,8 +786,8 @@ extern "C" int fl_import_device(fl_system *s, int n, const void *dev_pos, const 
 
 static int clear_grid(fl_system *s) {
     // InsertParticlesCUDA clears FGRIDCNT/FGRIDOFF (cpp:2336-2337); here one
-    // memset clears the counts, the scan ticket and the scan descriptors.
-    FL_CUDA_TRY(cudaMemsetAsync(s->cnt, 0, grid_block_bytes(s), s->stream));
+    // launch clears the counts, the scan ticket and the scan descriptors.
+    FL_TRY(fl_launch_clear(s, s->cnt, grid_block_bytes(s) / 8));
     s->tiles_listed = 0;
     return FL_OK;
 }

@@ -271,6 +271,7 @@ int fl_launch_adj_apply_exponent(fl_system *s, float4 *gx, float4 *gv, float4 *g
 int fl_launch_compose(fl_system *s, int n, const uint32_t *src, const uint32_t *in, uint32_t *out);
 // dst[k][0..n) = src[k][0..n) for k < count (<= 3), one kernel pass
 int fl_launch_copy3(fl_system *s, int n, int count, const float4 *const *src, float4 *const *dst);
+int fl_launch_clear(fl_system *s, void *p, size_t words);   // eight-byte words
 int fl_launch_insert(fl_system *s, uint32_t *gcell_pre_or_null);
 int fl_launch_scan(fl_system *s, int count);
 int fl_launch_scatter_index(fl_system *s);

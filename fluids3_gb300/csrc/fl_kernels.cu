@@ -870,18 +870,37 @@ __global__ void k_integrity(const __grid_constant__ DevParams P0, const SceneTab
     if (b) atomicAdd(bad, b);
 }
 
+// Clears `words` eight-byte words.
+constexpr int kClearWords = 4;   // a thread (and pass)
+__global__ void __launch_bounds__(kThreads) k_clear(unsigned long long *__restrict__ p, size_t words) {
+    follow_previous();
+    for (size_t b = (size_t)blockIdx.x * (kThreads * kClearWords); b < words;
+         b += (size_t)gridDim.x * (kThreads * kClearWords))
+#pragma unroll
+        for (int k = 0; k < kClearWords; k++) {
+            const size_t w = b + (size_t)k * kThreads + threadIdx.x;
+            if (w < words) p[w] = 0;
+        }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // Launch wrappers.
 
 
+int fl_launch_clear(fl_system *s, void *p, size_t words) {
+    const int blocks = std::min(blocks_for((long long)words, kThreads * kClearWords), 16 * s->num_sms);
+    launch(k_clear, blocks, kThreads, 0, s->stream, (unsigned long long *)p, words);
+    FL_LAUNCH_CHECK("clear");
+    return FL_OK;
+}
+
 int fl_launch_insert(fl_system *s, uint32_t *gcell_pre_or_null) {
     if (s->n == 0) return FL_OK;
     auto kern = s->batched ? k_insert<true> : k_insert<false>;
-    kern<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->cell_pre, s->rank_tmp, gcell_pre_or_null,
-        s->cnt);
+    launch(kern, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+           s->f[F_POS].cur<float4>(), s->cell_pre, s->rank_tmp, gcell_pre_or_null, s->cnt);
     FL_LAUNCH_CHECK("insert");
     return FL_OK;
 }
