@@ -176,10 +176,13 @@ k_adj_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, con
               const float4 *__restrict__ F, const float *__restrict__ rho,
               const float4 *__restrict__ xo_b, const float4 *__restrict__ vo_b, const float4 *__restrict__ eo_b,
               float4 *__restrict__ xa, float4 *__restrict__ ea, float4 *__restrict__ fb,
-              float4 *__restrict__ v_out, float2 *__restrict__ rr) {
+              float4 *__restrict__ v_out, float2 *__restrict__ rr, uint32_t *__restrict__ counts,
+              uint32_t *__restrict__ revcnt) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < 2) counts[s] = 0;
     if (s >= n) return;
+    if (revcnt) revcnt[s] = 0;
     const DevParams &P = scene_params(P0, T, s);
     const float3 xb_o = xyz(xo_b[s]), vb_o = xyz(vo_b[s]), eb_o = xyz(eo_b[s]);
     const uint32_t dst = src[s];
@@ -1233,17 +1236,20 @@ __global__ void k_compose(int n, const uint32_t *__restrict__ src, const uint32_
     out[s] = src ? (in ? in[src[s]] : src[s]) : (uint32_t)s;
 }
 
-// Up to three float4 arrays copied in one pass (tape saves and restores):
-// dst_k[i] = src_k[i] for k < count.
-struct Copy3 {
+// What a tape saves or restores at one point of a step, in one pass: up to
+// three float4 arrays of n, and one of `words` 4-byte words.
+struct TapeCopy {
     const float4 *src[3];
     float4 *dst[3];
-    int count;
+    int count, words;
+    const uint32_t *wsrc;
+    uint32_t *wdst;
 };
 
-__global__ void __launch_bounds__(kThreads) k_copy3(int n, const __grid_constant__ Copy3 c) {
+__global__ void __launch_bounds__(kThreads) k_tape_copy(int n, const __grid_constant__ TapeCopy c) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < c.words) c.wdst[i] = c.wsrc[i];
     if (i >= n) return;
     for (int k = 0; k < c.count; k++) c.dst[k][i] = c.src[k][i];
 }
@@ -1253,26 +1259,38 @@ __global__ void __launch_bounds__(kThreads) k_copy3(int n, const __grid_constant
 // ---------------------------------------------------------------------------
 // Launch wrappers.
 
-int fl_launch_copy3(fl_system *s, int n, int count, const float4 *const *src, float4 *const *dst) {
-    if (n == 0 || count == 0) return FL_OK;
-    Copy3 c = {};
+int fl_launch_tape_copy(fl_system *s, int count, const float4 *const *src, float4 *const *dst, int words,
+                        const void *wsrc, void *wdst) {
+    const int n = count > 0 ? s->n : 0, most = n > words ? n : words;
+    if (most == 0) return FL_OK;
+    TapeCopy c = {};
     c.count = count;
     for (int k = 0; k < count && k < 3; k++) { c.src[k] = src[k]; c.dst[k] = dst[k]; }
-    launch(k_copy3, blocks_for(n, kThreads), kThreads, 0, s->stream, n, c);
-    FL_LAUNCH_CHECK("copy3");
+    c.words = words;
+    c.wsrc = (const uint32_t *)wsrc;
+    c.wdst = (uint32_t *)wdst;
+    launch(k_tape_copy, blocks_for(most, kThreads), kThreads, 0, s->stream, n, c);
+    FL_LAUNCH_CHECK("tape_copy");
     return FL_OK;
 }
 
 static bool adj_prune(const fl_system *s) { return s->D.prune && s->codes_valid; }
 
+// The transposition saves work but adds three launches: it pays on large
+// systems, where the reverse step is bound by throughput.
+static bool walks_reverse(const fl_system *s) {
+    return s->adj_revmode == FL_REVERSE_WALK ||
+           (s->adj_revmode == FL_REVERSE_AUTO && s->n < FL_REVERSE_TRANSPOSE_MIN);
+}
+
 int fl_launch_adj_advance(fl_system *s, const float *time_ptr, const float4 *force, const float4 *xo_b,
                           const float4 *vo_b, const float4 *eo_b, float4 *xa, float4 *ea, float4 *fb, float4 *v_out,
-                          float2 *rr) {
+                          float2 *rr, uint32_t *counts, uint32_t *revcnt) {
     if (s->n == 0) return FL_OK;
-    k_adj_advance<<<blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream>>>(
-        s->D, fl_scene_tab(s), s->n, time_ptr, s->P.dt, s->f[F_GCELL].cur<uint32_t>(), s->src,
-        s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(),
-        force, s->f[F_PRESS].cur<float>(), xo_b, vo_b, eo_b, xa, ea, fb, v_out, rr);
+    launch(k_adj_advance, blocks_for(s->n, kAdjThreads), kAdjThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+           time_ptr, s->P.dt, s->f[F_GCELL].cur<uint32_t>(), s->src, s->f[F_POS].cur<float4>(),
+           s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>(), force, s->f[F_PRESS].cur<float>(), xo_b, vo_b, eo_b,
+           xa, ea, fb, v_out, rr, counts, walks_reverse(s) ? nullptr : revcnt);
     FL_LAUNCH_CHECK("adj_advance");
     return FL_OK;
 }
@@ -1286,22 +1304,17 @@ int fl_launch_adj_force(fl_system *s, const float2 *rr, const float4 *fb, float4
     if (s->max_points > (int)kSlotMask)
         return fl_fail(FL_ERR_CAPACITY, "adjoint: %d points (at most %u)", s->max_points, kSlotMask);
     const bool pr = adj_prune(s);
-    // the transposition saves work but adds three launches: it pays on
-    // large systems, where the reverse step is bound by throughput
-    const bool walk = s->adj_revmode == FL_REVERSE_WALK ||
-                      (s->adj_revmode == FL_REVERSE_AUTO && s->n < FL_REVERSE_TRANSPOSE_MIN);
-    if (walk) {
+    if (walks_reverse(s)) {
         auto walk = pr ? k_adj_revwalk<true> : k_adj_revwalk<false>;
         launch(walk, blocks_for(s->n, kThreads), kThreads, grouping_smem(kThreads, kBandKeys), s->stream, s->D,
                fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
                s->upbits, revlist, revcnt);
         FL_LAUNCH_CHECK("adj_revwalk");
     } else {
-        FL_CUDA_TRY(cudaMemsetAsync(revcnt, 0, 4 * (size_t)s->n, s->stream));
         auto scatter = pr ? k_adj_revscatter<true> : k_adj_revscatter<false>;
-        scatter<<<blocks_for(s->n, kThreads), kThreads, 0, s->stream>>>(
-            s->D, fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt,
-            s->upbits, s->hitlist, s->hitcnt, revlist, revcnt);
+        launch(scatter, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+               s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->cnt, s->upbits, s->hitlist,
+               s->hitcnt, revlist, revcnt);
         FL_LAUNCH_CHECK("adj_revscatter");
         launch(k_adj_revsort, blocks_for(s->n, kThreads), kThreads, 0, s->stream, s->n, s->D.hcap, revlist, revcnt,
                revlong, revlong_count);
@@ -1379,7 +1392,7 @@ int fl_launch_adj_rescale(fl_system *s, float4 *gx, float4 *gv, float4 *ge, uint
 
 int fl_launch_compose(fl_system *s, int n, const uint32_t *src, const uint32_t *in, uint32_t *out) {
     if (n == 0) return FL_OK;
-    k_compose<<<blocks_for(n, kThreads), kThreads, 0, s->stream>>>(n, src, in, out);
+    launch(k_compose, blocks_for(n, kThreads), kThreads, 0, s->stream, n, src, in, out);
     FL_LAUNCH_CHECK("compose");
     return FL_OK;
 }

@@ -247,9 +247,10 @@ void fl_tape_touch(fl_system *s);
 void fl_tape_free(fl_system *s);
 
 // ---- launch wrappers (fl_kernels.cu, fl_scan.cu, fl_adjoint.cu) ------------
+// clears counts[0..2) and, when the reverse lists will be transposed, revcnt
 int fl_launch_adj_advance(fl_system *s, const float *time_ptr, const float4 *force, const float4 *xo_b,
                           const float4 *vo_b, const float4 *eo_b, float4 *xa, float4 *ea, float4 *fb, float4 *v_out,
-                          float2 *rr);
+                          float2 *rr, uint32_t *counts, uint32_t *revcnt);
 // crowd / crowd_count: the list of points whose pair lists overflowed
 // (capacity n; the count starts at zero); revlong / revlong_count: the
 // points whose transposed reverse lists are walked again (capacity n; the
@@ -269,8 +270,10 @@ int fl_launch_adj_rescale(fl_system *s, float4 *gx, float4 *gv, float4 *ge, uint
 // the cotangents times 2^gexp of their scene
 int fl_launch_adj_apply_exponent(fl_system *s, float4 *gx, float4 *gv, float4 *ge, const int *gexp);
 int fl_launch_compose(fl_system *s, int n, const uint32_t *src, const uint32_t *in, uint32_t *out);
-// dst[k][0..n) = src[k][0..n) for k < count (<= 3), one kernel pass
-int fl_launch_copy3(fl_system *s, int n, int count, const float4 *const *src, float4 *const *dst);
+// dst[k][0..n) = src[k][0..n) for k < count (<= 3) and wdst[0..words) =
+// wsrc[0..words) (4-byte words), in one launch
+int fl_launch_tape_copy(fl_system *s, int count, const float4 *const *src, float4 *const *dst, int words,
+                        const void *wsrc, void *wdst);
 int fl_launch_clear(fl_system *s, void *p, size_t words);   // eight-byte words
 int fl_launch_insert(fl_system *s, uint32_t *gcell_pre_or_null);
 int fl_launch_scan(fl_system *s, int count);

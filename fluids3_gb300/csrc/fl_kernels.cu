@@ -870,7 +870,9 @@ __global__ void k_integrity(const __grid_constant__ DevParams P0, const SceneTab
     if (b) atomicAdd(bad, b);
 }
 
-// Clears `words` eight-byte words.
+// Clears `words` eight-byte words. (A memset would keep the launches on both
+// sides of it from being dependent ones: gradients of 65,536 points 3,356 us
+// with it, 3,191 without.)
 constexpr int kClearWords = 4;   // a thread (and pass)
 __global__ void __launch_bounds__(kThreads) k_clear(unsigned long long *__restrict__ p, size_t words) {
     follow_previous();

@@ -94,23 +94,31 @@ void fl_tape_touch(fl_system *s) {
 }
 
 // The live (pos, vel, veval) copies to / from a {pos, vel, veval} x cap
-// block, in one kernel pass.
-static int save_state(fl_system *s, const fl_tape *t, float4 *dst) {
+// block, and with a save the step's time to `time`, in one launch.
+static int save_state(fl_system *s, const fl_tape *t, float4 *dst, float *time) {
     const float4 *src[3] = {s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>()};
     float4 *out[3] = {dst, dst + t->cap, dst + 2 * (size_t)t->cap};
-    return fl_launch_copy3(s, s->n, 3, src, out);
+    return fl_launch_tape_copy(s, dst ? 3 : 0, src, out, 1, s->time_dev + s->time_slot, time);
+}
+
+// The same of a replayed step k, whose recorded time is set.
+static int save_replayed(fl_system *s, const fl_tape *t, float4 *dst, int k) {
+    const float4 *src[3] = {s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>()};
+    float4 *out[3] = {dst, dst + t->cap, dst + 2 * (size_t)t->cap};
+    return fl_launch_tape_copy(s, 3, src, out, 1, t->time + k, s->time_dev + s->time_slot);
 }
 
 static int load_state(fl_system *s, const fl_tape *t, const float4 *blk) {
     const float4 *src[3] = {blk, blk + t->cap, blk + 2 * (size_t)t->cap};
     float4 *out[3] = {s->f[F_POS].cur<float4>(), s->f[F_VEL].cur<float4>(), s->f[F_VEVAL].cur<float4>()};
-    return fl_launch_copy3(s, s->n, 3, src, out);
+    return fl_launch_tape_copy(s, 3, src, out, 0, nullptr, nullptr);
 }
 
-static int save_force(fl_system *s, float4 *dst) {
+// The step's force to `dst` (or null) and its densities to `rho` (or null).
+static int save_step(fl_system *s, float4 *dst, float *rho) {
     const float4 *src[1] = {s->f[F_FORCE].cur<float4>()};
     float4 *out[1] = {dst};
-    return fl_launch_copy3(s, s->n, 1, src, out);
+    return fl_launch_tape_copy(s, dst ? 1 : 0, src, out, rho ? s->n : 0, s->f[F_PRESS].cur<void>(), rho);
 }
 
 extern "C" int fl_tape_begin(fl_system *s, int max_steps, int every) {
@@ -221,9 +229,7 @@ int fl_tape_pre_step(fl_system *s) {
         return fl_fail(FL_ERR_CAPACITY, "tape full: it holds %d steps (fl_tape_begin max_steps)", t->max_steps);
     if (k == 0) t->n = s->n;
     else if (s->n != t->n) { t->broken = 1; return FL_OK; }
-    if (k % t->every == 0) FL_TRY(save_state(s, t, t->ck + (size_t)(k / t->every) * 3 * t->cap));
-    FL_CUDA_TRY(cudaMemcpyAsync(t->time + k, s->time_dev + s->time_slot, sizeof(float),
-                                cudaMemcpyDeviceToDevice, s->stream));
+    FL_TRY(save_state(s, t, k % t->every == 0 ? t->ck + (size_t)(k / t->every) * 3 * t->cap : nullptr, t->time + k));
     if (t->keep_lists && t->every == 1) {   // this step's density pass writes into slot k
         t->own_list = s->hitlist;
         t->own_cnt = s->hitcnt;
@@ -235,18 +241,17 @@ int fl_tape_pre_step(fl_system *s) {
 
 int fl_tape_post_step(fl_system *s) {
     fl_tape *t = s->tape;
+    float *rho = nullptr;
     if (t->own_list) {
         s->hitlist = t->own_list;
         s->hitcnt = t->own_cnt;
         t->own_list = t->own_cnt = nullptr;
-        if (!t->broken && s->n)
-            FL_CUDA_TRY(cudaMemcpyAsync(t->seg_rho + (size_t)t->steps * t->cap, s->f[F_PRESS].cur<void>(),
-                                        4 * (size_t)s->n, cudaMemcpyDeviceToDevice, s->stream));
+        rho = t->seg_rho + (size_t)t->steps * t->cap;
     }
     if (t->broken) return FL_OK;
     // every = 1: keep the step's force (sorted order) so the reverse pass
     // need not recompute it
-    if (t->every == 1) FL_TRY(save_force(s, t->force + (size_t)t->steps * t->cap));
+    FL_TRY(save_step(s, t->every == 1 ? t->force + (size_t)t->steps * t->cap : nullptr, rho));
     FL_TRY(fl_launch_compose(s, s->n, s->src, t->steps == 0 ? nullptr : t->ident[t->ident_cur],
                              t->ident[t->ident_cur ^ 1]));
     t->ident_cur ^= 1;
@@ -302,9 +307,8 @@ static int backward_step(fl_system *s, fl_tape *t, const float4 *state, const fl
     uint32_t *own_list = s->hitlist, *own_cnt = s->hitcnt;
     if (slot >= 0) {
         FL_TRY(fl_rebuild_grid(s));
-        if (s->n)
-            FL_CUDA_TRY(cudaMemcpyAsync(s->f[F_PRESS].cur<void>(), t->seg_rho + (size_t)slot * t->cap,
-                                        4 * (size_t)s->n, cudaMemcpyDeviceToDevice, s->stream));
+        FL_TRY(fl_launch_tape_copy(s, 0, nullptr, nullptr, s->n, t->seg_rho + (size_t)slot * t->cap,
+                                   s->f[F_PRESS].cur<void>()));
         s->hitlist = t->seg_list + (size_t)slot * t->list_words;
         s->hitcnt = t->seg_cnt + (size_t)slot * t->cap;
         s->lists_valid = 1;
@@ -313,9 +317,8 @@ static int backward_step(fl_system *s, fl_tape *t, const float4 *state, const fl
     }
     const int c = t->gcur, x = c ^ 1;
     const int r = [&]() {
-        FL_CUDA_TRY(cudaMemsetAsync(t->crowd_count, 0, 2 * sizeof(uint32_t), s->stream));
         FL_TRY(fl_launch_adj_advance(s, t->time + k, force, t->g[c][0], t->g[c][1], t->g[c][2], t->xa, t->ea,
-                                     t->fb, t->g[x][1], t->rr));
+                                     t->fb, t->g[x][1], t->rr, t->crowd_count, t->revcnt));
         FL_TRY(fl_launch_adj_force(s, t->rr, t->fb, t->xa, t->ea, t->pc, t->g[x][2], t->revlist,
                                    t->revcnt, t->crowd, t->crowd_count, t->revlong, t->crowd_count + 1));
         FL_TRY(fl_launch_adj_density(s, t->revlist, t->revcnt, t->ea, t->xa, t->g[x][0], t->crowd,
@@ -347,9 +350,7 @@ static int run_reverse(fl_system *s, fl_tape *t) {
         // state before each step and the force it computed
         FL_TRY(load_state(s, t, ck));
         for (int k = t0; k < t1; k++) {
-            FL_TRY(save_state(s, t, t->seg + (size_t)(k - t0) * blk));
-            FL_CUDA_TRY(cudaMemcpyAsync(s->time_dev + s->time_slot, t->time + k, sizeof(float),
-                                        cudaMemcpyDeviceToDevice, s->stream));
+            FL_TRY(save_replayed(s, t, t->seg + (size_t)(k - t0) * blk, k));
             uint32_t *own_list = s->hitlist, *own_cnt = s->hitcnt;
             if (t->keep_lists) {   // the step's density pass (one that writes pair lists) fills the slot
                 s->hitlist = t->seg_list + (size_t)(k - t0) * t->list_words;
@@ -359,10 +360,8 @@ static int run_reverse(fl_system *s, fl_tape *t) {
             s->hitlist = own_list;
             s->hitcnt = own_cnt;
             FL_TRY(r);
-            FL_TRY(save_force(s, t->force + (size_t)(k - t0) * t->cap));
-            if (t->keep_lists && s->n)
-                FL_CUDA_TRY(cudaMemcpyAsync(t->seg_rho + (size_t)(k - t0) * t->cap, s->f[F_PRESS].cur<void>(),
-                                            4 * (size_t)s->n, cudaMemcpyDeviceToDevice, s->stream));
+            FL_TRY(save_step(s, t->force + (size_t)(k - t0) * t->cap,
+                             t->keep_lists ? t->seg_rho + (size_t)(k - t0) * t->cap : nullptr));
         }
         for (int k = t1 - 1; k >= t0; k--)
             FL_TRY(backward_step(s, t, t->seg + (size_t)(k - t0) * blk, t->force + (size_t)(k - t0) * t->cap, k,
