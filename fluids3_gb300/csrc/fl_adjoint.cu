@@ -48,8 +48,8 @@ constexpr int kAdjThreads = 128;
 __device__ __forceinline__ const DevParams &scene_params(const DevParams &P0, const SceneTab &T, int s) {
     return T.params ? T.params[T.point_scene[s]] : P0;
 }
-constexpr int kReduceThreads = 512;
-constexpr int kReduceChunk = 4096;   // points per partial-sum block
+constexpr int kReduceThreads = 128, kFinalThreads = 384;
+constexpr int kReduceChunk = 1024;   // points per partial-sum block
 
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 
@@ -749,12 +749,11 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 // cells from the list k_adj_revwalk recorded; the finished dL/dX goes
 // through the permutation. A neighbour's position and dL/drho come in one load
 // (xr; two loads took 113 us at 1,200,000 points, one takes 98). With
-// walk_overflow off (as fl_backward launches
-// it) a point whose list overflowed is left to k_adj_crowd_density, which
-// spreads its pairs over a block; on, the point walks them itself. (The
-// per-thread walk is kept compiled in: without it this kernel's list loops
-// were given fewer registers and more resident warps, and ran 40% slower
-// on the wave tank.)
+// walk_overflow off (as fl_backward launches it) a point whose list overflowed
+// is left to k_adj_crowd_density, which spreads its pairs over a block; on,
+// the point walks them itself. (The per-thread walk is kept compiled in:
+// without it this kernel's list loops were given fewer registers and more
+// resident warps, and ran 40% slower on the wave tank.)
 template <bool PRUNE>
 __global__ void __launch_bounds__(kAdjThreads)
 k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
@@ -1050,9 +1049,11 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
 }
 
 // Parameter partials summed per scene in double, in a fixed order: block
-// (chunk, scene) sums its chunk, then one warp per scene adds the chunk sums
-// onto the running totals. Few blocks run, so a thread's loads wait together
-// (one by one: 12 us at 65,536 points).
+// (chunk, scene) sums its chunk, then one block per scene adds the chunk sums
+// onto the running totals. Bound by the FP64 units, two additions a cycle and
+// multiprocessor: chunks of 4,096 points left most multiprocessors idle
+// (65,536 points: 13 us, and 6 for the totals by one warp; gradients of 10
+// steps 3,077 us so, 2,996 with chunks of 1,024 and four warps a total).
 __global__ void __launch_bounds__(kReduceThreads)
 k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, const int *__restrict__ sn,
                 int nchunks, double *__restrict__ partial) {
@@ -1087,19 +1088,26 @@ k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, co
     }
 }
 
-__global__ void k_param_final(int nscenes, int nchunks, const double *__restrict__ partial,
-                              const int *__restrict__ gexp, double *__restrict__ acc) {
+// Warp w adds parameter w % 3 over the chunks w / 3 (mod 4), lane by lane.
+__global__ void __launch_bounds__(kFinalThreads)
+k_param_final(int nchunks, const double *__restrict__ partial, const int *__restrict__ gexp,
+              double *__restrict__ acc) {
     follow_previous();
-    // one warp per scene: lane l takes chunks l, l+32, ...; fixed shuffle tree
-    const int scene = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (scene >= nscenes) return;
-    const unsigned lane = threadIdx.x & 31u;
-    for (int j = 0; j < 3; j++) {
-        double t = 0.0;
-        for (int c = (int)lane; c < nchunks; c += 32) t += partial[((size_t)scene * nchunks + c) * 3 + j];
-        for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+    const int scene = blockIdx.x, w = (int)(threadIdx.x >> 5), j = w % 3;
+    constexpr int kParts = kFinalThreads / 96;
+    __shared__ double s_sum[kParts * 3];
+    double t = 0.0;
+#pragma unroll 4
+    for (int c = (w / 3) * 32 + (int)(threadIdx.x & 31u); c < nchunks; c += kParts * 32)
+        t += partial[((size_t)scene * nchunks + c) * 3 + j];
+    for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+    if ((threadIdx.x & 31u) == 0) s_sum[w] = t;
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        t = s_sum[threadIdx.x];
+        for (int p = 1; p < kParts; p++) t += s_sum[p * 3 + (int)threadIdx.x];
         // the partials carry the cotangent's current scale 2^-gexp
-        if (lane == 0) acc[scene * 3 + j] += gexp ? ldexp(t, gexp[scene]) : t;
+        acc[scene * 3 + (int)threadIdx.x] += gexp ? ldexp(t, gexp[scene]) : t;
     }
 }
 
@@ -1365,7 +1373,7 @@ int fl_launch_param_reduce(fl_system *s, const float4 *pc, const int *sbase, con
     dim3 grid((unsigned)nchunks, (unsigned)s->nscenes);
     launch(k_param_partial, grid, kReduceThreads, 0, s->stream, pc, sbase, sn, nchunks, partial);
     FL_LAUNCH_CHECK("param_partial");
-    launch(k_param_final, blocks_for(s->nscenes, 4), 128, 0, s->stream, s->nscenes, nchunks, partial, gexp, acc);
+    launch(k_param_final, s->nscenes, kFinalThreads, 0, s->stream, nchunks, partial, gexp, acc);
     FL_LAUNCH_CHECK("param_final");
     return FL_OK;
 }

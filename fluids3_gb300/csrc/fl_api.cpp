@@ -110,7 +110,7 @@ static void free_grid(fl_system *s) {
 }
 
 // Grid block: [cnt (grid_pad) | ticket (256 B) | descriptors] in one
-// allocation so one memset clears all of it; off is separate.
+// allocation so one launch clears all of it; off is separate.
 static size_t grid_block_bytes(const fl_system *s) {
     return s->grid_pad * sizeof(uint32_t) + fl_scan_scratch_bytes(s->scan_tiles);
 }
@@ -916,8 +916,9 @@ static int reset_auto(fl_system *s) {
 
 static int run_step(fl_system *s, TimingState *t) {
     // InsertParticles, PrefixSumCells, CountingSortFull, ComputePressure,
-    // ComputeForce + Advance (cpp:507-515) as eight launches (the sort is a
-    // cell sort of the point indices, one for crowded cells, and a gather).
+    // ComputeForce + Advance (cpp:507-515); the sort is a cell sort of the
+    // point indices, one for crowded cells, and a gather, and the force pass
+    // leaves crowded tiles to launches of their own.
     const bool taped = fl_tape_recording(s) != 0;
     if (taped) FL_TRY(fl_tape_pre_step(s));
     FL_TRY(record(s, t, 0));

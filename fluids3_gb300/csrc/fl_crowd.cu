@@ -25,8 +25,8 @@ namespace {
 constexpr int kCrowdThreads = 512;   // (256: 5-20% slower; 128: half as fast)
 constexpr int kCrowdSlots = 8;       // candidates a warp and round
 // From this many tiles a multiprocessor in a class (twice as many of the packed
-// ones, which differ more), a warp takes each by itself: nothing is lost to the adding warp and the waits on it, and there is
-// work for every warp. Force + advance, dam break of 1,048,576 points after
+// ones, which differ more), a warp takes each by itself: nothing is lost to the
+// adding warp and the waits on it, and there is work for every warp. Force + advance, dam break of 1,048,576 points after
 // 110 and 170 steps, shared | alone: 1,562 | 944, 12,711 | 7,775 us; of 131,072
 // after 170 steps (a line at 8 a multiprocessor) 2,640 | 5,978 us.
 constexpr uint32_t kAloneTiles = 16;

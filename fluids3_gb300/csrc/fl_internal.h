@@ -112,7 +112,7 @@ struct fl_system {
 
     // grid: C + 1 entries (entry C is the out-of-range bin), padded to whole
     // scan tiles. One allocation holds [cnt | scan ticket | scan descriptors]
-    // so a single memset clears all three at the start of a step.
+    // so a single launch clears all three at the start of a step.
     uint32_t *cnt;
     uint32_t *off;
     size_t grid_pad;

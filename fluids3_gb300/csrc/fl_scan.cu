@@ -9,8 +9,8 @@
 // at a time, until it meets an inclusive prefix. A descriptor is 64 bits:
 //   [63:62] flag (1 = aggregate, 2 = inclusive prefix), [61:32] launch
 //   epoch, [31:0] value.
-// The host zeroes the descriptors and the ticket before every launch (one
-// memset that also clears the counts in the fused step); the epoch field
+// The descriptors and the ticket are zeroed before every launch (by the one
+// that also clears the counts in the fused step); the epoch field
 // is a second guard against reading a descriptor left by another launch.
 // Every wait is bounded: after `spin_limit` polls (kSpinLimit in the step)
 // the CTA records FL_DEV_SPIN_TIMEOUT in the device error word and stops
