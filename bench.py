@@ -76,7 +76,11 @@ ALGO_BYTES = {
 # Bytes per point this implementation moves beyond those: the index scatter
 # between the counting atomics and the cell sort (R cell + rank, W index).
 IMPL_BYTES = {"scatter": 12}
-KERNELS_PER_STEP = 8   # insert, scan, scatter, cell sort, crowded-cell sort, gather, density, force+advance
+# clear, insert, scan, scatter, cell sort, crowded-cell sort, gather, density,
+# force + advance, crowded tiles a block each, crowded tiles a warp each (the
+# last from 512 points a multiprocessor)
+KERNELS_PER_STEP = 11
+ALONE_TILES_FROM = 512 * 152
 
 
 def parse():
@@ -910,7 +914,7 @@ def our_arm(args, rank, world, local_rank):
         "adjoint": adjoint,
         "fit": fit,
         "clocks": clocks.summary(t0, t1),
-        "gpu_launches": KERNELS_PER_STEP * args.steps,
+        "gpu_launches": (KERNELS_PER_STEP - (scene.n < ALONE_TILES_FROM)) * args.steps,
         "device_status": status,
         "points_in_range": n_in,
     }
