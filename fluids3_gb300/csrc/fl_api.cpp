@@ -1117,6 +1117,7 @@ static int capture_pair(fl_system *s) {
         return fl_fail(FL_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
     s->graph_steps = 2;
+    s->graph_n = s->n;
     for (int k = 0; k < F_COUNT; k++) s->graph_live[k] = live[k];
     return FL_OK;
 }
@@ -1157,10 +1158,12 @@ static int run_steps_graph(fl_system *s, int nsteps) {
     update_auto(s);
     const int pairs = nsteps / 2;
     if (pairs > 0) {
-        bool match = s->graph_exec != nullptr;
+        // the captured launches hold the live copies and the point count (a
+        // restored checkpoint may have another)
+        bool match = s->graph_exec != nullptr && s->graph_n == s->n;
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
-            for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));
+        for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));
         s->passes_steps[passes_of_step(s, false)] += 2 * (int64_t)pairs;
         s->time_host_valid = 0;   // the device slot now holds the time
         s->have_insert = 0;

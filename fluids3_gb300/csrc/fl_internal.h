@@ -182,7 +182,7 @@ struct fl_system {
 
     // graph replay for fl_run_steps
     cudaGraphExec_t graph_exec;
-    int graph_steps;
+    int graph_steps, graph_n;   // the captured steps, their point count
     int graph_live[F_COUNT];
 
     // checkpoints: per slot, one copy of every field's live buffer + time
