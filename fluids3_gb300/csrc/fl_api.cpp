@@ -896,11 +896,11 @@ static int passes_of_step(const fl_system *s, bool taped) {
 // crowded tiles are found, and shared between warps, in every step.
 constexpr uint32_t kAutoCellsOn = 512, kAutoCellsOff = 384;
 
-static void update_auto(fl_system *s) {
+static void update_auto(fl_system *s, uint32_t at_least = 0) {
     if (s->passes != FL_PASSES_AUTO || !s->crowd_host) return;
     volatile const uint32_t *h = s->crowd_host;
     if (h[1] != s->auto_epoch) return;   // no count of the current state has arrived yet
-    const uint32_t big = h[0];
+    const uint32_t now = h[0], big = now > at_least ? now : at_least;
     if (!s->auto_cells && big >= kAutoCellsOn) s->auto_cells = 1;
     else if (s->auto_cells && big < kAutoCellsOff) s->auto_cells = 0;
 }
@@ -1124,10 +1124,13 @@ static int capture_pair(fl_system *s) {
 
 static int run_steps_graph(fl_system *s, int nsteps);
 
-// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps. What a
-// chunk's steps count as comes from the counts of the chunk two before it, the
-// second chunk's from the first two steps (waited for, while the steps queued
-// after them keep the GPU busy).
+// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps. What the
+// first two chunks count as comes from whatever has reached the host by then,
+// a later one's from the chunk two before it, which the host waits for (one
+// chunk stays queued): the larger of its second step's largest cell, copied
+// aside for this, and of the last that was reported, so that a crowd which
+// formed and dispersed within a chunk is seen. Calls of up to two chunks wait
+// for nothing.
 constexpr int kAutoChunk = 32;
 
 extern "C" int fl_run_steps(fl_system *s, int nsteps) {
@@ -1137,17 +1140,24 @@ extern "C" int fl_run_steps(fl_system *s, int nsteps) {
         for (int k = 0; k < nsteps; k++) FL_TRY(fl_run(s));
         return FL_OK;
     }
+    update_auto(s);
     if (s->passes != FL_PASSES_AUTO || nsteps <= kAutoChunk) return run_steps_graph(s, nsteps);
     int left = nsteps;
     for (int k = 0; left > 0; k++) {
         const int c = left < kAutoChunk ? left : kAutoChunk;
-        if (k == 0) {
-            FL_TRY(run_steps_graph(s, 2));
-            FL_CUDA_TRY(cudaEventRecord(s->ev_auto[1], s->stream));
-        } else {
+        uint32_t *early = s->crowd_host + 2 + (k & 1);
+        if (k == 1) update_auto(s);
+        if (k >= 2) {
             FL_CUDA_TRY(cudaEventSynchronize(s->ev_auto[k & 1]));
+            update_auto(s, *(volatile uint32_t *)early);
         }
-        FL_TRY(run_steps_graph(s, k == 0 ? c - 2 : c));
+        if (left > 2 * kAutoChunk) {   // a chunk two on will look at this one
+            FL_TRY(run_steps_graph(s, 2));
+            FL_CUDA_TRY(cudaMemcpyAsync(early, s->crowd_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
+            FL_TRY(run_steps_graph(s, c - 2));
+        } else {
+            FL_TRY(run_steps_graph(s, c));
+        }
         FL_CUDA_TRY(cudaEventRecord(s->ev_auto[k & 1], s->stream));
         left -= c;
     }
@@ -1155,7 +1165,6 @@ extern "C" int fl_run_steps(fl_system *s, int nsteps) {
 }
 
 static int run_steps_graph(fl_system *s, int nsteps) {
-    update_auto(s);
     const int pairs = nsteps / 2;
     if (pairs > 0) {
         // the captured launches hold the live copies and the point count (a

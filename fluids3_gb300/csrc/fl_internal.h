@@ -148,7 +148,7 @@ struct fl_system {
     int64_t passes_steps[2]; // fused steps issued with the per-point passes / the cell tasks
     uint32_t *crowd_dev;   // largest in-range cell above 128 points, this step (0: none)
     uint32_t *crowd_epoch; // device: the state's epoch (bumped when the state is replaced)
-    uint32_t *crowd_host;  // page-locked [count, epoch], written by each step's sort
+    uint32_t *crowd_host;  // page-locked [count, epoch], written by each step's sort; [2], [3]: fl_run_steps
     void *crowd_report;    // its device-side address
     uint32_t auto_epoch;   // host: the current state's epoch
     int adj_revmode;       // FL_REVERSE_*: how the adjoint finds its reverse pair lists

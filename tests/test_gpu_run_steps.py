@@ -4,6 +4,8 @@ needs no tolerance.
 """
 from __future__ import annotations
 
+import time
+
 import pytest
 
 import fluids3_gb300 as F
@@ -43,3 +45,31 @@ def test_restoring_a_checkpoint_of_fewer_points_steps_those_points(first, more):
             got = s.state()
             for k in FIELDS + ("gridcnt", "gridoff"):
                 assert_bit_equal(got[k], want[n][k], f"{n} points restored: {k}")
+
+
+@pytest.mark.parametrize("steps", [33, 50, 64])
+def test_calls_of_up_to_64_steps_return_before_the_queued_work_is_done(steps):
+    """RunSteps queues its steps and returns: behind 64 queued steps, a call
+    of 33 to 64 leaves most of that work unfinished when it returns, in the
+    default mode as with the per-point passes. (Were it to wait for its first
+    steps, the queued ones would be done by then.) The states are equal."""
+    sc = scenes.wave_tank(n=1_000_000)
+    out = {}
+    for mode in ("auto", "points"):
+        with F.FluidSystem(sc.params, sc.n) as s:
+            s.SetNeighbourPasses(mode)
+            s.SetParticles(sc.pos, sc.vel, sc.veval, clr=sc.clr)
+            s.RunSteps(2)   # captures the pair
+            s.Sync()
+            t0 = time.perf_counter()
+            s.RunSteps(64)
+            s.RunSteps(steps)
+            t1 = time.perf_counter()
+            s.Sync()
+            t2 = time.perf_counter()
+            # (waiting for the queued 64 takes a third or more of the time)
+            assert t1 - t0 < 0.2 * (t2 - t0), (mode, t1 - t0, t2 - t0)
+            assert sum(s.PassesSteps()) == 2 + 64 + steps
+            out[mode] = s.state()
+    for k in FIELDS + ("gridcnt", "gridoff"):
+        assert_bit_equal(out["auto"][k], out["points"][k], f"{steps} steps: {k}")
