@@ -352,13 +352,16 @@ static int run_reverse(fl_system *s, fl_tape *t) {
         for (int k = t0; k < t1; k++) {
             FL_TRY(save_replayed(s, t, t->seg + (size_t)(k - t0) * blk, k));
             uint32_t *own_list = s->hitlist, *own_cnt = s->hitcnt;
-            if (t->keep_lists) {   // the step's density pass (one that writes pair lists) fills the slot
+            const int own_passes = s->passes;
+            if (t->keep_lists) {   // the step's density pass fills the slot; like a taped step's, it counts as per-point
                 s->hitlist = t->seg_list + (size_t)(k - t0) * t->list_words;
                 s->hitcnt = t->seg_cnt + (size_t)(k - t0) * t->cap;
+                if (s->passes == FL_PASSES_CELL_TASKS || s->passes == FL_PASSES_AUTO) s->passes = FL_PASSES_PER_POINT;
             }
             const int r = fl_step_fused(s);
             s->hitlist = own_list;
             s->hitcnt = own_cnt;
+            s->passes = own_passes;
             FL_TRY(r);
             FL_TRY(save_step(s, t->force + (size_t)(k - t0) * t->cap,
                              t->keep_lists ? t->seg_rho + (size_t)(k - t0) * t->cap : nullptr));

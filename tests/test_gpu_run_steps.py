@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import time
 
+import numpy as np
 import pytest
 
 import fluids3_gb300 as F
@@ -73,3 +74,22 @@ def test_calls_of_up_to_64_steps_return_before_the_queued_work_is_done(steps):
             out[mode] = s.state()
     for k in FIELDS + ("gridcnt", "gridoff"):
         assert_bit_equal(out["auto"][k], out["points"][k], f"{steps} steps: {k}")
+
+
+@pytest.mark.parametrize("keep,want", [(True, (4, 0)), (False, (0, 4))])
+def test_what_replayed_steps_of_a_tape_count_as(keep, want):
+    """Backward replays the steps of each segment: with kept pair lists they
+    count as per-point steps, else by the mode set. (Taped steps count as
+    per-point steps in every mode.)"""
+    sc = scenes.dam_break(n=3000, seed=5)
+    w = np.ones((3, sc.n, 3), np.float32)
+    with F.FluidSystem(sc.params, sc.n) as s:
+        s.SetParticles(sc.pos, sc.vel, sc.veval, clr=sc.clr)
+        s.SetNeighbourPasses("cells")
+        s.TapeBegin(4, 2, keep_lists=keep)
+        for _ in range(4):
+            s.Run()
+        assert s.PassesSteps() == (4, 0)
+        s.Backward(*w)
+        assert tuple(a - b for a, b in zip(s.PassesSteps(), (4, 0))) == want
+        assert s.NeighbourPasses() == "cells"
