@@ -62,6 +62,7 @@ SIGNATURES = [
     ("fl_get_phase_times", C.c_int, [vp, C.POINTER(C.c_double), C.POINTER(C.c_int)]),
     ("fl_prefix_sum_noalloc", C.c_int, [vp, vp, C.c_int, C.c_int, vp, vp]),
     ("fl_test_scan_timeout", C.c_int, [vp, C.c_int]),
+    ("fl_test_density_block", C.c_int, [vp]),
     ("fl_test_scan_noalloc_timeout", C.c_int, [vp, vp, C.c_int, vp, C.c_int, vp]),
     ("fl_set_reverse_lists", C.c_int, [vp, C.c_int]),
     ("fl_neighbour_passes_in_use", C.c_int, [vp]),

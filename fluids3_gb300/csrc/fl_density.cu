@@ -63,7 +63,7 @@ constexpr float kUnits = 1000.0f;               // half the widest side of the b
 constexpr float kBase = 2048.0f;                // squares are split into kBase * high + low, both exact in half
 constexpr float kFar = 6.0e4f;                  // times kBase: beyond any square
 constexpr int kDensityThreads = 128;
-constexpr int kRowsMaxThreads = 256;
+constexpr int kRowsThreads = 256, kMaxThreads = 1024;   // k_density_rows: up to the first, and beyond
 
 __device__ __forceinline__ uint32_t half2_bits(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
@@ -438,8 +438,12 @@ __device__ __forceinline__ void finish(const DevParams &P, const Sum &s, int i, 
     pairdata[2 * (size_t)i + 1] = make_float4(e.x, e.y, e.z, 0.0f);
 }
 
-template <bool BATCH>
-__global__ void __launch_bounds__(kRowsMaxThreads, 1280 / kRowsMaxThreads)
+// Blocks of up to 256 threads are compiled for 40 resident warps (above); the
+// larger ones a caller may pin or the tuner times (fl_set_launch_shapes) have
+// an instantiation of their own: one block of 1,024 threads and its rings,
+// 128 KB, fit a multiprocessor, two do not.
+template <bool BATCH, int MOST>
+__global__ void __launch_bounds__(MOST, MOST == kRowsThreads ? 1280 / kRowsThreads : 1)
 k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
                const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
                float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
@@ -552,7 +556,7 @@ __device__ __forceinline__ bool shared_tiles(uint32_t count, int workers) { retu
 // The first `workers` blocks take the tiles that the sort's gather listed and
 // that are set apart (workers 0: none are), the others 32 slots a warp.
 template <bool BATCH>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(kMaxThreads)
 k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
           const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
           float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
@@ -605,12 +609,17 @@ k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const f
     if (i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
 }
 
+size_t rows_smem(int threads) { return (size_t)(threads / 32) * 32 * kRing * sizeof(uint32_t); }
+
 }  // namespace
 
 int fl_density_init() {
     const int most = 32 * kWarpWords * (int)sizeof(uint32_t);
     FL_CUDA_TRY(cudaFuncSetAttribute(k_density<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     FL_CUDA_TRY(cudaFuncSetAttribute(k_density<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    const int rows = (int)rows_smem(kMaxThreads);
+    FL_CUDA_TRY(cudaFuncSetAttribute(k_density_rows<false, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows));
+    FL_CUDA_TRY(cudaFuncSetAttribute(k_density_rows<true, kMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows));
     return FL_OK;
 }
 
@@ -623,15 +632,16 @@ int fl_launch_density(fl_system *s) {
     // without a new one read them through the old grid) may be anywhere, or
     // NaN: each point walks alone, as with gridSrch > 2 (in any scene).
     const bool rows = !s->D.prune || !s->codes_valid;
-    const int bs = rows ? std::min(fl_density_block(s), kRowsMaxThreads) : fl_density_block(s);
-    const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
+    const int bs = fl_density_block(s);
     if (rows) {
-        auto kern = s->batched ? k_density_rows<true> : k_density_rows<false>;
-        launch(kern, blocks_for(s->n, bs), bs, (size_t)(bs / 32) * 32 * kRing * sizeof(uint32_t), s->stream, s->D,
-               fl_scene_tab(s), s->n, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off,
-               s->f[F_VEVAL].cur<float4>(), s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
+        auto kern = bs <= kRowsThreads ? (s->batched ? k_density_rows<true, kRowsThreads> : k_density_rows<false, kRowsThreads>)
+                                       : (s->batched ? k_density_rows<true, kMaxThreads> : k_density_rows<false, kMaxThreads>);
+        launch(kern, blocks_for(s->n, bs), bs, rows_smem(bs), s->stream, s->D, fl_scene_tab(s), s->n,
+               s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),
+               s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
     } else {
         const int workers = s->tiles_listed ? std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32) : 0;
+        const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
         auto kern = s->batched ? k_density<true> : k_density<false>;
         launch(kern, workers + blocks_for(s->n, bs), bs, smem, s->stream, s->D, fl_scene_tab(s), s->n,
                s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),
@@ -639,6 +649,12 @@ int fl_launch_density(fl_system *s) {
         s->tiles_listed = 0;   // the list is used up
     }
     FL_LAUNCH_CHECK("density");
+    s->ran_density_block = bs;
     s->lists_valid = 1;
     return FL_OK;
+}
+
+extern "C" int fl_test_density_block(const fl_system *s) {
+    if (!s) return fl_fail(FL_ERR_ARG, "fl_test_density_block: null system");
+    return s->ran_density_block;
 }

@@ -487,6 +487,10 @@ int fl_test_scan_timeout(fl_system *s, int spin_limit);
 int fl_test_scan_noalloc_timeout(const uint32_t *d_counts, uint32_t *d_offsets, int n, uint32_t *d_status,
                                  int spin_limit, void *stream);
 
+/* Test hook: threads per block of the last density pass that was launched (0:
+ * none yet; FL_PASSES_POINT_PAIRS's walk has a fixed block and leaves it). */
+int fl_test_density_block(const fl_system *s);
+
 /* How fl_backward finds each point's reverse pairs (no counterpart in the
  * reference): FL_REVERSE_WALK walks the point's reverse block (one launch);
  * FL_REVERSE_TRANSPOSE transposes the density pass's pair lists (atomics,
