@@ -171,13 +171,13 @@ __device__ __forceinline__ float3 clamp_adjoint(float3 u, float L, float3 ub) {
 // to pre-sort index src[s].
 __global__ void __launch_bounds__(kAdjThreads)
 k_adj_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float *time_ptr, float dt,
-              const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ src,
-              const float4 *__restrict__ X, const float4 *__restrict__ V, const float4 *__restrict__ E,
-              const float4 *__restrict__ F, const float *__restrict__ rho,
-              const float4 *__restrict__ xo_b, const float4 *__restrict__ vo_b, const float4 *__restrict__ eo_b,
-              float4 *__restrict__ xa, float4 *__restrict__ ea, float4 *__restrict__ fb,
-              float4 *__restrict__ v_out, float2 *__restrict__ rr, uint32_t *__restrict__ counts,
-              uint32_t *__restrict__ revcnt) {
+              const uint32_t *gcell, const uint32_t *src,
+              const float4 *X, const float4 *V, const float4 *E,
+              const float4 *F, const float *rho,
+              const float4 *xo_b, const float4 *vo_b, const float4 *eo_b,
+              float4 *xa, float4 *ea, float4 *fb,
+              float4 *v_out, float2 *rr, uint32_t *counts,
+              uint32_t *revcnt) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < 2) counts[s] = 0;
@@ -506,10 +506,10 @@ __device__ __forceinline__ void rev_walk_point(const DevParams &P, int s, const 
 
 template <bool PRUNE>
 __global__ void __launch_bounds__(kThreads)
-k_adj_revwalk(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-              const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-              const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-              uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+k_adj_revwalk(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+              const uint32_t *gcell, const uint32_t *off,
+              const uint32_t *cnt, const uint32_t *upbits,
+              uint32_t *revlist, uint32_t *revcnt) {
     follow_previous();
     extern __shared__ uint32_t s_dyn[];
     const int s = PRUNE ? band_grouped_slot(n, pos, gcell, 0, s_dyn) : (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -521,11 +521,11 @@ k_adj_revwalk(const __grid_constant__ DevParams P0, const SceneTab T, int n, con
 // sort in registers), a grid-stride loop over the listed count.
 template <bool PRUNE>
 __global__ void __launch_bounds__(kThreads)
-k_adj_revwalk_listed(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *__restrict__ pos,
-                     const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-                     const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-                     const uint32_t *__restrict__ listed, const uint32_t *__restrict__ listed_count,
-                     uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+k_adj_revwalk_listed(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *pos,
+                     const uint32_t *gcell, const uint32_t *off,
+                     const uint32_t *cnt, const uint32_t *upbits,
+                     const uint32_t *listed, const uint32_t *listed_count,
+                     uint32_t *revlist, uint32_t *revcnt) {
     follow_previous();
     const uint32_t m = *listed_count;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
@@ -548,11 +548,11 @@ constexpr uint32_t kScatterBatch = 4;
 
 template <bool PRUNE>
 __global__ void __launch_bounds__(kThreads)
-k_adj_revscatter(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-                 const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-                 const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-                 const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
-                 uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt) {
+k_adj_revscatter(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+                 const uint32_t *gcell, const uint32_t *off,
+                 const uint32_t *cnt, const uint32_t *upbits,
+                 const uint32_t *hitlist, const uint32_t *hitcnt,
+                 uint32_t *revlist, uint32_t *revcnt) {
     follow_previous();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
@@ -630,8 +630,8 @@ __device__ __forceinline__ void sort_row(uint32_t *row, uint32_t c) {   // entry
 }
 
 __global__ void __launch_bounds__(kThreads)
-k_adj_revsort(int n, int hcap_in, uint32_t *__restrict__ revlist, uint32_t *__restrict__ revcnt,
-              uint32_t *__restrict__ listed, uint32_t *__restrict__ listed_count) {
+k_adj_revsort(int n, int hcap_in, uint32_t *revlist, uint32_t *revcnt,
+              uint32_t *listed, uint32_t *listed_count) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= (unsigned)n) return;   // whole warp past n
@@ -672,13 +672,13 @@ k_adj_revsort(int n, int hcap_in, uint32_t *__restrict__ revlist, uint32_t *__re
 template <bool PRUNE>
 __global__ void __launch_bounds__(kAdjThreads, 8)
 k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
-            const float4 *__restrict__ pos, const float4 *__restrict__ veval, const float2 *__restrict__ rr,
-            const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
-            const uint32_t *__restrict__ upbits, const uint32_t *__restrict__ hitlist,
-            const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ src,
-            const float4 *__restrict__ fb, float4 *__restrict__ xa, float4 *ea, float4 *__restrict__ pc,
-            float4 *__restrict__ e_out,
-            const uint32_t *__restrict__ revlist, const uint32_t *__restrict__ revcnt, const CrowdList crowd) {
+            const float4 *pos, const float4 *veval, const float2 *rr,
+            const uint32_t *gcell, const uint32_t *off, const uint32_t *cnt,
+            const uint32_t *upbits, const uint32_t *hitlist,
+            const uint32_t *hitcnt, const uint32_t *src,
+            const float4 *fb, float4 *xa, float4 *ea, float4 *pc,
+            float4 *e_out,
+            const uint32_t *revlist, const uint32_t *revcnt, const CrowdList crowd) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = scene_params(P0, T, s < n ? s : 0);
@@ -757,12 +757,12 @@ k_adj_force(const __grid_constant__ DevParams P0, const SceneTab T, int n,
 template <bool PRUNE>
 __global__ void __launch_bounds__(kAdjThreads)
 k_adj_density(const __grid_constant__ DevParams P0, const SceneTab T, int n,
-              const float4 *__restrict__ pos, const float4 *__restrict__ xr, const uint32_t *__restrict__ gcell,
-              const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
-              const uint32_t *__restrict__ upbits, const uint32_t *__restrict__ hitlist,
-              const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revlist,
-              const uint32_t *__restrict__ revcnt, const uint32_t *__restrict__ src,
-              const float4 *__restrict__ xa, float4 *__restrict__ x_out, bool walk_overflow) {
+              const float4 *pos, const float4 *xr, const uint32_t *gcell,
+              const uint32_t *off, const uint32_t *cnt,
+              const uint32_t *upbits, const uint32_t *hitlist,
+              const uint32_t *hitcnt, const uint32_t *revlist,
+              const uint32_t *revcnt, const uint32_t *src,
+              const float4 *xa, float4 *x_out, bool walk_overflow) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
@@ -934,13 +934,13 @@ __device__ __forceinline__ void block_sum(float (&v)[K], float (*s_red)[K]) {
 // the parameter partials).
 template <bool PRUNE>
 __global__ void __launch_bounds__(kCrowdThreads)
-k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *__restrict__ pos,
-                  const float4 *__restrict__ veval, const float2 *__restrict__ rr,
-                  const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-                  const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-                  const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
-                  const uint32_t *__restrict__ src, const float4 *__restrict__ fb, float4 *__restrict__ xa,
-                  float4 *__restrict__ e_out, float4 *__restrict__ xr, float4 *__restrict__ pc, const CrowdList L) {
+k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *pos,
+                  const float4 *veval, const float2 *rr,
+                  const uint32_t *gcell, const uint32_t *off,
+                  const uint32_t *cnt, const uint32_t *upbits,
+                  const uint32_t *hitcnt, const uint32_t *revcnt,
+                  const uint32_t *src, const float4 *fb, float4 *xa,
+                  float4 *e_out, float4 *xr, float4 *pc, const CrowdList L) {
     follow_previous();
     __shared__ float s_red[kCrowdThreads / 32][10];
     __shared__ uint32_t s_nlist;
@@ -990,11 +990,11 @@ k_adj_crowd_force(const __grid_constant__ DevParams P0, const SceneTab T, const 
 // k_adj_density wrote for it.
 template <bool PRUNE>
 __global__ void __launch_bounds__(kCrowdThreads)
-k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *__restrict__ pos,
-                    const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-                    const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-                    const uint32_t *__restrict__ hitcnt, const uint32_t *__restrict__ revcnt,
-                    const uint32_t *__restrict__ src, const float4 *__restrict__ xr, float4 *__restrict__ x_out,
+k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, const float4 *pos,
+                    const uint32_t *gcell, const uint32_t *off,
+                    const uint32_t *cnt, const uint32_t *upbits,
+                    const uint32_t *hitcnt, const uint32_t *revcnt,
+                    const uint32_t *src, const float4 *xr, float4 *x_out,
                     const CrowdList L) {
     follow_previous();
     __shared__ float s_red[kCrowdThreads / 32][3];
@@ -1055,8 +1055,8 @@ k_adj_crowd_density(const __grid_constant__ DevParams P0, const SceneTab T, cons
 // (65,536 points: 13 us, and 6 for the totals by one warp; gradients of 10
 // steps 3,077 us so, 2,996 with chunks of 1,024 and four warps a total).
 __global__ void __launch_bounds__(kReduceThreads)
-k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, const int *__restrict__ sn,
-                int nchunks, double *__restrict__ partial) {
+k_param_partial(const float4 *pc, const int *sbase, const int *sn,
+                int nchunks, double *partial) {
     follow_previous();
     const int chunk = blockIdx.x, scene = blockIdx.y;
     const int b = sbase[scene], m = sn[scene];
@@ -1090,8 +1090,8 @@ k_param_partial(const float4 *__restrict__ pc, const int *__restrict__ sbase, co
 
 // Warp w adds parameter w % 3 over the chunks w / 3 (mod 4), lane by lane.
 __global__ void __launch_bounds__(kFinalThreads)
-k_param_final(int nchunks, const double *__restrict__ partial, const int *__restrict__ gexp,
-              double *__restrict__ acc) {
+k_param_final(int nchunks, const double *partial, const int *gexp,
+              double *acc) {
     follow_previous();
     const int scene = blockIdx.x, w = (int)(threadIdx.x >> 5), j = w % 3;
     constexpr int kParts = kFinalThreads / 96;
@@ -1143,8 +1143,8 @@ __device__ __forceinline__ uint32_t gmax_bits(const float4 a, const float4 b, co
 }
 
 __global__ void __launch_bounds__(kGmaxThreads)
-k_adj_gmax(int n, const uint16_t *__restrict__ point_scene, const float4 *__restrict__ gx,
-           const float4 *__restrict__ gv, const float4 *__restrict__ ge, uint32_t *__restrict__ gmax) {
+k_adj_gmax(int n, const uint16_t *point_scene, const float4 *gx,
+           const float4 *gv, const float4 *ge, uint32_t *gmax) {
     follow_previous();
     __shared__ uint32_t s_max[kGmaxThreads / 32];
     const int b0 = blockIdx.x * kGmaxPoints;
@@ -1194,8 +1194,8 @@ __device__ __forceinline__ int rescale_exponent(uint32_t bits) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-k_adj_rescale(int n, const uint16_t *__restrict__ point_scene, float4 *__restrict__ gx, float4 *__restrict__ gv,
-              float4 *__restrict__ ge, const uint32_t *__restrict__ gmax) {
+k_adj_rescale(int n, const uint16_t *point_scene, float4 *gx, float4 *gv,
+              float4 *ge, const uint32_t *gmax) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1212,8 +1212,8 @@ k_adj_rescale(int n, const uint16_t *__restrict__ point_scene, float4 *__restric
 // The gradient itself from its mantissa: times 2^gexp (float; infinite
 // where it overflows).
 __global__ void __launch_bounds__(kThreads)
-k_adj_apply_exponent(int n, const uint16_t *__restrict__ point_scene, float4 *__restrict__ gx,
-                     float4 *__restrict__ gv, float4 *__restrict__ ge, const int *__restrict__ gexp) {
+k_adj_apply_exponent(int n, const uint16_t *point_scene, float4 *gx,
+                     float4 *gv, float4 *ge, const int *gexp) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1226,7 +1226,7 @@ k_adj_apply_exponent(int n, const uint16_t *__restrict__ point_scene, float4 *__
     gx[i] = a; gv[i] = b; ge[i] = c;
 }
 
-__global__ void k_adj_bump(int nscenes, uint32_t *__restrict__ gmax, int *__restrict__ gexp) {
+__global__ void k_adj_bump(int nscenes, uint32_t *gmax, int *gexp) {
     follow_previous();
     const int sc = blockIdx.x * blockDim.x + threadIdx.x;
     if (sc >= nscenes) return;
@@ -1236,8 +1236,8 @@ __global__ void k_adj_bump(int nscenes, uint32_t *__restrict__ gmax, int *__rest
 
 // Identity tracking across recorded steps: out[s] = in[src[s]] (in null:
 // out = src; src null: the identity).
-__global__ void k_compose(int n, const uint32_t *__restrict__ src, const uint32_t *__restrict__ in,
-                          uint32_t *__restrict__ out) {
+__global__ void k_compose(int n, const uint32_t *src, const uint32_t *in,
+                          uint32_t *out) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;

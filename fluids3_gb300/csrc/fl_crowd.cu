@@ -90,6 +90,7 @@ __device__ __forceinline__ void crowded_tile(const DevParams &P0, const SceneTab
     const bool active = gc != kUndef;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
     ForcePoint fp = crowd_point(P, i, active, a);
+    const float4 *const records = after_wait(a.pairdata);
     struct Record {
         float4 q, v;
     };
@@ -104,7 +105,7 @@ __device__ __forceinline__ void crowded_tile(const DevParams &P0, const SceneTab
             PS, seg, gc, a.off,
             [&](bool ok, uint32_t j) {
                 Record d = {make_float4(0.f, 0.f, 0.f, 1.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-                if (ok) load_record(a.pairdata, j, d.q, d.v);
+                if (ok) load_record(records, j, d.q, d.v);
                 return d;
             },
             [&](const Record &d) {

@@ -444,10 +444,10 @@ __device__ __forceinline__ void finish(const DevParams &P, const Sum &s, int i, 
 // 128 KB, fit a multiprocessor, two do not.
 template <bool BATCH, int MOST>
 __global__ void __launch_bounds__(MOST, MOST == kRowsThreads ? 1280 / kRowsThreads : 1)
-k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-               const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
-               float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
-               float4 *__restrict__ pairdata) {
+k_density_rows(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+               const uint32_t *gcell, const uint32_t *off, const float4 *veval,
+               float *press, uint32_t *hitlist, uint32_t *hitcnt,
+               float4 *pairdata) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
@@ -557,10 +557,10 @@ __device__ __forceinline__ bool shared_tiles(uint32_t count, int workers) { retu
 // that are set apart (workers 0: none are), the others 32 slots a warp.
 template <bool BATCH>
 __global__ void __launch_bounds__(kMaxThreads)
-k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-          const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
-          float *__restrict__ press, uint32_t *__restrict__ hitlist, uint32_t *__restrict__ hitcnt,
-          float4 *__restrict__ pairdata, const CrowdTiles tiles, int workers) {
+k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+          const uint32_t *gcell, const uint32_t *off, const float4 *veval,
+          float *press, uint32_t *hitlist, uint32_t *hitcnt,
+          float4 *pairdata, const CrowdTiles tiles, int workers) {
     follow_previous();
     extern __shared__ __align__(16) uint32_t s_dyn[];
     if ((int)blockIdx.x < workers) {

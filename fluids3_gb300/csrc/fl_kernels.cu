@@ -33,9 +33,9 @@ namespace {
 // last) and one scan over all of them yields each scene's segments.
 template <bool BATCH>
 __global__ void __launch_bounds__(kThreads)
-k_insert(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-         uint32_t *__restrict__ cell_out, uint32_t *__restrict__ rank_out,
-         uint32_t *__restrict__ gcell_out, uint32_t *__restrict__ cnt) {
+k_insert(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+         uint32_t *cell_out, uint32_t *rank_out,
+         uint32_t *gcell_out, uint32_t *cnt) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
@@ -68,8 +68,8 @@ k_insert(const __grid_constant__ DevParams P0, const SceneTab T, int n, const fl
 
 // Place each point's index at its arrival slot inside its cell's segment.
 __global__ void __launch_bounds__(kThreads)
-k_scatter_index(int n, const uint32_t *__restrict__ cell_pre, const uint32_t *__restrict__ rank,
-                const uint32_t *__restrict__ off, uint32_t *__restrict__ src) {
+k_scatter_index(int n, const uint32_t *cell_pre, const uint32_t *rank,
+                const uint32_t *off, uint32_t *src) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -394,14 +394,14 @@ __device__ __forceinline__ void publish_tile(const DevParams &P0, const SceneTab
 }
 
 template <bool BATCH, int ROWS, bool LATE = false>
-__global__ void __launch_bounds__(kThreads)
-k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *__restrict__ src,
-                const uint32_t *__restrict__ cell_pre, const uint32_t *__restrict__ off,
-                const float4 *__restrict__ pos_in, const float4 *__restrict__ vel_in,
-                const float4 *__restrict__ veval_in, const uint32_t *__restrict__ clr_in,
-                float4 *__restrict__ pos_out, float4 *__restrict__ vel_out, float4 *__restrict__ veval_out,
-                uint32_t *__restrict__ clr_out, uint32_t *__restrict__ gcell_out,
-                uint32_t *__restrict__ gndx_out, uint32_t *__restrict__ upbits, const CrowdTiles tiles) {
+__global__ void __launch_bounds__(kThreads, 8)
+k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *src,
+                const uint32_t *cell_pre, const uint32_t *off,
+                const float4 *pos_in, const float4 *vel_in,
+                const float4 *veval_in, const uint32_t *clr_in,
+                float4 *pos_out, float4 *vel_out, float4 *veval_out,
+                uint32_t *clr_out, uint32_t *gcell_out,
+                uint32_t *gndx_out, uint32_t *upbits, const CrowdTiles tiles) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= (unsigned)n) return;   // whole warp past n
@@ -412,19 +412,26 @@ k_gather_sorted(const __grid_constant__ DevParams P0, const SceneTab T, int n, c
         const uint32_t c = cell_pre[i];
         const DevParams &P = BATCH ? T.params[T.cell_scene[c]] : P0;
         const int local = (int)c - P.cell_base;
-        float4 p = pos_in[i];
+        float4 p = pos_in[i], v, e;   // (every load before the first store: they may alias, to the compiler)
+        uint32_t k = 0;
+        if (!LATE) {   // LATE: velocities, evaluated velocities, colours come from k_gather_late
+            v = vel_in[i];
+            e = veval_in[i];
+            k = clr_in[i];
+        }
+        const uint32_t first = off[c];
+        upwords = (uint32_t)P.upwords;
         if (ROWS >= 1) code = band_code(P, local, p);
         p.w = __uint_as_float(code);
-        pos_out[s] = p;
-        if (!LATE) {   // LATE: velocities, evaluated velocities, colours come from k_gather_late
-            vel_out[s] = vel_in[i];
-            veval_out[s] = veval_in[i];
-            clr_out[s] = clr_in[i];
-        }
         cell = (local == P.ncells) ? kUndef : c;
+        pos_out[s] = p;
+        if (!LATE) {
+            vel_out[s] = v;
+            veval_out[s] = e;
+            clr_out[s] = k;
+        }
         gcell_out[s] = cell;
-        gndx_out[s] = (uint32_t)s - off[c];
-        upwords = (uint32_t)P.upwords;
+        gndx_out[s] = (uint32_t)s - first;
     }
     if constexpr (ROWS >= 1)   // (lane 0 holds a point: s0 < n)
         publish_tile<BATCH, ROWS>(P0, T, (size_t)(s >> 5), code, cell, off, upbits,
@@ -443,18 +450,19 @@ __device__ __forceinline__ float4 load3_or_zero(const float *__restrict__ a, uin
 }
 
 __global__ void __launch_bounds__(kThreads)
-k_gather_late(int n, const uint32_t *__restrict__ src, const float *__restrict__ vel3,
-              const float *__restrict__ veval3, const uint32_t *__restrict__ clr, float4 *__restrict__ vel_out,
-              float4 *__restrict__ veval_out, uint32_t *__restrict__ clr_out, float4 *__restrict__ pairdata) {
+k_gather_late(int n, const uint32_t *src, const float *vel3,
+              const float *veval3, const uint32_t *clr, float4 *vel_out,
+              float4 *veval_out, uint32_t *clr_out, float4 *pairdata) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = src[s];
-    vel_out[s] = load3_or_zero(vel3, i);
-    const float4 e = load3_or_zero(veval3, i);
+    const float4 v = load3_or_zero(vel3, i), e = load3_or_zero(veval3, i);
+    const uint32_t k = clr ? clr[i] : 0u;
+    vel_out[s] = v;
     veval_out[s] = e;
     pairdata[2 * (size_t)s + 1] = e;
-    clr_out[s] = clr ? clr[i] : 0u;
+    clr_out[s] = k;
 }
 
 // Phase-API counting sort (countingSortFull, fluids4.0/fluid_kernels.cu:56-87)
@@ -463,15 +471,15 @@ k_gather_late(int n, const uint32_t *__restrict__ src, const float *__restrict__
 // step's gather does.
 template <bool BATCH, bool PRUNE>
 __global__ void __launch_bounds__(kThreads)
-k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *__restrict__ src,
-             const uint32_t *__restrict__ off, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
-             const float4 *__restrict__ veval, const float4 *__restrict__ force,
-             const float *__restrict__ press, const uint32_t *__restrict__ clr,
-             const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ gndx,
-             float4 *__restrict__ pos_o, float4 *__restrict__ vel_o,
-             float4 *__restrict__ veval_o, float4 *__restrict__ force_o,
-             float *__restrict__ press_o, uint32_t *__restrict__ clr_o,
-             uint32_t *__restrict__ gcell_o, uint32_t *__restrict__ gndx_o, uint32_t *__restrict__ upbits,
+k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, const uint32_t *src,
+             const uint32_t *off, const float4 *pos, const float4 *vel,
+             const float4 *veval, const float4 *force,
+             const float *press, const uint32_t *clr,
+             const uint32_t *gcell, const uint32_t *gndx,
+             float4 *pos_o, float4 *vel_o,
+             float4 *veval_o, float4 *force_o,
+             float *press_o, uint32_t *clr_o,
+             uint32_t *gcell_o, uint32_t *gndx_o, uint32_t *upbits,
              const CrowdTiles tiles) {
     follow_previous();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -481,6 +489,9 @@ k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, cons
         const uint32_t i = src[s];
         cell = gcell[i];
         float4 p = pos[i];
+        const float4 v = vel[i], e = veval[i], f = force[i];   // (every load before the first store)
+        const float d = press[i];
+        const uint32_t k = clr[i], r = gndx[i];
         if (PRUNE) {
             if (cell != kUndef) {
                 const DevParams &P = BATCH ? T.params[T.cell_scene[cell]] : P0;
@@ -489,13 +500,13 @@ k_gather_all(const __grid_constant__ DevParams P0, const SceneTab T, int n, cons
             p.w = __uint_as_float(code);
         }
         pos_o[s] = p;
-        vel_o[s] = vel[i];
-        veval_o[s] = veval[i];
-        force_o[s] = force[i];
-        press_o[s] = press[i];
-        clr_o[s] = clr[i];
+        vel_o[s] = v;
+        veval_o[s] = e;
+        force_o[s] = f;
+        press_o[s] = d;
+        clr_o[s] = k;
         gcell_o[s] = cell;
-        gndx_o[s] = gndx[i];
+        gndx_o[s] = r;
     }
     if constexpr (PRUNE)
         publish_tile<BATCH, 1>(P0, T, (size_t)(s >> 5), code, cell, off, upbits, (uint32_t)P0.upwords, tiles);
@@ -631,12 +642,12 @@ __device__ __forceinline__ ForcePoint force_point(const DevParams &P, int i, boo
 
 template <bool PRUNE, bool LIST, bool BATCH>
 __global__ void __launch_bounds__(kForceThreads)
-k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *__restrict__ pos,
-        const float4 *__restrict__ veval, const float *__restrict__ press,
-        const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
-        const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ upbits,
-        const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
-        const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ force) {
+k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+        const float4 *veval, const float *press,
+        const uint32_t *gcell, const uint32_t *off,
+        const uint32_t *cnt, const uint32_t *upbits,
+        const uint32_t *hitlist, const uint32_t *hitcnt,
+        const float4 *pairdata, const CrowdTiles over, float4 *force) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
@@ -644,7 +655,7 @@ k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const flo
     const bool active = gc != kUndef;
     ForcePoint fp = force_point(P, i, active, pos, veval, press);
     if constexpr (LIST) {
-        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, after_wait(pairdata), over)) return;
     } else {
         force_by_walk<PRUNE>(P, active, gc, fp, pos, veval, press, off, cnt, upbits);
     }
@@ -655,8 +666,8 @@ k_force(const __grid_constant__ DevParams P0, const SceneTab T, int n, const flo
 template <bool BATCH>
 __global__ void __launch_bounds__(kThreads)
 k_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, float time, float dt, float ss,
-          const uint32_t *__restrict__ gcell, const float4 *__restrict__ force,
-          float4 *__restrict__ pos, float4 *__restrict__ vel, float4 *__restrict__ veval) {
+          const uint32_t *gcell, const float4 *force,
+          float4 *pos, float4 *vel, float4 *veval) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -685,14 +696,14 @@ template <bool PRUNE, bool LIST, bool BATCH>
 __global__ void __launch_bounds__(kForceThreads, 8)
 k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, float *time_dev, int slot,
                 float dt,
-                const float4 *__restrict__ pos_in, const float4 *__restrict__ veval_in,
-                const float *__restrict__ press, const uint32_t *__restrict__ gcell,
-                const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
-                const uint32_t *__restrict__ upbits,
-                const uint32_t *__restrict__ hitlist, const uint32_t *__restrict__ hitcnt,
-                const float4 *__restrict__ pairdata, const CrowdTiles over, float4 *__restrict__ vel,
-                float4 *__restrict__ force, float4 *__restrict__ pos_out, float4 *__restrict__ veval_out,
-                uint32_t *__restrict__ err, int base, float *__restrict__ host_pos) {
+                const float4 *pos_in, const float4 *veval_in,
+                const float *press, const uint32_t *gcell,
+                const uint32_t *off, const uint32_t *cnt,
+                const uint32_t *upbits,
+                const uint32_t *hitlist, const uint32_t *hitcnt,
+                const float4 *pairdata, const CrowdTiles over, float4 *vel,
+                float4 *force, float4 *pos_out, float4 *veval_out,
+                uint32_t *err, int base, float *host_pos) {
     follow_previous();
     // host_pos (fl_run_from_host): the new positions also go straight into
     // the caller's page-locked float3 array, in slot order, while the pass
@@ -705,7 +716,7 @@ k_force_advance(const __grid_constant__ DevParams P0, const SceneTab T, int n, f
     const bool active = gc != kUndef;
     ForcePoint fp = force_point(P, i, active, pos_in, veval_in, press);
     if constexpr (LIST) {
-        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, pairdata, over)) return;
+        if (!force_from_list<BATCH>(P, i, active ? hitcnt[i] : 0u, fp, hitlist, after_wait(pairdata), over)) return;
     } else {
         force_by_walk<PRUNE>(P, active, gc, fp, pos_in, veval_in, press, off, cnt, upbits);
     }
@@ -742,9 +753,10 @@ __global__ void __launch_bounds__(kThreads) k_copy_state(int n, const __grid_con
     for (int k = 0; k < 4; k++) { c.dst4[k][i] = v[k]; c.dst1[k][i] = w[k]; }
 }
 
+// (launched plainly: it does not wait)
 __global__ void k_set_word(uint32_t *word, uint32_t value) { *word = value; }
 
-__global__ void k_pack3(int n, const float4 *__restrict__ src, float *__restrict__ dst) {
+__global__ void k_pack3(int n, const float4 *src, float *dst) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -752,7 +764,7 @@ __global__ void k_pack3(int n, const float4 *__restrict__ src, float *__restrict
     dst[3 * i + 0] = v.x; dst[3 * i + 1] = v.y; dst[3 * i + 2] = v.z;
 }
 
-__global__ void k_unpack3(int n, const float *__restrict__ src, float4 *__restrict__ dst) {
+__global__ void k_unpack3(int n, const float *src, float4 *dst) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -782,8 +794,8 @@ __global__ void k_unpack3_set(int n, const __grid_constant__ Unpack3Set u) {
 
 // FGCELL readback of a batched system: internal cell entries count one
 // out-of-range bin per earlier scene; the reference layout does not.
-__global__ void k_gcell_ref(int n, const uint32_t *__restrict__ gcell, const uint16_t *__restrict__ scene,
-                            uint32_t *__restrict__ out) {
+__global__ void k_gcell_ref(int n, const uint32_t *gcell, const uint16_t *scene,
+                            uint32_t *out) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -791,7 +803,7 @@ __global__ void k_gcell_ref(int n, const uint32_t *__restrict__ gcell, const uin
     out[i] = (g == kUndef) ? kUndef : g - (uint32_t)scene[i];
 }
 
-__global__ void k_grid_identity(int n, const uint32_t *__restrict__ gcell, uint32_t *__restrict__ dst) {
+__global__ void k_grid_identity(int n, const uint32_t *gcell, uint32_t *dst) {
     follow_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -809,9 +821,9 @@ constexpr int kConsChunk = 8192;
 constexpr int kConsThreads = 256;
 
 __global__ void __launch_bounds__(kConsThreads)
-k_conservation(const __grid_constant__ DevParams P0, const SceneTab T, const int *__restrict__ sbase,
-               const int *__restrict__ sn, int nchunks, const float4 *__restrict__ pos,
-               const float4 *__restrict__ vel, double *__restrict__ partial) {
+k_conservation(const __grid_constant__ DevParams P0, const SceneTab T, const int *sbase,
+               const int *sn, int nchunks, const float4 *pos,
+               const float4 *vel, double *partial) {
     follow_previous();
     const int chunk = blockIdx.x, scene = blockIdx.y;
     const DevParams &P = T.params ? T.params[scene] : P0;
@@ -852,8 +864,8 @@ k_conservation(const __grid_constant__ DevParams P0, const SceneTab T, const int
 // cell g must carry gcell == g and gndx == its rank; tail slots must be UNDEF.
 template <bool BATCH>
 __global__ void k_integrity(const __grid_constant__ DevParams P0, const SceneTab T, int gcells, int n,
-                            const uint32_t *__restrict__ off, const uint32_t *__restrict__ cnt,
-                            const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ gndx,
+                            const uint32_t *off, const uint32_t *cnt,
+                            const uint32_t *gcell, const uint32_t *gndx,
                             unsigned long long *bad) {
     follow_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -874,7 +886,7 @@ __global__ void k_integrity(const __grid_constant__ DevParams P0, const SceneTab
 // sides of it from being dependent ones: gradients of 65,536 points 3,356 us
 // with it, 3,191 without.)
 constexpr int kClearWords = 4;   // a thread (and pass)
-__global__ void __launch_bounds__(kThreads) k_clear(unsigned long long *__restrict__ p, size_t words) {
+__global__ void __launch_bounds__(kThreads) k_clear(unsigned long long *p, size_t words) {
     follow_previous();
     for (size_t b = (size_t)blockIdx.x * (kThreads * kClearWords); b < words;
          b += (size_t)gridDim.x * (kThreads * kClearWords))

@@ -72,7 +72,7 @@ __device__ __forceinline__ uint32_t look_back(const uint64_t *status, int last, 
 }
 
 __global__ void __launch_bounds__(kThreads)
-k_scan(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, uint64_t *status,
+k_scan(const uint32_t *in, uint32_t *out, uint64_t *status,
        uint32_t *ticket, int ntiles, uint32_t epoch, int inclusive, uint32_t *err, int spin_limit,
        uint32_t first_tile) {
     follow_previous();

@@ -34,8 +34,12 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 // A pair record -- (position, density), (evaluated velocity, 0) -- in one
 // 256-bit load: with two 128-bit ones the force pass waited on twice the
 // requests (1,000,000 points 94 -> 87 us, 250,000 with gridSrch 3 88 -> 73).
+// To the compiler the load is a function of its address, free to move (volatile,
+// the batched force pass took 56 -> 60 registers and 120 -> 138 us): pairdata
+// has to be a pointer got after the wait (after_wait), and no kernel that calls
+// this writes the records.
 __device__ __forceinline__ void load_record(const float4 *__restrict__ pairdata, uint32_t j, float4 &q, float4 &v) {
-    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
         : "l"(pairdata + 2 * (size_t)j));
 }
