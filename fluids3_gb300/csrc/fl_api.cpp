@@ -878,22 +878,21 @@ static int record(fl_system *s, TimingState *t, int k) {
     return FL_OK;
 }
 
-// Whether steps count as cell-task steps (fl_passes_steps,
-// fl_neighbour_passes_in_use): by mode, or with FL_PASSES_AUTO while a cell is
-// crowded.
-static bool cells_selected(const fl_system *s) {
+// Whether packed tiles may be walked apart (k_density_packed), and steps count
+// as cell-task steps: by mode, or with FL_PASSES_AUTO while a cell is crowded.
+bool fl_cells_selected(const fl_system *s) {
     return s->passes == FL_PASSES_CELL_TASKS || (s->passes == FL_PASSES_AUTO && s->auto_cells);
 }
 
 static int passes_of_step(const fl_system *s, bool taped) {
-    return cells_selected(s) && s->D.prune && !taped && s->n > 0 ? 1 : 0;
+    return fl_cells_selected(s) && s->D.prune && !taped && s->n > 0 ? 1 : 0;
 }
 
 // FL_PASSES_AUTO: every step's sort records the largest in-range cell above
 // 128 points and sends it to page-locked host memory; the next call reads
-// whatever copy has arrived (a step or two old, no wait) and switches what
-// the steps count as, with hysteresis. The kernels are the same either way:
-// crowded tiles are found, and shared between warps, in every step.
+// whatever copy has arrived (a step or two old, no wait) and switches, with
+// hysteresis. A search block of 8 cells holds kPackedBlock (4,096) points from
+// a largest cell of 512 on: below, the launch for packed tiles would find none.
 constexpr uint32_t kAutoCellsOn = 512, kAutoCellsOff = 384;
 
 static void update_auto(fl_system *s, uint32_t at_least = 0) {
@@ -905,8 +904,8 @@ static void update_auto(fl_system *s, uint32_t at_least = 0) {
     else if (s->auto_cells && big < kAutoCellsOff) s->auto_cells = 0;
 }
 
-// The state was replaced (particles set, checkpoint restored): back to the
-// per-point passes until a count of the new state arrives (the counts
+// The state was replaced (particles set, checkpoint restored): no launch for
+// packed tiles until a count of the new state arrives (the counts
 // carry the state's epoch, so an older count in flight is ignored).
 static int reset_auto(fl_system *s) {
     s->auto_cells = 0;
@@ -1118,19 +1117,19 @@ static int capture_pair(fl_system *s) {
     }
     s->graph_steps = 2;
     s->graph_n = s->n;
+    s->graph_cells = fl_cells_selected(s);
     for (int k = 0; k < F_COUNT; k++) s->graph_live[k] = live[k];
     return FL_OK;
 }
 
 static int run_steps_graph(fl_system *s, int nsteps);
 
-// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps. What the
-// first two chunks count as comes from whatever has reached the host by then,
-// a later one's from the chunk two before it, which the host waits for (one
-// chunk stays queued): the larger of its second step's largest cell, copied
-// aside for this, and of the last that was reported, so that a crowd which
-// formed and dispersed within a chunk is seen. Calls of up to two chunks wait
-// for nothing.
+// With FL_PASSES_AUTO a long call runs in chunks of kAutoChunk steps. The first
+// two chunks' passes come from whatever has reached the host by then, a later
+// one's from the chunk two before it, which the host waits for (one chunk stays
+// queued): the larger of its second step's largest cell, copied aside for this,
+// and of the last that was reported, so that a crowd which formed and dispersed
+// within a chunk is seen. Calls of up to two chunks wait for nothing.
 constexpr int kAutoChunk = 32;
 
 extern "C" int fl_run_steps(fl_system *s, int nsteps) {
@@ -1169,7 +1168,7 @@ static int run_steps_graph(fl_system *s, int nsteps) {
     if (pairs > 0) {
         // the captured launches hold the live copies and the point count (a
         // restored checkpoint may have another)
-        bool match = s->graph_exec != nullptr && s->graph_n == s->n;
+        bool match = s->graph_exec != nullptr && s->graph_n == s->n && s->graph_cells == fl_cells_selected(s);
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
         for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));

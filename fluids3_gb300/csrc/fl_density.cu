@@ -25,6 +25,10 @@
 //      rounding, same order), so neither the filter nor the candidates that
 //      another point of the warp brought in change a bit of the result.
 //
+// Two classes of tiles go other ways (crowded_tile, packed_tile below): crowded
+// ones that are few are shared by whole blocks of k_density, packed ones that
+// are many are walked apart, without the filter, by k_density_packed.
+//
 // What bounds it: instruction issue (88 warp instructions a point, half of them
 // the sum's: about 24 visits a warp, the lanes' mean being 16). A thread per
 // point over flag-pruned candidates took 157, and its chain of dependent loads
@@ -39,6 +43,7 @@
 // too little work for tcgen05's descriptors, and the accumulator's signs
 // are wanted in registers at once.
 #include <algorithm>
+#include <type_traits>
 
 #include <cuda_fp16.h>
 
@@ -551,7 +556,165 @@ __device__ __noinline__ void crowded_tile(const DevParams &P0, const SceneTab &T
 // fewer than would keep every warp of those blocks busy by itself. Density
 // launch with and without sharing, dam break after 90 steps: 65,536 points 172
 // and 290 us, 1,048,576 points 823 and 470 us.
-__device__ __forceinline__ bool shared_tiles(uint32_t count, int workers) { return count < 3u * (uint32_t)workers; }
+__host__ __device__ __forceinline__ bool shared_tiles(uint32_t count, int workers) { return count < 3u * (uint32_t)workers; }
+
+// A packed tile by one warp, for when there are such tiles for every warp.
+// Points that close together are nearly all pairs of one another, so nothing is
+// filtered but by the tile's box: all lanes test every candidate, in order, four
+// of them a round trip to shared memory and two an instruction (packed FP32).
+// Bound by the FP32 pipe. Wave tank of 4,000,000 points after 250, 300 and 340
+// steps (largest cell 14,051, 17,717, 97,686), density launches: 20.5, 49.3 and
+// 139 ms by the filter, 12.5, 27.1 and 69.3 so; 1,000,000 points after 400 steps
+// 27.6 and 13.4.
+constexpr int kPackedCap = 256;                    // candidates staged per round
+constexpr int kPackedRow = kPackedCap + 4;         // x, y, z, slot: a row each; a round's last four are made whole
+constexpr int kPackedThreads = 128, kPackedBlocksPerSm = 8;
+
+template <bool BATCH>
+__device__ __forceinline__ void packed_tile(const DevParams &P0, const SceneTab &T, uint32_t tile, int n,
+                                         const float4 *__restrict__ pos, const uint32_t *__restrict__ gcell,
+                                         const uint32_t *__restrict__ off, const float4 *__restrict__ veval,
+                                         float *__restrict__ press, uint32_t *__restrict__ hitlist,
+                                         uint32_t *__restrict__ hitcnt, float4 *__restrict__ pairdata,
+                                         uint32_t *s_warp) {
+    const unsigned lane = lane_id(), below = (1u << lane) - 1u;
+    float *const s_x = reinterpret_cast<float *>(s_warp), *const s_y = s_x + kPackedRow, *const s_z = s_y + kPackedRow;
+    uint32_t *const s_slot = s_warp + 3 * kPackedRow;
+    const int i = (int)(tile * 32u + lane);
+    const uint32_t gc = (i < n) ? gcell[i] : kUndef;
+    const bool active = gc != kUndef;
+    const DevParams &P = (BATCH && i < n) ? T.params[T.point_scene[i]] : P0;
+    Sum s;
+    s.p = active ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    s.sum = 0.0f;
+    s.nh = 0;
+    s.next = hitlist + list_at(P, i, 0);
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    unsigned heads = segment_heads(gc, active);
+    while (heads) {
+        const unsigned seg = next_segment(heads, act);
+        const bool mine = (seg >> lane) & 1u;
+        const int first = __ffs(seg) - 1, last = 31 - __clz(seg);
+        const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + first]] : P0;
+        const int ca = (int)__shfl_sync(0xffffffffu, gc, first), cb = (int)__shfl_sync(0xffffffffu, gc, last);
+        const Box box = box_of(s.p, seg);
+        const float bx = box.ex + PS.band, by = box.ey + PS.band, bz = box.ez + PS.band;
+        const float rd2 = PS.rd2, d2 = PS.d2, none = __int_as_float(0x7fffffff);   // (NaN passes no test)
+        const uint32_t cap = (uint32_t)PS.hcap;
+        const float px = mine ? s.p.x : none;
+        const uint64_t x2 = pk2(px, px), y2 = pk2(s.p.y, s.p.y), z2 = pk2(s.p.z, s.p.z), r2 = pk2(rd2, rd2),
+                       k2 = pk2(d2, d2);
+        RowRange own = {0u, 0xffffffffu};
+        // candidate e (its distance and term) is a pair: the next of the list
+        // while it has room (ROOM), and the next term of the sum
+        auto pair = [&](auto room, auto ranges, int e, float dsq, float t) {
+            bool hit = dsq < rd2 && dsq > 0.0f;
+            if (decltype(ranges)::value) hit = hit && s_slot[e] - own.lo < own.len;
+            s.sum += hit ? t : 0.0f;
+            if (decltype(room)::value) {
+                if (hit && s.nh < cap) s.next[32u * s.nh] = s_slot[e];
+            }
+            s.nh += hit ? 1u : 0u;
+        };
+        auto round = [&](auto room, auto ranges, int count) {
+            for (int e = 0; e < count; e += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(s_x + e), y = *reinterpret_cast<const float4 *>(s_y + e),
+                             z = *reinterpret_cast<const float4 *>(s_z + e);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint64_t dx = sub2(x2, h ? pk2(x.z, x.w) : pk2(x.x, x.y)),
+                                   dy = sub2(y2, h ? pk2(y.z, y.w) : pk2(y.x, y.y)),
+                                   dz = sub2(z2, h ? pk2(z.z, z.w) : pk2(z.x, z.y));
+                    float xa, xb, ya, yb, za, zb, ta, tb;
+                    up2(mul2(dx, dx), xa, xb);
+                    up2(mul2(dy, dy), ya, yb);
+                    up2(mul2(dz, dz), za, zb);
+                    const float da = xa + ya + za, db = xb + yb + zb;   // (in scalar: see pk2)
+                    const uint64_t t = mul2(sub2(r2, pk2(da, db)), k2);
+                    up2(mul2(mul2(t, t), t), ta, tb);
+                    pair(room, ranges, e + 2 * h, da, ta);
+                    pair(room, ranges, e + 2 * h + 1, db, tb);
+                }
+            }
+        };
+        int cnt = 0;
+        auto drain = [&]() {
+            if (lane < 4) s_x[cnt + (int)lane] = none;
+            __syncwarp();
+            const std::true_type yes;
+            const std::false_type no;
+            if (__any_sync(0xffffffffu, mine && s.nh < cap)) round(yes, yes, cnt);
+            else if (ca != cb) round(no, yes, cnt);
+            else round(no, no, cnt);
+            cnt = 0;
+            __syncwarp();
+        };
+        for (int r = 0; r < 4; r++) {
+            const int at = ((r >> 1) * PS.gridRes.z + (r & 1)) * PS.gridRes.x - PS.nadj;
+            const uint32_t lo = off[ca + at], hi = off[cb + at + 2];
+            if (ca != cb && mine) {   // points of several cells: each takes its own block's candidates
+                own.lo = off[(int)gc + at];
+                own.len = off[(int)gc + at + 2] - own.lo;
+            }
+            if (lo == hi) continue;
+            float4 next = pos[min(lo + lane, hi - 1u)];
+            for (uint32_t jb = lo; jb < hi; jb += 32u) {
+                const float4 q = next;
+                const uint32_t j = jb + lane;
+                next = pos[min(j + 32u, hi - 1u)];
+                const bool keep = j < hi && fabsf(q.x - box.ox) <= bx && fabsf(q.y - box.oy) <= by && fabsf(q.z - box.oz) <= bz;
+                const unsigned kept = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const int e = cnt + __popc(kept & below);
+                    s_x[e] = q.x, s_y[e] = q.y, s_z[e] = q.z;
+                    s_slot[e] = j;
+                }
+                cnt += __popc(kept);
+                if (cnt > kPackedCap - 32) drain();
+            }
+            if (ca != cb && cnt) drain();   // the next row has other ranges
+        }
+        if (cnt) drain();
+    }
+    if (i < n) finish(P, s, i, active, veval, press, hitcnt, pairdata);
+}
+
+// Whether packed tiles are walked apart: too many to be shared, and not few
+// beside the crowded ones (they are done before the others begin, so a launch
+// of few of them ends in waits). Density of the wave tank by the filter | so:
+// 4,000,000 points after 160, 170 and 180 steps (12,630, 15,690 and 18,935
+// packed tiles, 0.28, 0.36 and 0.47 of the crowded) 2.21 | 2.26, 2.41 | 2.41,
+// 2.66 | 2.58 ms; 1,000,000 after 210 (3,877, 0.72) 1.23 | 1.08.
+__device__ __forceinline__ bool walked_apart(uint32_t crowded, uint32_t packed, int workers) {
+    return !shared_tiles(packed, workers) && 5ull * packed >= 2ull * crowded;
+}
+
+// The packed tiles that are walked apart, a warp each. Launched before
+// k_density, which then finds none (a kernel of its own: with this walk in
+// k_density, inlined or called, its own tiles take 5-9% longer).
+template <bool BATCH>
+__global__ void __launch_bounds__(kPackedThreads)
+k_density_packed(const __grid_constant__ DevParams P0, const SceneTab T, int n, const float4 *pos,
+                 const uint32_t *gcell, const uint32_t *off, const float4 *veval, float *press, uint32_t *hitlist,
+                 uint32_t *hitcnt, float4 *pairdata, const CrowdTiles tiles, int workers) {
+    follow_previous();
+    __shared__ __align__(16) uint32_t s_rows[kPackedThreads / 32][4 * kPackedRow];
+    volatile uint32_t *const counters = tiles.counters;
+    const uint32_t crowded = counters[0], packed = counters[1];
+    if (!walked_apart(crowded, packed, workers)) return;
+    for (;;) {
+        uint32_t k = 0;
+        if (lane_id() == 0) k = atomicAdd(&tiles.counters[3], 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= packed) break;
+        packed_tile<BATCH>(P0, T, tile_at(tiles, k, packed), n, pos, gcell, off, veval, press, hitlist, hitcnt, pairdata,
+                           s_rows[threadIdx.x >> 5]);
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&tiles.counters[4], 1u) == gridDim.x - 1) counters[1] = 0;   // every block has read it
+}
 
 // The first `workers` blocks take the tiles that the sort's gather listed and
 // that are set apart (workers 0: none are), the others 32 slots a warp.
@@ -641,6 +804,13 @@ int fl_launch_density(fl_system *s) {
                s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
     } else {
         const int workers = s->tiles_listed ? std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32) : 0;
+        if (workers && fl_cells_selected(s) && !shared_tiles((uint32_t)(s->n + 31) / 32, workers)) {
+            auto packed = s->batched ? k_density_packed<true> : k_density_packed<false>;
+            launch(packed, kPackedBlocksPerSm * s->num_sms, kPackedThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
+                   s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),
+                   s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata, s->tiles, workers);
+            FL_LAUNCH_CHECK("density_packed");
+        }
         const size_t smem = (size_t)(bs / 32) * kWarpWords * sizeof(uint32_t);
         auto kern = s->batched ? k_density<true> : k_density<false>;
         launch(kern, workers + blocks_for(s->n, bs), bs, smem, s->stream, s->D, fl_scene_tab(s), s->n,

@@ -145,7 +145,7 @@ struct fl_system {
     int passes;            // FL_PASSES_*: the neighbour passes of the fused step
     int auto_cells;        // FL_PASSES_AUTO: a cell is crowded (hysteresis state)
     int capturing;         // run_step is being captured into the step-pair graph
-    int64_t passes_steps[2]; // fused steps issued with the per-point passes / the cell tasks
+    int64_t passes_steps[2]; // fused steps issued as per-point steps / as cell-task steps
     uint32_t *crowd_dev;   // largest in-range cell above 128 points, this step (0: none)
     uint32_t *crowd_epoch; // device: the state's epoch (bumped when the state is replaced)
     uint32_t *crowd_host;  // page-locked [count, epoch], written by each step's sort; [2], [3]: fl_run_steps
@@ -185,6 +185,7 @@ struct fl_system {
     cudaGraphExec_t graph_exec;
     int graph_steps, graph_n;   // the captured steps, their point count
     int graph_live[F_COUNT];
+    bool graph_cells;      // whether they walk packed tiles apart (fl_cells_selected)
 
     // checkpoints: per slot, one copy of every field's live buffer + time
     // one more slot than the caller's: the autotuner's own
@@ -300,6 +301,7 @@ int fl_launch_gather_all(fl_system *s);
 int fl_density_init();   // once per process is enough; outside any stream capture
 int fl_density_block(const fl_system *s);
 int fl_launch_density(fl_system *s);
+bool fl_cells_selected(const fl_system *s);   // whether a launch of its own walks packed tiles (fl_api.cpp)
 int fl_launch_force(fl_system *s);
 // slots [begin, end) (end < 0: n); both whole blocks of fl_force_block(s)
 // threads, except end == n

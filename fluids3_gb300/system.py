@@ -397,12 +397,13 @@ class FluidSystem:
         call("fl_set_launch_shapes", self._h, shapes)
 
     def SetNeighbourPasses(self, mode: str) -> None:
-        """Neighbour passes of the fused step. "points", "cells" and "auto"
-        (default) run the same kernels and differ in what their steps count as
-        (PassesSteps): "auto" as "points" until the largest cell reaches 512
-        points, as "cells" from then until it falls below 384. "pairs": a
-        density walk shared by two points of a cell that visit the same
-        candidates (every density pass of the system). Results are
+        """Neighbour passes: "points", densities from a walk that 32 slots
+        share; "cells", the same with a launch of its own for tiles whose
+        search blocks hold over 4,096 points, where a step has many of them;
+        "auto" (default), "points" until the largest cell reaches 512 points,
+        "cells" from then until it falls below 384; "pairs", a density walk
+        shared by two points of a cell that visit the same candidates. The
+        mode holds for every density pass of the system. Results are
         bit-identical."""
         call("fl_set_neighbour_passes", self._h, PASSES.index(mode))
 
@@ -414,8 +415,8 @@ class FluidSystem:
         return PASSES[call("fl_neighbour_passes_in_use", self._h)]
 
     def PassesSteps(self) -> tuple:
-        """Fused steps issued so far that counted as per-point steps and as
-        cell-task steps."""
+        """Fused steps issued so far as per-point steps and as cell-task steps
+        (taped steps count as per-point steps)."""
         c = (C.c_int64 * 2)()
         call("fl_passes_steps", self._h, c)
         return int(c[0]), int(c[1])

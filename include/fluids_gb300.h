@@ -335,24 +335,27 @@ int fl_set_launch_shapes(fl_system *s, const int *shapes);
 
 /* Which neighbour passes the fused step (fl_run, fl_run_steps,
  * fl_run_from_host) uses; all give bit-identical densities, forces and
- * states. FL_PASSES_PER_POINT, FL_PASSES_CELL_TASKS and FL_PASSES_AUTO (the
- * default) run the same kernels: each point's density and pair list from a
- * walk that 32 consecutive slots share, its force from the list, and crowded
- * tiles of slots shared between warps wherever a step has them. The three
- * differ in what their steps count as (fl_passes_steps): with FL_PASSES_AUTO
- * as per-point steps until the largest in-range cell reaches 512 points, as
- * cell-task steps from then until it falls below 384 (each step's sort records
- * the largest cell; a fused-step call acts on the last value that has reached
- * the host, a step or two old); steps of a search with gridSrch other than 2
- * and taped steps always count as per-point steps. FL_PASSES_POINT_PAIRS:
- * where gridSrch is 2, one thread walks the search block once for two points
- * of a cell with the same lower-band bits (which visit the same candidates in
- * the same order); this one holds for every density pass of the system (fused
- * step, phase entry points, tapes). No counterpart in the reference (which has
- * only the per-point walk). fl_neighbour_passes returns the mode set;
- * fl_neighbour_passes_in_use what the next fused step counts as
- * (FL_PASSES_AUTO resolved with the latest count on the host: after
- * fl_sync, the last step's). */
+ * states. FL_PASSES_PER_POINT: each point's density and pair list from a walk
+ * that 32 consecutive slots share, its force from the list, and crowded tiles
+ * of slots shared between warps wherever a step has them.
+ * FL_PASSES_CELL_TASKS: the same, except that tiles whose search blocks hold
+ * over 4,096 points, where a step has enough of them for a warp each, take
+ * their densities in a launch of their own that tests every candidate (nearly
+ * all are pairs there): faster in a deep collapse, and nothing but one more
+ * launch before it. FL_PASSES_AUTO (the default): FL_PASSES_PER_POINT until
+ * the largest in-range cell reaches 512 points (below that no search block
+ * holds so many), FL_PASSES_CELL_TASKS from then until it falls below 384
+ * (each step's sort records the largest cell; a fused-step call acts on the
+ * last value that has reached the host, a step or two old).
+ * FL_PASSES_POINT_PAIRS: where gridSrch is 2, one thread walks the search
+ * block once for two points of a cell with the same lower-band bits (which
+ * visit the same candidates in the same order). The mode holds for every
+ * density pass of the system (fused step, phase entry points, tapes); it
+ * changes nothing where gridSrch is not 2 (in every scene). No counterpart in
+ * the reference (which has only the per-point walk). fl_neighbour_passes
+ * returns the mode set; fl_neighbour_passes_in_use the passes that the next
+ * fused step takes (FL_PASSES_AUTO resolved with the latest count on the host:
+ * after fl_sync, the last step's). */
 #define FL_PASSES_PER_POINT   0
 #define FL_PASSES_CELL_TASKS  1
 #define FL_PASSES_POINT_PAIRS 2
@@ -360,8 +363,10 @@ int fl_set_launch_shapes(fl_system *s, const int *shapes);
 int fl_set_neighbour_passes(fl_system *s, int mode);
 int fl_neighbour_passes(const fl_system *s);
 int fl_neighbour_passes_in_use(fl_system *s);
-/* Fused steps issued since creation that counted as per-point steps
- * (counts[0]) and as cell-task steps (counts[1]). */
+/* Fused steps issued since creation as per-point steps (counts[0]) and as
+ * cell-task steps (counts[1]). Steps of a search with gridSrch other than 2,
+ * taped steps and the replays of a tape that keeps its pair lists count as
+ * per-point steps in every mode. */
 int fl_passes_steps(const fl_system *s, int64_t *counts);
 
 /* Wait for the system stream; returns FL_ERR_DEVICE if a kernel raised the
