@@ -63,7 +63,14 @@ constexpr int kMaskRow = kWords + 1;            // (odd: the rows of a tile fall
 // of them, and the points' product rows, whose place the masks then take
 constexpr int kWarpWords = kCap * 4 + 32 * 8 + 32 * 8;
 static_assert(32 * kMaskRow <= 32 * 8, "the masks fit where the product rows were");
-constexpr int kMaxSegments = 8;                 // runs of points a warp takes one by one; beyond, lanes walk alone
+// Runs of points that a warp takes one by one, and cells that its points may lie
+// in; beyond, the lanes walk alone: in spray, a run's union of blocks holds few
+// candidates of any one point. Density launch of 1,000,000 points spread evenly,
+// cells of 2h with 1, 2, 3, 5 and 8 points: 44, 50, 60, 74, 81 us with 6 cells,
+// 134, 95, 88, 82, 80 with as many as there are (8 runs then), 44, 51, 58, 73, 89
+// with 4. The wave tank (1,000,000) after 4 steps 136, 153, 136, the dam break
+// (65,536) 29.1, 29.4, 30.9; with 2 runs that took 31.9.
+constexpr int kMaxSegments = 4, kMaxCells = 6;
 constexpr float kUnits = 1000.0f;               // half the widest side of the box, in units (2 x stays exact in half)
 constexpr float kBase = 2048.0f;                // squares are split into kBase * high + low, both exact in half
 constexpr float kFar = 6.0e4f;                  // times kBase: beyond any square
@@ -760,7 +767,9 @@ k_density(const __grid_constant__ DevParams P0, const SceneTab T, int n, const f
     s.next = hitlist + list_at(P, i, 0);
     const unsigned act = __ballot_sync(0xffffffffu, active);
     unsigned heads = segment_heads(gc, active);
-    if (__popc(heads) <= kMaxSegments) {
+    const uint32_t before = __shfl_up_sync(0xffffffffu, gc, 1);
+    const unsigned cells = __ballot_sync(0xffffffffu, active && (lane == 0 || before != gc));
+    if (__popc(cells) <= kMaxCells && __popc(heads) <= kMaxSegments) {
         while (heads) {
             const unsigned seg = next_segment(heads, act);
             const DevParams &PS = BATCH ? T.params[T.point_scene[i - (int)lane + __ffs(seg) - 1]] : P0;
