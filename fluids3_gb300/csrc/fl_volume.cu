@@ -21,14 +21,15 @@
 // uneven counts cost 10% more; bricks of 4 x 4 x 4, two voxels a lane, were no
 // faster.
 //
-// k_sample_wide: a warp per voxel, a lane per point, for lattices so coarse
-// that a brick's voxels share few points: 32^3 voxels over 1,000,000 points
-// 122 us (a thread per voxel: too few of them), 205 (bricks), 20.
+// k_sample_wide: 1 to 32 lanes a voxel, each a part of its points, for lattices
+// so coarse that a brick's voxels share few points: 32^3 voxels over 1,000,000
+// points 122 us (a thread per voxel as it was), 205 (bricks), 20 (32 lanes).
 //
 // The reference's exponent, -(sqrt(d2 dsq))^2 / h2, is formed as
 // d2 dsq times -1 / h2 (as high and low parts): fewer roundings, no square
 // root and no division.
 #include <math.h>
+#include <type_traits>
 
 #include "fl_internal.h"
 
@@ -150,7 +151,17 @@ k_sample_bricks(const __grid_constant__ DevParams P, const __grid_constant__ Lat
             cnt = 0;
             __syncwarp();
         };
-        for (int y = y0 - 1; y <= y1 + srch - 2; y++)
+        // most bricks of a volume may hold no point: its rows of cells are looked
+        // at together first, a lane each (20,000 points in a mostly empty box,
+        // 192^3 voxels: 113 us without, 85 with)
+        const int zs = z1 - z0 + srch, rows = (y1 - y0 + srch) * zs;
+        bool filled = rows > 32;
+        if ((int)lane < rows && !filled) {
+            const int row = ((y0 - 1 + (int)lane / zs) * P.gridRes.z + z0 - 1 + (int)lane % zs) * P.gridRes.x;
+            filled = off[row + x0 - 1] < off[row + x1 + srch - 1];
+        }
+        const int y_end = __any_sync(0xffffffffu, filled) ? y1 + srch - 2 : y0 - 2;
+        for (int y = y0 - 1; y <= y_end; y++)
             for (int z = z0 - 1; z <= z1 + srch - 2; z++) {
                 const int row = (y * P.gridRes.z + z) * P.gridRes.x;
                 const uint32_t lo = off[row + x0 - 1], hi = off[row + x1 + srch - 1];
@@ -174,42 +185,57 @@ k_sample_bricks(const __grid_constant__ DevParams P, const __grid_constant__ Lat
     if (exists) out[((size_t)iz * L.res.y + iy) * L.res.x + ix] = v * L.scalar;
 }
 
+template <int LANES>   // a power of two up to 32
 __global__ void __launch_bounds__(kVolumeThreads)
 k_sample_wide(const __grid_constant__ DevParams P, const __grid_constant__ Lattice L, const float4 *__restrict__ pos,
               const uint32_t *__restrict__ off, float *__restrict__ out) {
-    const unsigned lane = lane_id();
-    const uint32_t i = blockIdx.x * (kVolumeThreads / 32) + (threadIdx.x >> 5), line = i / (uint32_t)L.res.x;
+    const uint32_t part = threadIdx.x % LANES;
+    const uint32_t i = blockIdx.x * (kVolumeThreads / LANES) + threadIdx.x / LANES, line = i / (uint32_t)L.res.x;
     const uint32_t iz = line / (uint32_t)L.res.y;
-    if (iz >= (uint32_t)L.res.z) return;
     const float px = voxel_at((int)(i % (uint32_t)L.res.x), L.res.x, L.bmin.x, L.bmax.x);
     const float py = voxel_at((int)(line % (uint32_t)L.res.y), L.res.y, L.bmin.y, L.bmax.y);
     const float pz = voxel_at((int)iz, L.res.z, L.bmin.z, L.bmax.z);
     const VoxelCell c = voxel_cell(P, px, py, pz);
+    const bool exists = iz < (uint32_t)L.res.z;
     float v = 0.0f;
-    if (c.in) {
+    if (exists && c.in) {
         const int cell = (c.y * P.gridRes.z + c.z) * P.gridRes.x + c.x;
         for (int r = 0; r < P.gridSrch * P.gridSrch; r++) {
             const int at = cell - P.nadj + P.adj[r * P.gridSrch];
             const uint32_t lo = off[at], hi = off[at + P.gridSrch];
-            for (uint32_t j = lo + lane; j < hi; j += 32u) {
+            for (uint32_t j = lo + part; j < hi; j += (uint32_t)LANES) {
                 const float4 q = pos[j];
                 const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
                 const float dsq = dx * dx + dy * dy + dz * dz;
                 if (dsq < P.rd2 && dsq > 0.0f) v += weight(L, dsq, P.d2);
             }
         }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
     }
-    if (lane == 0) out[i] = v * L.scalar;
+#pragma unroll
+    for (int d = LANES / 2; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if (exists && part == 0) out[i] = v * L.scalar;
 }
 
-// Bricks while the brick's widened box is small enough against a voxel's search
-// block: both sides measured over spacings of 0.4 to 14 world units, 20,000 to
-// 1,000,000 points and both search blocks; they cross at about 1.0 of the block
-// with gridSrch 2 (spacing 2.3-3.1: 250,000 points at 2.3 66 | 115 us, bricks |
-// wide, at 3.0 63 | 52) and 3.4 with gridSrch 3 (2.3: 148 | 128, 1.5: 188 |
-// 422), in between srch^3 / 8.
+// Lanes a voxel when not by bricks: as many as leave the chip's threads full
+// once (a power of two up to 32). 16^3, 32^3, 48^3 and 64^3 voxels over
+// 1,000,000 points in a third of its box: one lane 60, 60, 60, 61 us, 32 lanes
+// 20, 29, 48, 88, the rule's 32, 8, 2, 1 lanes 20, 29, 49, 61.
+int wide_lanes(long long voxels, int num_sms) {
+    int lanes = 1;
+    while (lanes < 32 && 2 * lanes * voxels <= 2048LL * num_sms) lanes *= 2;
+    return lanes;
+}
+
+// Bricks for lattices of at least 20,000 voxels (fewer are too few warps: 16^3
+// over the middle of 250,000 points, 0.4 apart) while the brick's
+// widened box is no more than 1.1 times a voxel's search block. Both sides
+// measured over spacings of 0.15 to 14 world units, 20,000 to 4,000,000 points
+// and both search blocks, bricks | lanes, us: gridSrch 2, 64^3 over 250,000
+// points, 0.8 apart (0.5 times) 51 | 100; 128^3 over 4,000,000, 2.6 apart (1.3)
+// 300 | 360, over 20,000 in a mostly empty box 39 | 38, 96^3, 3.5 apart (2.1)
+// 232 | 216; gridSrch 3, 64^3, 0.15 apart (0.86) 41 | 38, 0.8 apart (1.8) 55 |
+// 43, 256^3 over 4,000,000, 1.3 apart (2.8) 1,280 | 728.
+constexpr long long kBrickVoxels = 20000;
 bool sample_bricks(const DevParams &P, const Lattice &L) {
     const float h = sqrtf(P.rd2);
     const float dx = (L.bmax.x - L.bmin.x) / (float)L.res.x, dy = (L.bmax.y - L.bmin.y) / (float)L.res.y,
@@ -218,7 +244,7 @@ bool sample_bricks(const DevParams &P, const Lattice &L) {
     const float side = (float)P.gridSrch;
     const float block = side * side * side * P.cellw.x * P.cellw.y * P.cellw.z;
     const float most = fmaxf(fmaxf(3.0f * fabsf(dx) / P.cellw.x, 3.0f * fabsf(dy) / P.cellw.y), fabsf(dz) / P.cellw.z);
-    return box <= 0.125f * side * side * side * block && most < (float)kBrickCells;
+    return (long long)L.res.x * L.res.y * L.res.z >= kBrickVoxels && box <= 1.1f * block && most < (float)kBrickCells;
 }
 
 }  // namespace
@@ -240,8 +266,20 @@ int fl_launch_sample_volume(fl_system *s, const int res[3], const float bmin[3],
         k_sample_bricks<<<blocks_for(n, kVolumeThreads / 32), kVolumeThreads, 0, s->stream>>>(
             s->D, L, bricks, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, out);
     } else {
-        k_sample_wide<<<blocks_for((long long)res[0] * res[1] * res[2], kVolumeThreads / 32), kVolumeThreads, 0,
-                        s->stream>>>(s->D, L, s->f[F_POS].cur<float4>(), s->off, out);
+        const long long n = (long long)res[0] * res[1] * res[2];
+        auto wide = [&](auto lanes) {
+            constexpr int kLanes = decltype(lanes)::value;
+            k_sample_wide<kLanes><<<blocks_for(n, kVolumeThreads / kLanes), kVolumeThreads, 0, s->stream>>>(
+                s->D, L, s->f[F_POS].cur<float4>(), s->off, out);
+        };
+        switch (wide_lanes(n, s->num_sms)) {
+        case 1: wide(std::integral_constant<int, 1>()); break;
+        case 2: wide(std::integral_constant<int, 2>()); break;
+        case 4: wide(std::integral_constant<int, 4>()); break;
+        case 8: wide(std::integral_constant<int, 8>()); break;
+        case 16: wide(std::integral_constant<int, 16>()); break;
+        default: wide(std::integral_constant<int, 32>());
+        }
     }
     FL_LAUNCH_CHECK("sample_volume");
     return FL_OK;
