@@ -1117,7 +1117,7 @@ static int capture_pair(fl_system *s) {
     }
     s->graph_steps = 2;
     s->graph_n = s->n;
-    s->graph_cells = fl_cells_selected(s);
+    s->graph_packed = fl_walks_packed_apart(s);
     for (int k = 0; k < F_COUNT; k++) s->graph_live[k] = live[k];
     return FL_OK;
 }
@@ -1166,9 +1166,9 @@ extern "C" int fl_run_steps(fl_system *s, int nsteps) {
 static int run_steps_graph(fl_system *s, int nsteps) {
     const int pairs = nsteps / 2;
     if (pairs > 0) {
-        // the captured launches hold the live copies and the point count (a
-        // restored checkpoint may have another)
-        bool match = s->graph_exec != nullptr && s->graph_n == s->n && s->graph_cells == fl_cells_selected(s);
+        // the captured launches hold the live copies, the point count (a restored
+        // checkpoint may have another) and whether packed tiles are walked apart
+        bool match = s->graph_exec != nullptr && s->graph_n == s->n && s->graph_packed == fl_walks_packed_apart(s);
         for (int k = 0; k < F_COUNT && match; k++) match = s->graph_live[k] == s->f[k].live;
         if (!match) FL_TRY(capture_pair(s));
         for (int p = 0; p < pairs; p++) FL_CUDA_TRY(cudaGraphLaunch(s->graph_exec, s->stream));

@@ -797,6 +797,12 @@ int fl_density_init() {
 
 int fl_density_block(const fl_system *s) { return s->blk_density ? s->blk_density : kDensityThreads; }
 
+static int density_workers(const fl_system *s) { return std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32); }
+
+bool fl_walks_packed_apart(const fl_system *s) {
+    return fl_cells_selected(s) && s->D.prune && !shared_tiles((uint32_t)(s->n + 31) / 32, density_workers(s));
+}
+
 int fl_launch_density(fl_system *s) {
     if (s->n == 0) return FL_OK;
     if (s->passes == FL_PASSES_POINT_PAIRS && s->D.prune && s->codes_valid) return fl_launch_density_pairs(s);
@@ -812,8 +818,8 @@ int fl_launch_density(fl_system *s) {
                s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),
                s->f[F_PRESS].cur<float>(), s->hitlist, s->hitcnt, s->pairdata);
     } else {
-        const int workers = s->tiles_listed ? std::min(kCrowdBlocksPerSm * s->num_sms, (s->n + 31) / 32) : 0;
-        if (workers && fl_cells_selected(s) && !shared_tiles((uint32_t)(s->n + 31) / 32, workers)) {
+        const int workers = s->tiles_listed ? density_workers(s) : 0;
+        if (workers && fl_walks_packed_apart(s)) {
             auto packed = s->batched ? k_density_packed<true> : k_density_packed<false>;
             launch(packed, kPackedBlocksPerSm * s->num_sms, kPackedThreads, 0, s->stream, s->D, fl_scene_tab(s), s->n,
                    s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, s->f[F_VEVAL].cur<float4>(),

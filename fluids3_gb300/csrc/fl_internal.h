@@ -185,7 +185,7 @@ struct fl_system {
     cudaGraphExec_t graph_exec;
     int graph_steps, graph_n;   // the captured steps, their point count
     int graph_live[F_COUNT];
-    bool graph_cells;      // whether they walk packed tiles apart (fl_cells_selected)
+    bool graph_packed;     // fl_walks_packed_apart as they were captured
 
     // checkpoints: per slot, one copy of every field's live buffer + time
     // one more slot than the caller's: the autotuner's own
@@ -301,7 +301,8 @@ int fl_launch_gather_all(fl_system *s);
 int fl_density_init();   // once per process is enough; outside any stream capture
 int fl_density_block(const fl_system *s);
 int fl_launch_density(fl_system *s);
-bool fl_cells_selected(const fl_system *s);   // whether a launch of its own walks packed tiles (fl_api.cpp)
+bool fl_cells_selected(const fl_system *s);       // by mode and largest cell (fl_api.cpp)
+bool fl_walks_packed_apart(const fl_system *s);   // and with points enough: a launch of its own walks packed tiles
 int fl_launch_force(fl_system *s);
 // slots [begin, end) (end < 0: n); both whole blocks of fl_force_block(s)
 // threads, except end == n
