@@ -87,6 +87,10 @@ struct BrickShared {
     uint32_t mask[kBrickWords][32];    // per voxel: which of them count
 };
 
+// SPARSE: most bricks hold no point, and leave early (20,000 points in a mostly
+// empty box, 192^3 voxels: 113 us without, 85 with; a box full of points takes
+// 2-5% longer with it).
+template <bool SPARSE>
 __global__ void __launch_bounds__(kVolumeThreads)
 k_sample_bricks(const __grid_constant__ DevParams P, const __grid_constant__ Lattice L, int3 bricks,
                 const float4 *__restrict__ pos, const uint32_t *__restrict__ gcell, const uint32_t *__restrict__ off,
@@ -151,16 +155,16 @@ k_sample_bricks(const __grid_constant__ DevParams P, const __grid_constant__ Lat
             cnt = 0;
             __syncwarp();
         };
-        // most bricks of a volume may hold no point: its rows of cells are looked
-        // at together first, a lane each (20,000 points in a mostly empty box,
-        // 192^3 voxels: 113 us without, 85 with)
-        const int zs = z1 - z0 + srch, rows = (y1 - y0 + srch) * zs;
-        bool filled = rows > 32;
-        if ((int)lane < rows && !filled) {
-            const int row = ((y0 - 1 + (int)lane / zs) * P.gridRes.z + z0 - 1 + (int)lane % zs) * P.gridRes.x;
-            filled = off[row + x0 - 1] < off[row + x1 + srch - 1];
+        int y_end = y1 + srch - 2;
+        if constexpr (SPARSE) {   // a look at all rows of cells first, a lane each
+            const int zs = z1 - z0 + srch, rows = (y1 - y0 + srch) * zs;
+            bool filled = rows > 32;
+            if ((int)lane < rows && !filled) {
+                const int row = ((y0 - 1 + (int)lane / zs) * P.gridRes.z + z0 - 1 + (int)lane % zs) * P.gridRes.x;
+                filled = off[row + x0 - 1] < off[row + x1 + srch - 1];
+            }
+            if (!__any_sync(0xffffffffu, filled)) y_end = y0 - 2;
         }
-        const int y_end = __any_sync(0xffffffffu, filled) ? y1 + srch - 2 : y0 - 2;
         for (int y = y0 - 1; y <= y_end; y++)
             for (int z = z0 - 1; z <= z1 + srch - 2; z++) {
                 const int row = (y * P.gridRes.z + z) * P.gridRes.x;
@@ -263,7 +267,10 @@ int fl_launch_sample_volume(fl_system *s, const int res[3], const float bmin[3],
     if (sample_bricks(s->D, L)) {
         const int3 bricks = make_int3((res[0] + 3) / 4, (res[1] + 3) / 4, (res[2] + 1) / 2);
         const long long n = (long long)bricks.x * bricks.y * bricks.z;
-        k_sample_bricks<<<blocks_for(n, kVolumeThreads / 32), kVolumeThreads, 0, s->stream>>>(
+        // points whose supports fill a twentieth of the box at most
+        const float box = fabsf((bmax[0] - bmin[0]) * (bmax[1] - bmin[1]) * (bmax[2] - bmin[2]));
+        auto kern = 20.0f * (float)s->n * s->D.rd2 * sqrtf(s->D.rd2) < box ? k_sample_bricks<true> : k_sample_bricks<false>;
+        kern<<<blocks_for(n, kVolumeThreads / 32), kVolumeThreads, 0, s->stream>>>(
             s->D, L, bricks, s->f[F_POS].cur<float4>(), s->f[F_GCELL].cur<uint32_t>(), s->off, out);
     } else {
         const long long n = (long long)res[0] * res[1] * res[2];

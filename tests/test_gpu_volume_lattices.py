@@ -53,3 +53,25 @@ def test_a_volume_without_points_is_zero():
         s.SetParticles(pos)
         for res in ((40, 40, 40), (8, 8, 8)):
             assert not s.SampleParticles(res, LO, (10.0, 30.0, 10.0), 1.0).any()
+
+
+@pytest.mark.parametrize("grid_density", [0.75, 2.0])
+@pytest.mark.parametrize("n", [1, 60, 690])
+def test_lattices_of_a_mostly_empty_box_equal_the_oracle(n, grid_density):
+    """Points whose supports fill little of the box (690: a twentieth of it,
+    about), most bricks without one: the lattice of bricks and its neighbours
+    in size and spacing."""
+    p = scenes.make_params(LO, HI, grid_density=grid_density)
+    rng = np.random.default_rng(n)
+    pos = (np.array([-12.0, 20.0, 7.0]) + rng.normal(0, 3.0, (n, 3))).astype(np.float32)
+    pos[: n // 3] = rng.uniform(np.array(LO) + 2, np.array(HI) - 2, (n // 3, 3))
+    with F.FluidSystem(p, n) as s:
+        s.SetParticles(pos)
+        s.SampleParticles((2, 2, 2), LO, HI)
+        got_pos, off, cnt = s.GetBuffer(F.FPOS), s.GetBuffer(F.FGRIDOFF), s.GetBuffer(F.FGRIDCNT)
+        for res, lo, hi in (((141, 139, 143), LO, HI), ((61, 67, 65), LO, HI), ((131, 30, 120), (-35, 10, -10), (20, 25, 31))):
+            got = s.SampleParticles(res, lo, hi, 0.5, sort_first=False)
+            want = O.sample_volume(p, got_pos, off, cnt, res, np.array(lo, np.float32), np.array(hi, np.float32), 0.5)
+            scale = max(float(np.abs(want).max()), 1e-30)
+            assert np.allclose(got, want, rtol=RTOL, atol=RTOL * scale), (res, float(np.abs(got - want).max() / scale))
+            assert (want > 0).any()
