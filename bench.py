@@ -5,9 +5,9 @@ Workload (N=1): the 4,000,000-point wave tank -- a jittered lattice filling
 the low-x 40% of a ~330-unit box, dam-break parameters (h = 0.01 m, cell 2h,
 gridSrch 2), X- wall forcing at frequency 0.2 and amplitude 0.3. One step
 is one full Run: insert, scan, index scatter, canonical cell sort (and the
-crowded-cell sort), gather, density, force + advance (eight kernels; the
-neighbour passes per --passes, by default switching from the per-point to
-the cell-task passes once a cell crowds past 512 points).
+crowded-cell sort), gather, density, force + advance, with launches of their
+own for crowded tiles (the neighbour passes per --passes, by default with
+one for the densities of packed tiles once a cell crowds past 512 points).
 
   value   device-timed throughput, state resident in HBM, graph replay of
           exactly K steps between CUDA events on the system stream, run as

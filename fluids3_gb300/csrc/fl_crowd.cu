@@ -10,8 +10,8 @@
 // their warp waited. Force and advance of a dam break as it collapses:
 // 32,768 points after 64 steps (0.9% of the points overflow) 223 -> 77 us,
 // after 100 steps (25%, up to 748 pairs) 585 -> 134 us; 65,536 points after
-// 160 steps (36%, up to 4,967 pairs) 3,340 -> 570 us. Half the issue slots are
-// used; the rest is the first warp's chain of additions and the waits on it.
+// 160 steps (36%, up to 4,967 pairs) 3,340 -> 570 us. 64% of the issue slots are
+// used there; the rest is the first warp's chain of additions and the waits on it.
 #include <algorithm>
 
 #include "fl_internal.h"
@@ -26,9 +26,10 @@ constexpr int kCrowdThreads = 512;   // (256: 5-20% slower; 128: half as fast)
 constexpr int kCrowdSlots = 8;       // candidates a warp and round
 // From this many tiles a multiprocessor in a class (twice as many of the packed
 // ones, which differ more), a warp takes each by itself: nothing is lost to the
-// adding warp and the waits on it, and there is work for every warp. Force + advance, dam break of 1,048,576 points after
-// 110 and 170 steps, shared | alone: 1,562 | 944, 12,711 | 7,775 us; of 131,072
-// after 170 steps (a line at 8 a multiprocessor) 2,640 | 5,978 us.
+// adding warp and the waits on it, and there is work for every warp. Force +
+// advance, dam break of 1,048,576 points after 110 and 170 steps, shared | alone:
+// 1,562 | 944, 12,711 | 7,775 us; of 131,072 after 170 steps (a line at 8 a
+// multiprocessor) 2,640 | 5,978 us.
 constexpr uint32_t kAloneTiles = 16;
 constexpr int kAloneThreads = 128, kAloneBlocksPerSm = 6;
 struct ForceShared {               // per warp

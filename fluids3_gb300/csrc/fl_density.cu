@@ -29,11 +29,12 @@
 // ones that are few are shared by whole blocks of k_density, packed ones that
 // are many are walked apart, without the filter, by k_density_packed.
 //
-// What bounds it: instruction issue (88 warp instructions a point, half of them
-// the sum's: about 24 visits a warp, the lanes' mean being 16). A thread per
-// point over flag-pruned candidates took 157, and its chain of dependent loads
-// left small scenes waiting: 2,048 points 35.0 us then, 18.4 now; 65,536:
-// 46.1, 24.7; 1,000,000 (wave tank): 164, 110. With gridSrch 3 (250,000
+// What bounds it: instruction issue (104 warp instructions a point of the wave
+// tank of 1,000,000 after 5 steps, half of them the sum's: about 24 visits a
+// warp, the lanes' mean being 16). A thread per point over flag-pruned
+// candidates took 157, and its chain of dependent loads left small scenes
+// waiting: 2,048 points 35.0 us then, 18.4 now; 65,536: 46.1, 24.7; 1,000,000
+// (wave tank, with the events around it): 189, 136. With gridSrch 3 (250,000
 // points, 165 candidates and 70 pairs a point) the rows take 69 us, the old
 // loop took 118 and the filter 140: there every third candidate is a pair, and
 // a warp's points come from more runs than one. Staging a row's run in shared
@@ -66,10 +67,10 @@ static_assert(32 * kMaskRow <= 32 * 8, "the masks fit where the product rows wer
 // Runs of points that a warp takes one by one, and cells that its points may lie
 // in; beyond, the lanes walk alone: in spray, a run's union of blocks holds few
 // candidates of any one point. Density launch of 1,000,000 points spread evenly,
-// cells of 2h with 1, 2, 3, 5 and 8 points: 44, 50, 60, 74, 81 us with 6 cells,
-// 134, 95, 88, 82, 80 with as many as there are (8 runs then), 44, 51, 58, 73, 89
+// cells of 2h with 1, 2, 3, 5 and 8 points: 44, 50, 59, 75, 81 us with 6 cells,
+// 134, 94, 88, 83, 81 with as many as there are (8 runs then), 44, 50, 57, 72, 88
 // with 4. The wave tank (1,000,000) after 4 steps 136, 153, 136, the dam break
-// (65,536) 29.1, 29.4, 30.9; with 2 runs that took 31.9.
+// (65,536) 28.1, 30.8, 29.4; with 2 runs that took 33.1.
 constexpr int kMaxSegments = 4, kMaxCells = 6;
 constexpr float kUnits = 1000.0f;               // half the widest side of the box, in units (2 x stays exact in half)
 constexpr float kBase = 2048.0f;                // squares are split into kBase * high + low, both exact in half

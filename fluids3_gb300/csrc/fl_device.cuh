@@ -214,7 +214,8 @@ __device__ __forceinline__ int band_grouped_slot(int n, const float4 *__restrict
 // warp w = i / 32, lane l = i % 32) entry t lives at
 // ((w * hcap + t) * 32 + l), so a warp reading entry t of all its lanes
 // touches one 128-byte line. Entries past hcap are not stored; the count
-// still records every pair, and the force pass re-walks such warps.
+// still records every pair, and the force pass leaves such warps to the kernels of
+// fl_crowd.cu.
 __device__ __forceinline__ size_t list_at(const DevParams &P, int i, uint32_t t) {
     return ((size_t)(i >> 5) * (size_t)P.hcap + t) * 32u + (uint32_t)(i & 31);
 }
